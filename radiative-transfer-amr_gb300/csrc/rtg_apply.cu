@@ -10,7 +10,7 @@
 // product from shared memory in 4 x 4 register tiles, factorised inflow face
 // fluxes, then every output DOF written in global order.  FP32 plans may hand
 // the scattering product to scat_tc_kernel (tcgen05 tensor cores, TF32 hi/lo
-// split).  The plan shape (rows per item, items per CTA, launches per
+// split), FP64 plans to rtg_scat64.cu (tcgen05, eight 8-bit digits).  The plan shape (rows per item, items per CTA, launches per
 // shared-memory class, tensor cores or not) is autotuned per handle
 // (tune_plan).  Columns too large for the tiled path use apply_col_kernel
 // (per-output chunks from shared memory) or apply_global_kernel (operands
@@ -25,7 +25,9 @@
 #include <string>
 #include <tuple>
 
+#include "rtg_apply_common.cuh"
 #include "rtg_internal.h"
+#include "rtg_scat64.h"
 
 namespace rtg {
 
@@ -39,11 +41,6 @@ __device__ __forceinline__ int gofs(int n) { return (n - 1) * n * (2 * n - 1) / 
 
 template <typename T>
 __device__ __forceinline__ T tabs(T v) { return v < T(0) ? -v : v; }
-
-__device__ __forceinline__ bool bdry_node(int bm, int i, int j, int nx, int ny) {
-    return ((bm & 1) && i == nx - 1) || ((bm & 2) && j == ny - 1) || ((bm & 4) && i == 0) ||
-           ((bm & 8) && j == 0);
-}
 
 // Face terms of one output node: outflow diagonal or inflow mortar couplings
 // to neighbour elements (rt/boundary_convection_matrix.py:258-524).
@@ -105,24 +102,6 @@ __device__ __forceinline__ T face_terms(const OpView<T>& v, const float* __restr
         }
     }
     return acc;
-}
-
-struct ApplyFlags {
-    bool scat, mass, merged, ic, bc, mask_rows;
-    float ic_sign;
-};
-
-__device__ __forceinline__ ApplyFlags decode(uint32_t flags) {
-    ApplyFlags f;
-    const bool sys = flags & RTG_SYSTEM;
-    f.scat = sys || (flags & RTG_SCAT);
-    f.mass = sys || (flags & RTG_MASS);
-    f.merged = f.scat && f.mass;   // (M - S) block with the joint drop rule
-    f.ic = sys || (flags & RTG_IC);
-    f.ic_sign = sys ? -1.f : 1.f;
-    f.bc = sys || (flags & RTG_BC);
-    f.mask_rows = flags & RTG_MASK_ROWS;
-    return f;
 }
 
 // ---------------------------------------------------------------- fast path
@@ -278,10 +257,12 @@ apply_col_kernel(OpView<T> v, const float* __restrict__ Wf32, const float* __res
 // before the epilogue; T and Fy reuse the W region.  Every global -> shared
 // copy is a cp.async, so a staging loop has all its loads in flight.
 // Shared memory: Xs[Nth][nijp] | column table | cell rows and flags | item
-// region: WsT[Nth][Mp] (later T | Fy[Mp][nijp]) | Ys[Mp][nijp] |
-// row table[Mp][kRowVals] | row -> cell.  Without the product (the
-// tensor-core path takes it) a CTA may hold any run of items of its column,
-// down to one, and Xs holds only the current item's rows.
+// region: WsT[Nth][Mp] (later T | Fy[Mp][nijp]) | Ys[Mp][nijp].  Without the
+// product (a tensor-core kernel takes it) Xs and the row table hold only the
+// current item's rows and there is no Ys: a quarter of the shared memory, so
+// that the FP64 kernel, bound by its pipe (two lanes a clock and SM), keeps four
+// CTAs on an SM (536 -> 456 us at 7.95e6 DOF against whole-column tables and
+// three).
 //
 // FP64 (kParity) keeps the reference's drop rules without per-term tests on
 // the common path:
@@ -403,14 +384,24 @@ __device__ __forceinline__ void store4(double* p, const double v[4]) {
     *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
 }
 
-// values of the per-row table: dxdydth/8 * wth_r, dx dth/4, dy dth/4, wth_r,
-// wth_r sin, wth_r cos, ThF_0..3 of the row's cell
-constexpr int kRowVals = 10;
+// values of the per-row table, every product of row constants made once per
+// row (an output then takes nx + ny + 7 FP64 operations and two per outflow
+// face; the FP64 kernel without the product is bound by them): dxdydth/8 wth_r,
+// +-dx dth/4 wth_r sin, +-dy dth/4 wth_r cos (the sign of IC in the operator),
+// the outflow coefficient wth_r ThF dcoeff of face F at 3 + F (0: no outflow),
+// W[R][R], a pad (an odd stride: rows in different banks)
+constexpr int kRowVals = 9;
 
 // threads of a tiled CTA: FP32 items are latency bound (more warps per SM),
 // FP64 ones register bound
 template <typename T>
 __host__ __device__ constexpr int tiled_threads() { return sizeof(T) == 8 ? 256 : 512; }
+
+// |v| > tol (false for NaN) by the bits: no work for the FP64 pipe
+__device__ __forceinline__ bool above(double v, double tol) {
+    const long long b = __double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFll;
+    return b > __double_as_longlong(tol) && b <= 0x7FF0000000000000ll;
+}
 
 // values of the per-column table: kw and sw per node, LGL weights in x and y,
 // the two derivative tables
@@ -426,13 +417,14 @@ __host__ __device__ __forceinline__ int col_int_words(int ncell, int nth_col) {
 // kProduct = false: the tensor-core kernel does the scattering product (FP32),
 // so the CTA neither stages W nor runs the product and fits three per SM
 template <typename T, bool kParity, bool kProduct = true>
-__global__ void __launch_bounds__(tiled_threads<T>(), sizeof(T) == 8 ? 3 : (kProduct ? 2 : 3))
+__global__ void __launch_bounds__(tiled_threads<T>(), sizeof(T) == 8 ? (kProduct ? 3 : 4) : (kProduct ? 2 : 3))
 apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* __restrict__ groups,
                    const TileItem* __restrict__ items, const TileCpl* __restrict__ cpl_ent, const T* __restrict__ x,
                    T* __restrict__ y) {
     extern __shared__ double2 smt4[];
     __shared__ __align__(16) TileCpl sc[kMaxItemCpl];
     __shared__ float s_rcp[kMaxNodes + 1];    // 1/n rounded to float
+    __shared__ uint8_t s_cls[kParity ? kMaxNodes * kMaxNodes : 1];   // scattering class per node
     T* smt = reinterpret_cast<T*>(smt4);
     if (v.stop && *v.stop) return;
     const int4 grp = groups[blockIdx.x];      // column, first item, end item
@@ -441,6 +433,9 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
     const ColDev C = v.cols[ci];
     const ApplyFlags fl = decode(flags);
     const bool scat = kProduct && fl.scat;
+    // without the product the other kernel adds its part: FP32 both add into a
+    // zeroed y at once, FP64 after this kernel has written y
+    constexpr bool kStore = kProduct || kParity;
     const int nij = C.nx * C.ny, Nth = C.nth_col, ncell = C.elem_end - C.elem_begin;
     const int nijp = (nij + 3) & ~3, Nthp = (Nth + 3) & ~3;
     // with the product every row of x is staged once per column; without it
@@ -449,15 +444,15 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
     const int xrows = kProduct ? Nth : grp.w;
     T* Xs = smt;                                                  // [xrows][nijp]
     T* colt = Xs + (size_t)xrows * nijp;                          // column table
-    T* rowt = colt + col_table_size(C.nx, C.ny);                  // [Nthp][kRowVals]
-    int* crow = reinterpret_cast<int*>(rowt + (size_t)Nthp * kRowVals);   // [ncell+1] first row; crow[ncell] = Nth
+    T* rowt = colt + col_table_size(C.nx, C.ny);                  // [Nthp or xrows][kRowVals]
+    int* crow = reinterpret_cast<int*>(rowt + (size_t)(kProduct ? Nthp : xrows) * kRowVals);   // [ncell+1] first row; crow[ncell] = Nth
     int* cflg = crow + ncell + 1;                                          // [ncell] element flags
     int* ccpl = cflg + ncell;                                              // [ncell+1] first coupling
     int* cang = ccpl + ncell + 1;                                          // [ncell] angular table offset
     int* rcell = cang + ncell;                                             // [Nth] cell of each row
     T* ireg = reinterpret_cast<T*>(crow + col_int_words(ncell, Nth));    // item region
     const T* kwn = colt;
-    const T* swn = colt + nij;
+    T* cwn = colt + nij;                 // dx dy / 8 wx_i wy_j sigma, from wx_i wy_j sigma once staged
     const T* wxs = colt + 2 * nij;
     const T* wys = wxs + C.nx;
     const T* Gxs = wys + C.ny;
@@ -508,25 +503,26 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
             for (int t = threadIdx.x; t < Nth * (nijp - nij); t += blockDim.x)
                 Xs[(t / (nijp - nij)) * nijp + nij + t % (nijp - nij)] = T(0);
     }
-    // the column's row table
-    for (int R = threadIdx.x; R < Nth; R += blockDim.x) {
-        const int k = rcell[R];
-        const int e = C.elem_begin + k;
-        const int r = R - crow[k], nth = crow[k + 1] - crow[k];
-        const T* A = v.ang + cang[k];
-        T* rw = rowt + R * kRowVals;
-        const T ar = A[r];
-        rw[0] = v.econst[4 * e] * ar;
-        rw[1] = v.econst[4 * e + 1];
-        rw[2] = v.econst[4 * e + 2];
-        rw[3] = ar;
-        rw[4] = A[nth + r];
-        rw[5] = A[2 * nth + r];
+    // row table of rows [R0, R1) (with the product the column's, else the item's)
+    auto row_table = [&](int R0, int R1) {
+        for (int R = R0 + threadIdx.x; R < R1; R += blockDim.x) {
+            const int k = rcell[R];
+            const int e = C.elem_begin + k;
+            const int r = R - crow[k], nth = crow[k + 1] - crow[k];
+            const T* A = v.ang + cang[k];
+            T* rw = rowt + (R - R0) * kRowVals;
+            const T ar = A[r], cx = v.econst[4 * e + 1], cy = v.econst[4 * e + 2], sg = T(fl.ic_sign);
+            rw[0] = v.econst[4 * e] * ar;
+            rw[1] = sg * cx * A[nth + r];
+            rw[2] = sg * cy * A[2 * nth + r];
 #pragma unroll
-        for (int F = 0; F < 4; ++F) rw[6 + F] = A[(3 + F) * nth + r];
-    }
+            for (int F = 0; F < 4; ++F)
+                rw[3 + F] = (cflg[k] & (1 << F)) ? (F % 2 == 0 ? cy : cx) * ar * A[(3 + F) * nth + r] : T(0);
+            rw[7] = v.W[v.W_off[C.sig] + (int64_t)R * Nth + R];
+        }
+    };
+    if constexpr (kProduct) row_table(0, Nth);
     const T* Wg = v.W + v.W_off[C.sig];
-    const T small = T(kSmall);
     const T dxdy8 = v.colc[ci];
     const float rny = __frcp_rn((float)C.ny);
     T* yc = y + C.dof_off;
@@ -560,6 +556,7 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
             }
         }
         if constexpr (!kProduct) {
+            row_table(it.row0, it.row0 + M);
             // the item's rows of x (its DOFs are contiguous: whole cells),
             // row R at Xs[R - row0]; the product does not run, so the pad
             // columns are never read
@@ -573,6 +570,13 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
             }
         }
         cp_async_wait_all();
+        if (iq == grp.y) {
+            __syncthreads();
+            for (int q = threadIdx.x; q < nij; q += blockDim.x) {
+                cwn[q] *= dxdy8;
+                if constexpr (kParity) s_cls[q] = par.scls[C.node_off + q];
+            }
+        }
         __syncthreads();
         if (scat) {
             const int tm = Mp / 4, tn = nijp / 4, ntile = tm * tn;
@@ -784,58 +788,54 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
             const int i = small_div(ij, rny), j = ij - i * C.ny;
             const int flg = cflg[k];
             if (fl.mask_rows && bdry_node(flg >> 4, i, j, C.nx, C.ny)) {
-                if constexpr (kProduct) yc[d] = T(0);   // tensor-core path: y was zeroed
+                if constexpr (kStore) yc[d] = T(0);   // FP32 tensor-core path: y was zeroed
                 continue;
             }
             const int R = crow[k] + r;
             const int m = R - it.row0;   // row within the item
             const int xr0 = kProduct ? R : m;   // row of Xs
-            const T* rw = rowt + R * kRowVals;
+            const T* rw = rowt + xr0 * kRowVals;
             const T xself = Xs[xr0 * nijp + ij];
             const T mterm = rw[0] * kwn[ij];
             T acc = T(0);
             if constexpr (kParity) {
-                if (scat) {
-                    const int node = C.node_off + ij;
-                    const T swv = swn[ij];
-                    const T cw = dxdy8 * swv;
-                    const int cls = par.scls[node];
-                    T s = T(0);
+                if (fl.scat) {
+                    const T cw = cwn[ij];
+                    const T vd = fma(-cw, rw[7], fl.merged ? mterm : T(0));
+                    acc = (above(vd, kSmall) ? vd : T(0)) * xself;
+                    const int cls = s_cls[ij];
                     if (cls == 1 || cls == 2) {
-                        s = Ys[m * nijp + ij];
+                        if constexpr (kProduct) acc = fma(-cw, Ys[m * nijp + ij], acc);   // else the tensor-core kernel adds it
                     } else if (cls == 3) {
-                        // own-cell terms only, some kept: test each one
-                        const bool skip_cross = !(tabs(swv) > small);
-                        const int c0 = skip_cross ? crow[k] : 0;
-                        const int c1 = skip_cross ? crow[k] + nth : Nth;
+                        // |wx wy sigma| <= 1e-14: own-cell terms only, some kept: test each one
+                        T s = T(0);
                         const float cwf = fabsf((float)cw);
                         const float hi = 1.e-14f * (1.f + 1.e-6f), lo = 1.e-14f * (1.f - 1.e-6f);
                         const float* Wf = par.Wf + v.W_off[C.sig];
-                        for (int c = c0; c < c1; ++c) {
+                        for (int c = crow[k]; c < crow[k] + nth; ++c) {
                             const T wv = Wg[(int64_t)R * Nth + c];
                             const float pf = cwf * fabsf(Wf[(int64_t)R * Nth + c]);
                             bool keep = pf > hi;
-                            if (!keep && pf >= lo) keep = tabs(cw * wv) > small;
-                            s = fma(keep && c != R ? wv : T(0), Xs[c * nijp + ij], s);
+                            if (!keep && pf >= lo) keep = tabs(cw * wv) > T(kSmall);
+                            s = fma(keep && c != R ? wv : T(0), Xs[(kProduct ? c : c - it.row0) * nijp + ij], s);
                         }
+                        acc = fma(-cw, s, acc);
                     }
-                    const T vd = (fl.merged ? mterm : T(0)) - cw * Wg[(int64_t)R * Nth + R];
-                    acc = -cw * s + (tabs(vd) > small ? vd : T(0)) * xself;
                 }
-                if (fl.mass && !fl.merged) acc += mterm * xself;
+                if (fl.mass && !fl.merged) acc = fma(mterm, xself, acc);
             } else {
-                if (scat) acc = -dxdy8 * swn[ij] * Ys[m * nijp + ij];
-                if (fl.mass) acc += mterm * xself;
+                if (scat) acc = -cwn[ij] * Ys[m * nijp + ij];
+                if (fl.mass) acc = fma(mterm, xself, acc);
             }
             if (fl.ic) {
                 const T* xr = Xs + xr0 * nijp;
                 T t1 = T(0), t2 = T(0);
                 const T* gy = Gys + j * C.ny;
-                for (int jj = 0; jj < C.ny; ++jj) t1 += gy[jj] * xr[i * C.ny + jj];
+                for (int jj = 0; jj < C.ny; ++jj) t1 = fma(gy[jj], xr[i * C.ny + jj], t1);
                 const T* gx = Gxs + i * C.nx;
-                for (int ii = 0; ii < C.nx; ++ii) t2 += gx[ii] * xr[ii * C.ny + j];
-                const T ic = rw[1] * wxs[i] * rw[4] * t1 + rw[2] * wys[j] * rw[5] * t2;
-                acc += T(fl.ic_sign) * ic;
+                for (int ii = 0; ii < C.nx; ++ii) t2 = fma(gx[ii], xr[ii * C.ny + j], t2);
+                acc = fma(rw[1], wxs[i] * t1, acc);
+                acc = fma(rw[2], wys[j] * t2, acc);
             }
             if (fl.bc && (i == 0 || j == 0 || i == C.nx - 1 || j == C.ny - 1)) {
                 acc += Fy[m * nijp + ij];
@@ -845,16 +845,25 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
                     const bool on = (F == 0 && i == C.nx - 1) || (F == 1 && j == C.ny - 1) || (F == 2 && i == 0) ||
                                     (F == 3 && j == 0);
                     if (!on) continue;
-                    const T dc = (F % 2 == 0) ? rw[2] : rw[1];
                     const T w = (F % 2 == 0) ? wys[j] : wxs[i];
-                    const T val = dc * w * rw[3] * rw[6 + F];
-                    if (!kParity || tabs(val) > T(kBcTol)) acc += val * xself;
+                    T val = rw[3 + F] * w;
+                    if constexpr (kParity) {
+                        // |value| > 1e-15, near it in the reference's order of the product
+                        if (!above(val, 2. * kBcTol)) {
+                            const int e = C.elem_begin + k;
+                            const T* A = v.ang + cang[k];
+                            val = ((F % 2 == 0) ? v.econst[4 * e + 2] : v.econst[4 * e + 1]) * w * A[r] *
+                                  A[(3 + F) * nth + r];
+                            if (!(tabs(val) > T(kBcTol))) continue;
+                        }
+                    }
+                    acc = fma(val, xself, acc);
                 }
             }
             // tensor-core path: the scattering kernel adds its part to the
             // same zeroed y concurrently; two terms on zero sum the same in
             // either order
-            if constexpr (kProduct)
+            if constexpr (kStore)
                 yc[d] = acc;
             else
                 atomicAdd(yc + d, acc);
@@ -927,19 +936,6 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint3
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
-}
-
-// bounded wait for the completion of phase `parity` of an mbarrier
-__device__ __forceinline__ bool mbar_wait(uint32_t mb, uint32_t parity) {
-    uint32_t done = 0;
-    for (int spin = 0; spin < (1 << 22) && !done; ++spin)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(mb), "r"(parity)
-            : "memory");
-    return done != 0;
 }
 
 __global__ void __launch_bounds__(kTcThreads)
@@ -1300,6 +1296,10 @@ struct ParityTables {
     std::vector<int> esc, etc;     // per coupling: offsets of dcoeff*Es and Et in the cleaned table
     std::vector<char> tested;      // per coupling: summed term by term
     std::vector<uint8_t> diag;     // per coupling: cleaned Es (bit 0) / Et (bit 1) diagonal
+    std::vector<uint8_t> scls;     // host copies of d_scls and d_thr
+    std::vector<uint64_t> thr;
+    Scat64* s64 = nullptr;         // the product on the tensor cores (plans with tc)
+    std::vector<char> s64_cols;    // the columns it covers
     int64_t nodes[4] = {0, 0, 0, 0};   // nodes per scattering class
     int64_t ntested = 0;
 };
@@ -1325,6 +1325,8 @@ struct ApplyPlan {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int64_t ndof = 0;
+    int tc = 0;                          // the tensor cores do the tiled columns' scattering product
+    std::vector<char> tiled;             // per column: in the tiled path
     const ParityTables* par = nullptr;   // FP64 tiled path
     bool own_par = false;
     std::vector<TuneRecord> tuning;
@@ -1333,6 +1335,7 @@ struct ApplyPlan {
 
 static void free_parity(const ParityTables* pt) {
     if (!pt) return;
+    free_scat64(pt->s64);
     cudaFree(pt->d_scls);
     cudaFree(pt->d_mortc);
     cudaFree(pt->d_colfull);
@@ -1501,6 +1504,8 @@ static ParityTables* build_parity(const rtg_handle* h) {
             }
         }
     }
+    pt->scls = scls;
+    pt->thr = thr;
     if (mortc.size() > (size_t)INT32_MAX) throw RtgError{RTG_ERR_ARG, "cleaned mortar table too large"};
     try {
         RTG_CUDA(cudaMalloc(&pt->d_scls, scls.size()));
@@ -1527,15 +1532,15 @@ static ParityTables* build_parity(const rtg_handle* h) {
 // Shared memory of a group: the column part (input, column table, cell
 // rows and flags) and the largest item region of its items.
 // xrows: rows of x staged (the column's nth_col with the product, the most
-// rows of an item of the group without it)
-static size_t tile_col_bytes(size_t vsize, int nth_col, int nx, int ny, int ncell, int xrows) {
-    const int nijp = (nx * ny + 3) & ~3, nthp = (nth_col + 3) & ~3;
+// rows of an item of the group without it, as many as the row table then has)
+static size_t tile_col_bytes(size_t vsize, int nth_col, int nx, int ny, int ncell, int xrows, bool product) {
+    const int nijp = (nx * ny + 3) & ~3, nthp = product ? (nth_col + 3) & ~3 : xrows;
     return vsize * ((size_t)xrows * nijp + (size_t)col_table_size(nx, ny) + (size_t)nthp * kRowVals) +
            sizeof(int) * col_int_words(ncell, nth_col) + 16;
 }
-static size_t tile_item_bytes(size_t vsize, int nx, int ny, int wcap, int M) {
+static size_t tile_item_bytes(size_t vsize, int nx, int ny, int wcap, int M, bool product) {
     const int nijp = (nx * ny + 3) & ~3, Mp = (M + 3) & ~3;
-    return vsize * ((size_t)wcap + (size_t)Mp * nijp);
+    return vsize * ((size_t)wcap + (product ? (size_t)Mp * nijp : 0));
 }
 
 // Dynamic shared memory that lets q CTAs of the tiled kernel share an SM,
@@ -1569,11 +1574,12 @@ static ApplyPlan* make_plan(const rtg_handle* h, const std::vector<int>* cap = n
                             const ParityTables* par = nullptr, int gcap = 0, int split = 0, int tc = 0) {
     const HostTables& t = h->host;
     constexpr bool parity = sizeof(T) == 8;
-    if (parity) tc = 0;
     std::vector<std::pair<int64_t, TcItem>> tcv;
     std::map<int, int64_t> sig_tile;   // signature -> its first W tile
     std::vector<float> wtiles;
     ApplyPlan* p = new ApplyPlan();
+    p->tc = tc;
+    p->tiled.assign(t.cols.size(), 0);
     std::vector<std::pair<int64_t, int4>> items[2];
     struct GroupRec {
         int64_t cost;
@@ -1592,7 +1598,7 @@ static ApplyPlan* make_plan(const rtg_handle* h, const std::vector<int>* cap = n
         const int ncell = C.elem_end - C.elem_begin;
         const int nij = C.nx * C.ny;
         const int rows_cap = cap ? (*cap)[ci] : kTileRows;
-        if ((!parity || par) && ncell <= kMaxCellsStaged) {
+        if ((!parity || (par && (!tc || scat64_fits(C)))) && ncell <= kMaxCellsStaged) {
             // split the column into items of whole cells; halve the rows per
             // item (down to 4) until every item fits next to the staged column
             std::vector<TileItem> its;
@@ -1600,7 +1606,7 @@ static ApplyPlan* make_plan(const rtg_handle* h, const std::vector<int>* cap = n
             std::vector<int64_t> icost;
             std::vector<std::vector<TileCpl>> ents;
             // column part of the shared memory with x rows xr
-            auto colb = [&](int xr) { return tile_col_bytes(sizeof(T), C.nth_col, C.nx, C.ny, ncell, xr); };
+            auto colb = [&](int xr) { return tile_col_bytes(sizeof(T), C.nth_col, C.nx, C.ny, ncell, xr, !tc); };
             bool fits = false;
             for (int rcap = rows_cap; rcap > 0 && !fits; rcap = rcap > 4 ? rcap / 2 : 0) {
                 its.clear();
@@ -1670,17 +1676,18 @@ static ApplyPlan* make_plan(const rtg_handle* h, const std::vector<int>* cap = n
                     ti.wcap = tc ? ti.tsz + Mp * nijp : std::max(C.nth_col * Mp, ti.tsz + Mp * nijp);
                     if ((ti.wcap & 3) || (ti.tsz & 3) || (nijp & 3))
                         throw RtgError{RTG_ERR_ARG, "tiled apply: unaligned shared-memory region"};
-                    ibytes.push_back(tile_item_bytes(sizeof(T), C.nx, C.ny, ti.wcap, M));
+                    ibytes.push_back(tile_item_bytes(sizeof(T), C.nx, C.ny, ti.wcap, M, !tc));
                     icost.push_back((int64_t)M * nij * (C.nth_col + C.nx + C.ny) + C.ndof);
                     ents.push_back(std::move(en));
                     its.push_back(ti);
                 }
                 for (size_t q = 0; q < its.size() && fits; ++q)
                     if (colb(tc ? (its[q].M + 3) & ~3 : C.nth_col) + ibytes[q] > kSmemBudget) fits = false;
-                if (tc && tc_smem_bytes(nij, C.nth_col) > kSmemBudget) fits = false;
+                if (!parity && tc && tc_smem_bytes(nij, C.nth_col) > kSmemBudget) fits = false;
             }
             if (fits) {
-                if (tc) {
+                p->tiled[ci] = 1;
+                if (!parity && tc) {
                     auto its_ = sig_tile.find(C.sig);
                     if (its_ == sig_tile.end()) {
                         const int n = C.nth_col;
@@ -1851,7 +1858,7 @@ static void set_plan_attributes(const ApplyPlan* p) {
     constexpr bool f64 = sizeof(T) == 8;
     raise_smem_limit((const void*)apply_col_kernel<T, T, f64>, std::max(p->g[0].smem, p->g[1].smem));
     if (p->ntiles) {
-        if (p->ntc)
+        if (p->tc)
             raise_smem_limit((const void*)apply_tiled_kernel<T, f64, false>, p->tile_smem);
         else
             raise_smem_limit((const void*)apply_tiled_kernel<T, f64>, p->tile_smem);
@@ -1893,7 +1900,7 @@ static void run_plan(const ApplyPlan* plan, const OpView<T>& v, const OpView<flo
             const int n = plan->tg_begin[q + 1] - plan->tg_begin[q];
             if (!n) continue;
             const int4* grp = plan->d_tgroups + plan->tg_begin[q];
-            if (plan->ntc)
+            if (plan->tc)
                 apply_tiled_kernel<T, f64, false><<<n, tiled_threads<T>(), plan->tg_smem[q], s>>>(
                     v, tp, flags, grp, plan->d_tiles, plan->d_tile_cpl, x, y), count_launch();
             else
@@ -1911,6 +1918,10 @@ static void run_plan(const ApplyPlan* plan, const OpView<T>& v, const OpView<flo
             }
         }
     }
+    if constexpr (f64) {
+        if (plan->tc && (flags & (RTG_SYSTEM | RTG_SCAT)))
+            launch_scat64(plan->par->s64, v, flags, x, y, s);
+    }
     for (int grp = 0; grp < 2; ++grp) {
         const ApplyGroup& G = plan->g[grp];
         if (G.nitems) {
@@ -1927,10 +1938,21 @@ static void run_plan(const ApplyPlan* plan, const OpView<T>& v, const OpView<flo
 }
 
 static int plan_launches(const ApplyPlan* p) {
-    int n = (p->g[0].nitems > 0) + (p->g[1].nitems > 0) + (p->nslow > 0) + (p->ntc > 0);
+    int n = (p->g[0].nitems > 0) + (p->g[1].nitems > 0) + (p->nslow > 0) + (p->tc > 0);
     for (int q = 0; q < kSmemClasses; ++q) n += p->tg_begin[q + 1] > p->tg_begin[q];
     return n;
 }
+
+// FP64 multiply-adds of the scattering product from which plans with the
+// tensor cores (rtg_scat64.cu) are timed beside those of the FP64 pipe, and from
+// which they alone are.  Whole applies, FP64 pipe against tensor cores, in us: 19.8
+// and 27.9 at 1.2e6 (33,056 DOF adaptive: an extra launch), 51.6 and 49.9 at 8.6e6
+// (218,581 DOF adaptive), 73 and 38 at 2.1e7, 459 and 103 at 1.6e8, 4067 and 870 at
+// 1.5e9 (7.95e6 DOF, two scatterers).
+constexpr int64_t kTc64Offer = 4'000'000, kTc64Alone = 100'000'000;
+
+// where the tensor-core kernel of a plan reports a wait that gave up
+static int* plan_status(const ApplyPlan* p) { return p->par ? scat64_status(p->par->s64) : p->d_status; }
 
 // Builds the plan of one shape (FP64: with the host-resolved drop rules).
 template <typename T>
@@ -1947,11 +1969,12 @@ static const OpView<T>& view_of(const rtg_handle* h) {
         return h->v32;
 }
 
-// Times a plan: one warm-up, best of three whole applies (CUDA events); a
+// Times a plan: one warm-up, best of three whole applies (CUDA events; a plan
+// whose first one takes over 1.5 times the best plan's is given up); a
 // tensor-core plan whose waits gave up throws.
 template <typename T>
 static float time_plan(rtg_handle* h, ApplyPlan* p, const T* x, T* y, cudaEvent_t e0, cudaEvent_t e1,
-                       cudaStream_t s) {
+                       cudaStream_t s, float best) {
     set_plan_attributes<T>(p);
     run_plan<T>(p, view_of<T>(h), h->v32, RTG_SYSTEM | RTG_MASK_ROWS, x, y, s);
     float tt = 1e30f;
@@ -1963,22 +1986,23 @@ static float time_plan(rtg_handle* h, ApplyPlan* p, const T* x, T* y, cudaEvent_
         float ms = 0.f;
         RTG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         tt = std::min(tt, ms);
+        if (tt > 1.5f * best) break;
     }
-    if (p->ntc) {
+    if (p->tc) {
         int st = 0;
-        RTG_CUDA(cudaMemcpy(&st, p->d_status, sizeof(int), cudaMemcpyDeviceToHost));
+        RTG_CUDA(cudaMemcpy(&st, plan_status(p), sizeof(int), cudaMemcpyDeviceToHost));
         if (st) {
             h->poisoned = true;
-            throw RtgError{RTG_ERR_TIMEOUT, "scat_tc_kernel: a wait for the tensor cores gave up"};
+            throw RtgError{RTG_ERR_TIMEOUT, "scattering product: a wait for the tensor cores gave up"};
         }
     }
     return tt;
 }
 
 // Autotuner of the apply: every plan shape of the candidate list (rows per
-// item 16/32/64, one CTA per column or per item, one launch or one per
-// shared-memory class, FP32: with or without the tensor-core scattering) is
-// built and the whole apply timed; the fastest plan is kept.
+// item 4 to 64, one CTA per column or per item, one launch or one per
+// shared-memory class, with or without the tensor-core scattering) is built
+// and the whole apply timed; the fastest plan is kept.
 template <typename T>
 static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
     constexpr bool f64 = sizeof(T) == 8;
@@ -1999,20 +2023,51 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
     try {
         RTG_CUDA(cudaMalloc(&x, sizeof(T) * std::max<int64_t>(N, 1)));
         RTG_CUDA(cudaMalloc(&y, sizeof(T) * std::max<int64_t>(N, 1)));
-        RTG_CUDA(cudaMemsetAsync(x, 0, sizeof(T) * N, s));
+        // a positive value (FP64 4.8e-4, FP32 0.75): zeros would skip work
+        RTG_CUDA(cudaMemsetAsync(x, 0x3F, sizeof(T) * N, s));
         RTG_CUDA(cudaEventCreate(&e0));
         RTG_CUDA(cudaEventCreate(&e1));
+        // the products of the columns the tensor cores can take, and whether they take all
+        int64_t prod = 0;
+        bool all_fit = true;
+        for (const ColDev& C : h->host.cols) {
+            if (C.elem_end - C.elem_begin > kMaxCellsStaged) continue;   // not tiled
+            prod += (int64_t)C.nx * C.ny * C.nth_col * C.nth_col;
+            all_fit &= scat64_fits(C);
+        }
+        if (f64 && all_fit && prod >= kTc64Offer) {
+            std::vector<int> cap(h->host.cols.size(), kTileRows);
+            ApplyPlan* probe = make_plan<T>(h, &cap, nullptr, kChunk64, par, 0, 0, 1);
+            try {
+                par->s64 = build_scat64(h, probe->tiled, par->scls.data(), par->thr.data(), par->d_thr);
+                par->s64_cols = probe->tiled;
+            } catch (...) {
+                free_plan(probe);
+                throw;
+            }
+            free_plan(probe);
+        }
+        const bool tc64 = f64 && par->s64;
         std::vector<PlanShape> shapes;
-        for (int rows : {16, 32, 64})
-            for (int gcap : {0, 1})
-                for (int split : {0, 1}) shapes.push_back(PlanShape{rows, gcap, split, 0});
-        // tensor-core scattering (FP32): one CTA per column, items of 32 or 64
+        if (f64 && prod < kTc64Alone) {
+            // one CTA per item, down to a cell: a column per CTA leaves the FP64 pipes
+            // of a small mesh's other SMs idle (84.6 against 51.6 us at 218,581 DOF)
+            for (int rows : {4, 8, 16, 32, 64}) shapes.push_back(PlanShape{rows, 1, 0, 0});
+        } else if (!tc64) {
+            for (int rows : {16, 32, 64})
+                for (int gcap : {0, 1})
+                    for (int split : {0, 1}) shapes.push_back(PlanShape{rows, gcap, split, 0});
+        }
+        // tensor-core scattering, FP32: one CTA per column, items of 32 or 64
         // rows, the scattering CTAs of one angular mesh next to each other
         // (one CTA per item ties with these on the two-scatterer problem, and
         // the heaviest-first order of the scattering CTAs is 1.7 % slower there;
         // both are left out of the list, rtg_apply_shape can still pin them)
         if (!f64)
             for (int rows : {32, 64}) shapes.push_back(PlanShape{rows, 0, 0, 2});
+        // FP64: one CTA per item (one per column leaves SMs idle at its end)
+        if (tc64)
+            for (int rows : {16, 32, 64}) shapes.push_back(PlanShape{rows, 1, 0, 1});
         // the plans are built on host threads at once (host tables read only;
         // each thread makes its own uploads), then timed one by one
         int dev = 0;
@@ -2040,10 +2095,14 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
             const PlanShape& sh = shapes[q];
             ApplyPlan* p = plans[q];
             plans[q] = nullptr;
+            if (f64 && sh.tc && p->tiled != par->s64_cols) {   // not the columns of the digit tables
+                free_plan(p);
+                continue;
+            }
             TuneRecord r{sh, 0, -1, p->ntiles, p->tg_begin[kSmemClasses], plan_launches(p)};
             float tt = 1e30f;
             try {
-                tt = time_plan<T>(h, p, x, y, e0, e1, s);
+                tt = time_plan<T>(h, p, x, y, e0, e1, s, tbest);
             } catch (...) {
                 free_plan(p);
                 for (ApplyPlan* rest : plans) free_plan(rest);
@@ -2060,6 +2119,7 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
                 free_plan(p);
             }
         }
+        if (!best) throw RtgError{RTG_ERR_ARG, "apply: no plan fits"};
     } catch (...) {
         free_plan(best);
         if (par) free_parity(par);
@@ -2134,14 +2194,15 @@ int apply_tuning(rtg_handle* h, int32_t* out, int cap_rows, cudaStream_t s) {
 }
 
 int apply_status(rtg_handle* h, cudaStream_t s) {
-    const ApplyPlan* p = h->plan32;
     if (h->poisoned) return RTG_ERR_TIMEOUT;
-    if (!p || !p->ntc) return RTG_OK;
-    int st = 0;
-    RTG_CUDA(cudaMemcpyAsync(&st, p->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
-    RTG_CUDA(cudaStreamSynchronize(s));
-    if (st) h->poisoned = true;
-    return st ? RTG_ERR_TIMEOUT : RTG_OK;
+    int st[2] = {0, 0};
+    const ApplyPlan* plans[2] = {h->plan32, h->plan64};
+    for (int q = 0; q < 2; ++q)
+        if (plans[q] && plans[q]->tc)
+            RTG_CUDA(cudaMemcpyAsync(&st[q], plan_status(plans[q]), sizeof(int), cudaMemcpyDeviceToHost, s));
+    if ((plans[0] && plans[0]->tc) || (plans[1] && plans[1]->tc)) RTG_CUDA(cudaStreamSynchronize(s));
+    if (st[0] || st[1]) h->poisoned = true;
+    return h->poisoned ? RTG_ERR_TIMEOUT : RTG_OK;
 }
 
 void free_apply_plans(rtg_handle* h) {

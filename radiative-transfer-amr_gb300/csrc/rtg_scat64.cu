@@ -1,0 +1,779 @@
+// FP64 scattering product on the tensor cores.
+//
+// Y[R][ij] = sum_c W[R][c] x[c][ij] over a column's angular nodes is the dense
+// contraction of the FP64 apply, and GB300 runs FP64 at 2 FMAs per SM and
+// clock: on the FP64 pipe the product took 3.3 of the 4.07 ms of an apply at
+// 7.95e6 DOF.  Here every operand is a sum of eight signed 8-bit digits (the
+// splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012, with
+// fixed-point digits): a row of W and a node's line of x are scaled by the
+// power of two of their largest entry to 62-bit fixed point, whose balanced
+// digits d_1 .. d_8 (|d_1| <= 64, |d_k| <= 128) are exact in FP16.  A digit
+// product is an integer below 2^14, and D_s = sum over i + j = s of W_i x_j, s =
+// 2 .. 9, accumulates in FP32 in tensor memory without rounding: with at most
+// 256 angular nodes |D_s| <= 2^24 for s <= 6, and D_7 .. D_9 (whose bound is
+// 2^24.8, reached by no sum of random digits) stand 2^40 and more below D_2.
+// The terms left out (s >= 10, and W and x below 2^-62 of their row's or node's
+// largest entry) are below 2^-58 of |W|_max |x|_max, finer than the rounding of
+// an FP64 sum.  The epilogue adds the eight integers in 64 bits.
+//
+// Drop rule (rt/preconditioner_matrix.py:450-495): a node of class 2 keeps the
+// terms with |W| >= t.  Where all nodes of a CTA drop all of a block of 16 rows
+// and 16 angular nodes, the block's digits are cleared before they are
+// multiplied.  The dropped terms of the other blocks are in the product; they
+// are summed by the CUDA cores while the tensor cores run and subtracted: each
+// is below 1e-14 / |cw|, and their sum, in FP32 over 8 terms and in pairs of FP32
+// beyond, is off by about 2^-26 of itself.  The test |W| < t runs on FP32
+// copies; the thresholds are moved at set-up to where the rounded test decides
+// as the exact one.  Nodes for which none does (two W entries of one FP32 value
+// on both sides of t), nodes with a non-finite x and nodes with max |x| outside
+// [2^-923, 2^977] are summed term by term in FP64.
+//
+// One CTA takes up to 128 rows and 32 nodes of a column: 8 accumulators of 32
+// columns fill half of the tensor memory, so two CTAs share an SM and one
+// stages while the other multiplies.  B holds the digits of x stacked along N
+// (row 32 (j - 1) + n), so that one tcgen05.mma multiplies W_i with x_1 ..
+// x_{9-i} into D_{i+1} .. D_9, which lie next to each other: 8 instructions per 16
+// angular nodes in place of 36.
+#include <algorithm>
+#include <cstring>
+#include <map>
+#include <vector>
+
+#include "rtg_apply_common.cuh"
+#include "rtg_scat64.h"
+
+namespace rtg {
+
+namespace {
+
+constexpr int kOzThreads = 256;
+constexpr int kOzM = 128;        // rows of a CTA (TMEM lanes)
+constexpr int kOzN = 32;         // nodes of a CTA, at most
+constexpr int kOzK = 16;         // angular nodes per stage: one tcgen05.mma step
+constexpr int kOzD = 8;          // digits
+constexpr int kOzMaxNth = 256;   // angular nodes a column may have (bound of the FP32 sums)
+constexpr int kDigBytes = kOzD * kOzK * 2;            // digits of a row of W per stage
+constexpr int kRowBytes = kDigBytes + kOzK * 4;       // and its FP32 copy
+constexpr int kABytes = kOzM * kRowBytes;
+constexpr int kBBytes = kOzD * kOzN * kOzK * 2;
+constexpr int kXfBytes = kOzK * kOzN * 4;
+constexpr int kOzSmem = 2 * (kABytes + kBBytes + kXfBytes) + kOzMaxNth * (int)sizeof(int2);
+
+struct OzItem {
+    int32_t col, row0, rows, n0, nn, drops;   // drops: a node of class 2;  rows row0 .. row0 + rows - 1, nodes perm[n0] .. perm[n0 + nn - 1]
+    int64_t tile;                           // first byte of the row tile's digits of W
+    int64_t wrange;                         // first of the row tile's |W| ranges (per stage, eight groups of 16 rows)
+};
+
+__device__ __forceinline__ uint64_t oz_desc(uint32_t addr) {
+    const uint64_t lbo = 128, sbo = 256;   // canonical K-major, no swizzle: core matrices along K, 8-row groups
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((lbo >> 4) << 16) | ((sbo >> 4) << 32) | (1ull << 46);
+}
+
+__device__ __forceinline__ void oz_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, int acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+
+// Q with v = Q 2^(E - 1084), |Q| < 2^62, for |v| < 2^(E - 1022), E >= 1 (bits below 2^(E - 1084) cut off)
+__device__ __forceinline__ long long oz_fixed(double v, int E) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    int e = (int)(b >> 52) & 0x7FF;
+    unsigned long long m = b & 0xFFFFFFFFFFFFFull;
+    if (e) m |= 1ull << 52;
+    else e = 1;
+    const int sh = E - e;
+    const unsigned long long q = sh < 63 ? (m << 9) >> sh : 0ull;
+    return (long long)b < 0 ? -(long long)q : (long long)q;
+}
+
+// the eight balanced digits of Q, each plus 128, in the bytes of the result (d_1 on top)
+__device__ __forceinline__ unsigned long long oz_digits(long long q) {
+    return ((unsigned long long)q + 0x0080808080808080ull) ^ 0x8000000000000000ull;
+}
+
+// digits k (bytes k of u and w) as FP16, exactly: 1024 + byte - 1152
+__device__ __forceinline__ uint32_t oz_pair(uint32_t u, uint32_t w, int k) {
+    const uint32_t b = (__byte_perm(u, w, ((unsigned)(4 + k) << 8) | (unsigned)k) & 0x00FF00FFu) | 0x64006400u;
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(b), "r"(0x64806480u));
+    return d;
+}
+
+// H 2^32 + L rounded once, for |H| < 2^46 and |L| < 2^50, with two FP64 operations
+// (the pipe takes 16 cycles for each of a warp's): its upper and lower parts
+// are put into the mantissas of 3 2^91 (one unit 2^40) and of 2^52 (one unit 1)
+__device__ __forceinline__ double oz_double(long long H, long long L) {
+    const long long t = ((H & 0xFF) << 32) + L;                  // H 2^32 + L = (H >> 8) 2^40 + t
+    const long long hi = (H >> 8) + (t >> 40), lo = t & 0xFFFFFFFFFFll;
+    const double a = __longlong_as_double(0x45B8000000000000ll + hi);
+    const double b = __longlong_as_double(0x4330000000000000ll | lo);
+    return (a - (0x1.8p92 + 0x1p52)) + b;
+}
+
+// v 2^e for v zero or normal, with v 2^e normal (integer work alone)
+__device__ __forceinline__ double oz_times_pow2(double v, int e) {
+    const int hi = __double2hiint(v);
+    return (hi << 1) ? __hiloint2double(hi + (e << 20), __double2loint(v)) : v;
+}
+
+// 16 f as a double, for f zero or normal (integer work alone)
+__device__ __forceinline__ double oz_widen16(float f) {
+    const uint32_t b = __float_as_uint(f);
+    const uint32_t hi = (b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (900u << 20));
+    return (b << 1) >= 0x01000000u ? __hiloint2double((int)hi, (int)(b << 29)) : 0.;
+}
+
+// 2^e as a double, -1022 <= e <= 1023
+__host__ __device__ __forceinline__ double oz_pow2(int e) {
+    const unsigned long long b = (unsigned long long)(e + 1023) << 52;
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)b);
+#else
+    double d;
+    std::memcpy(&d, &b, 8);
+    return d;
+#endif
+}
+
+// acc += (w0, w1) * x, two FP32 fused multiply-adds
+__device__ __forceinline__ void fma2(unsigned long long& acc, float w0, float w1, unsigned long long x) {
+    asm("{\n\t.reg .b64 w;\n\tmov.b64 w, {%1, %2};\n\tfma.rn.f32x2 %0, w, %3, %0;\n\t}"
+        : "+l"(acc)
+        : "f"(w0), "f"(w1), "l"(x));
+}
+
+// hi + lo += t (two sums side by side): the rounding error of hi + t goes to lo,
+// exactly where |hi| >= |t|
+__device__ __forceinline__ void add_pair(unsigned long long& hi, unsigned long long& lo, unsigned long long t) {
+    asm("{\n\t.reg .b64 s, z, e, m;\n\tmov.b64 m, {%3, %3};\n\t"
+        "add.rn.f32x2 s, %0, %2;\n\t"
+        "fma.rn.f32x2 z, %0, m, s;\n\t"      // z = s - hi
+        "fma.rn.f32x2 e, z, m, %2;\n\t"      // e = t - z
+        "add.rn.f32x2 %1, %1, e;\n\t"
+        "mov.b64 %0, s;\n\t}"
+        : "+l"(hi), "+l"(lo)
+        : "l"(t), "f"(-1.f));
+}
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// Warps 0-7 stage x, sum the corrections and write y; warp 8 brings the digits
+// of W in, one stage ahead, and issues the multiplies.
+__global__ void __launch_bounds__(kOzThreads + 32, 2)
+scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items,
+              const unsigned char* __restrict__ digits, const int* __restrict__ frow,
+              const int64_t* __restrict__ sig_row, const float2* __restrict__ wrange,
+              const uint8_t* __restrict__ perm, const uint64_t* __restrict__ thr, const float* __restrict__ thr32,
+              const double* __restrict__ x, double* __restrict__ y, int* __restrict__ status) {
+    extern __shared__ __align__(128) unsigned char osm[];
+    __shared__ __align__(8) uint64_t s_bar[6];   // W arrived 0, 1; multiplied 0, 1; x staged 0, 1
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort, s_tmax, s_tmin, s_bad, s_need;
+    __shared__ unsigned s_max[kOzN];
+    __shared__ int s_E[kOzN];          // exponent field of the node's largest |x|; 0: node not in the product
+    __shared__ float s_thr[kOzN];
+    __shared__ float2 s_wr[kOzMaxNth / kOzK][8];   // range of |W| per stage and 16 rows
+    __shared__ int s_node[kOzN];       // node in the column
+    __shared__ double s_g[kOzN];       // -cw 2^(E - 1056); 0: nothing to add
+    if (v.stop && *v.stop) return;
+    const OzItem it = items[blockIdx.x];
+    if (v.skip && v.skip[it.col]) return;
+    const ColDev C = v.cols[it.col];
+    const bool mask_rows = flags & RTG_MASK_ROWS;
+    const int nij = C.nx * C.ny, Nth = C.nth_col, ncell = C.elem_end - C.elem_begin;
+    const int np = (it.nn + 7) & ~7;
+    const int tcols = np <= 16 ? 128 : 256;
+    const int rows8 = (it.rows + 7) & ~7;
+    const int nch = (Nth + kOzK - 1) / kOzK;
+    unsigned char* As = osm;
+    unsigned char* Bs = As + 2 * kABytes;
+    float* Xf = reinterpret_cast<float*>(Bs + 2 * kBBytes);   // [2][kOzK][kOzN]
+    float* Cf = reinterpret_cast<float*>(As);                 // after the product: the corrections [2][kOzN][kOzM]
+    // per angular row: DOF offset in the column; nth and, from bit 8, the inflow-boundary faces of its cell
+    int2* s_row = reinterpret_cast<int2*>(Xf + 2 * kOzK * kOzN);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
+    const unsigned char* wsrc = digits + it.tile;
+    // a stage's image: the digits of the rows, then (read where terms are dropped) FP32 W [kOzK][rows8]
+    const uint32_t stage = (uint32_t)rows8 * kRowBytes, dig = (uint32_t)rows8 * kDigBytes;
+    const uint32_t as_addr = (uint32_t)__cvta_generic_to_shared(As);
+    if (tid == 0) {
+        s_abort = 0;
+        s_tmax = 0;
+        s_tmin = 0x7F7FFFFF;
+        s_bad = 0;
+        s_need = 0;
+        for (int q = 0; q < 6; ++q)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8 * q), "r"(q < 4 ? 1 : kOzThreads / 32)
+                         : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // the first stages' digits travel while the tables are made
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        const uint32_t bytes = it.drops ? stage : dig;
+        bulk_load(as_addr, wsrc, bytes, bar);
+        if (nch > 1) bulk_load(as_addr + kABytes, wsrc + stage, bytes, bar + 8);
+    }
+    // node tid's constants (loaded before they are needed)
+    float t_node = 0.f;
+    double cw = 0.;
+    float lo = 3.4e38f;   // smallest |W| of stage tid - 32
+    if (tid < kOzN) {
+        s_max[tid] = 0u;
+        const int ij = perm[it.n0 + min(tid, it.nn - 1)];   // the pad nodes repeat the last (their x is zero)
+        s_node[tid] = ij;
+        t_node = thr32[C.node_off + ij];
+        cw = v.colc[it.col] * v.sw[C.node_off + ij];
+    } else if (tid - 32 < nch) {
+        for (int q = 0; q < 8; ++q) {
+            const float2 w = wrange[it.wrange + 8 * (tid - 32) + q];
+            s_wr[tid - 32][q] = w;
+            lo = fminf(lo, w.x);
+        }
+    }
+    if (warp == 8) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s_tmem);
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(tcols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    // the column's rows, and per node the largest |x| (a lane takes a node)
+    const double* xc = x + C.dof_off;
+    for (int k = warp; k < ncell; k += kOzThreads / 32 + 1) {
+        const ElemDev E = v.elems[C.elem_begin + k];
+        const int off = nij * E.row;
+        for (int r = lane; r < E.nth; r += 32) s_row[E.row + r] = make_int2(off + r, E.nth | (E.flags >> 4) << 8);
+        if (lane < it.nn) {
+            const double* xk = xc + off + s_node[lane] * E.nth;
+            unsigned mx = 0;
+#pragma unroll 4
+            for (int r = 0; r < E.nth; ++r) {
+                const double xv = xk[r];
+                const unsigned hi = (unsigned)__double2hiint(xv) & 0x7FFFFFFFu;
+                mx = max(mx, hi ? hi : (__double2loint(xv) ? 1u : 0u));
+            }
+            atomicMax(&s_max[lane], mx);
+        }
+    }
+    __syncthreads();
+    if (tid < kOzN) {
+        int E = 0;
+        double g = 0.;
+        float t = t_node;
+        if (tid < it.nn) {
+            const unsigned mx = s_max[tid];
+            const int e = (int)(mx >> 20);
+            if (e < 100 || e > 2000 || t != t) {
+                g = mx ? -cw : 0.;          // summed term by term below, or x is zero
+                if (mx) s_bad = 1;
+                if (mx || t != t) t = 0.f;
+            } else {
+                E = e;
+                g = -cw * oz_pow2(e - 1056);
+                atomicMax(&s_tmax, __float_as_int(t));
+                atomicMin(&s_tmin, __float_as_int(t));
+            }
+        }
+        s_E[tid] = E;
+        s_g[tid] = g;
+        s_thr[tid] = t;
+    }
+    __syncthreads();
+    // largest and smallest threshold of the CTA's nodes (0: nothing is dropped)
+    const float tmax = __int_as_float(s_tmax), tmin = __int_as_float(s_tmin);
+    if (tmax > 0.f) {
+        // the stages in which some |W| may be dropped
+        if (lo < tmax) atomicOr(&s_need, 1 << (tid - 32));
+        __syncthreads();
+    }
+    const int needs = s_need;
+    // correction tile of the thread: rows 16 warp + 4 (lane % 4) .., nodes 4 (lane / 4) ..
+    // (two nodes side by side; the sum is corr + cerr)
+    unsigned long long corr[4][2] = {}, cerr[4][2] = {};
+    bool ok = true;
+    if (warp == 8) {
+        // kind::f16: D F32 (bits 4-5 = 1), A and B FP16 (bits 7-9, 10-12 = 0), K-major, N >> 3 at bit 17, M >> 4 at 24
+        const uint32_t idesc0 = (1u << 4) | ((uint32_t)(kOzM >> 4) << 24);
+        if (lane == 0) {
+            for (int ch = 0; ch < nch && ok; ++ch) {
+                const int b = ch & 1;
+                const uint32_t par = (uint32_t)((ch >> 1) & 1);
+                ok = mbar_wait(bar + 32 + 8 * b, par) && mbar_wait(bar + 8 * b, par);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t aa = as_addr + b * kABytes;
+                const uint64_t db = oz_desc((uint32_t)__cvta_generic_to_shared(Bs + b * kBBytes));
+#pragma unroll
+                for (int i = 0; i < kOzD; ++i) {
+                    const uint32_t n = (uint32_t)(((kOzD - i) * np + 15) & ~15);   // columns past D_9 are not read
+                    oz_mma(tmem + (uint32_t)(i * np), oz_desc(aa + (uint32_t)(i * rows8 * 32)), db,
+                           idesc0 | ((n >> 3) << 17), ch > 0 || i > 0);
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                 bar + 16 + 8 * b)
+                             : "memory");
+                // stage ch - 1 multiplied: its W buffer takes stage ch + 1 (0 and 1 are on their way)
+                if (ch >= 1 && ch + 1 < nch) {
+                    ok = mbar_wait(bar + 16 + 8 * (b ^ 1), (uint32_t)(((ch - 1) >> 1) & 1));
+                    if (ok)
+                        bulk_load(as_addr + (b ^ 1) * kABytes, wsrc + (int64_t)(ch + 1) * stage,
+                                  needs >> (ch + 1) & 1 ? stage : dig, bar + 8 * (b ^ 1));
+                }
+            }
+            if (!ok) s_abort = 1;
+        }
+        __syncwarp();
+    } else {
+        // thread -> (two angular nodes, one node): eight digits of each into B
+        const int kp = 8 * (warp & 1) + 2 * (lane & 3), nb = 8 * (warp >> 1) + (lane >> 2);
+        const bool bact = nb < np;
+        const int En = bact ? s_E[nb] : 0, ijn = s_node[nb & (kOzN - 1)];
+        auto load_x = [&](int c) -> double {
+            if (!En || c >= Nth) return 0.;
+            const int2 ro = s_row[c];
+            return xc[ro.x + ijn * (ro.y & 0xFF)];
+        };
+        const uint32_t boff = (uint32_t)((nb >> 3) * 256 + (kp >> 3) * 128 + (nb & 7) * 16 + (kp & 7) * 2);
+        float th[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) th[j] = s_thr[4 * (lane >> 2) + j];
+        // nodes are in the order of their thresholds, of which a column has few (four nodes
+        // of a symmetric rule share one): one test for the four nodes of every thread
+        const bool same = __all_sync(0xffffffffu, th[0] == th[1] && th[0] == th[2] && th[0] == th[3]);
+        double x0 = load_x(kp), x1 = load_x(kp + 1);
+        for (int ch = 0; ch < nch; ++ch) {
+            const int b = ch & 1, c0 = ch * kOzK;
+            unsigned char* Bb = Bs + b * kBBytes;
+            float* Xb = Xf + b * kOzK * kOzN;
+            const bool need = needs >> ch & 1;
+            // stage ch - 2 has been multiplied: its buffers are free
+            if (ch >= 2 && !mbar_wait(bar + 16 + 8 * b, (uint32_t)(((ch >> 1) - 1) & 1))) {
+                s_abort = 1;
+                ok = false;
+            }
+            if (bact) {
+                const long long q0 = En ? oz_fixed(x0, En) : 0ll, q1 = En ? oz_fixed(x1, En) : 0ll;
+                const unsigned long long u0 = oz_digits(q0), u1 = oz_digits(q1);
+                const uint32_t h0 = (uint32_t)(u0 >> 32), l0 = (uint32_t)u0, h1 = (uint32_t)(u1 >> 32), l1 = (uint32_t)u1;
+#pragma unroll
+                for (int j = 0; j < kOzD; ++j)
+                    *reinterpret_cast<uint32_t*>(Bb + boff + j * np * 32) =
+                        j < 4 ? oz_pair(h0, h1, 3 - j) : oz_pair(l0, l1, 7 - j);
+                if (need) {
+                    // x in units of 2^(E - 1052) for the corrections
+                    Xb[kp * kOzN + nb] = (float)(int)(q0 >> 32);
+                    Xb[(kp + 1) * kOzN + nb] = (float)(int)(q1 >> 32);
+                }
+            }
+            // a block of which every node drops every term is taken out of the product
+            const float2 wr = s_wr[ch][warp];   // smallest and largest |W| of the warp's 16 rows
+            if (need && 16 * warp < rows8 && wr.y < tmin) {
+                ok = mbar_wait(bar + 8 * b, (uint32_t)((ch >> 1) & 1)) && ok;
+                if (16 * lane < min(512, rows8 * 32 - 512 * warp))
+#pragma unroll
+                    for (int k = 0; k < kOzD; ++k)
+                        *reinterpret_cast<uint4*>(As + b * kABytes + k * rows8 * 32 + 512 * warp + 16 * lane) =
+                            make_uint4(0u, 0u, 0u, 0u);
+            }
+            // generic-proxy writes -> visible to the tensor cores
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar + 32 + 8 * b) : "memory");
+            x0 = load_x(c0 + kOzK + kp);
+            x1 = load_x(c0 + kOzK + kp + 1);
+            if (needs == 0) continue;
+            // every warp has staged x (and is done with the stage before)
+            const uint32_t par = (uint32_t)((ch >> 1) & 1);
+            ok = mbar_wait(bar + 32 + 8 * b, par) && ok;
+            if (!need || 16 * warp >= it.rows) continue;
+            if (wr.x >= tmax || wr.y < tmin) continue;
+            ok = mbar_wait(bar + 8 * b, par) && ok;
+            const float* wp = reinterpret_cast<const float*>(As + b * kABytes + dig) + 16 * warp + 4 * (lane & 3);
+            const float* xp = Xb + 4 * (lane >> 2);
+#pragma unroll
+            for (int c8 = 0; c8 < kOzK; c8 += 8) {
+                unsigned long long part[4][2] = {};
+                if (same) {
+#pragma unroll 4
+                    for (int c = c8; c < c8 + 8; ++c) {
+                        const float4 w4 = *reinterpret_cast<const float4*>(wp + c * rows8);
+                        const ulonglong2 x4 = *reinterpret_cast<const ulonglong2*>(xp + c * kOzN);
+                        const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float w = fabsf(wv[i]) < th[0] ? wv[i] : 0.f;
+                            fma2(part[i][0], w, w, x4.x);
+                            fma2(part[i][1], w, w, x4.y);
+                        }
+                    }
+                } else {
+#pragma unroll 2
+                    for (int c = c8; c < c8 + 8; ++c) {
+                        const float4 w4 = *reinterpret_cast<const float4*>(wp + c * rows8);
+                        const ulonglong2 x4 = *reinterpret_cast<const ulonglong2*>(xp + c * kOzN);
+                        const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float a = fabsf(wv[i]);
+                            fma2(part[i][0], a < th[0] ? wv[i] : 0.f, a < th[1] ? wv[i] : 0.f, x4.x);
+                            fma2(part[i][1], a < th[2] ? wv[i] : 0.f, a < th[3] ? wv[i] : 0.f, x4.y);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    add_pair(corr[i][0], cerr[i][0], part[i][0]);
+                    add_pair(corr[i][1], cerr[i][1], part[i][1]);
+                }
+            }
+        }
+        if (!ok) s_abort = 1;
+    }
+    // the last commit follows every multiply of the CTA
+    if (ok && !mbar_wait(bar + 16 + 8 * ((nch - 1) & 1), (uint32_t)(((nch - 1) >> 1) & 1))) s_abort = 1;
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (s_abort) {
+        // give the copies and multiplies in flight one more bounded wait each before the memory is let go
+        for (int q = 0; q < 2; ++q) {
+            mbar_wait(bar + 8 * q, 0);
+            mbar_wait(bar + 16 + 8 * q, 0);
+        }
+        if (tid == 0 && status) atomicExch(status, RTG_ERR_TIMEOUT);
+    } else {
+        // corrections to [node][row] (the buffers are free)
+        if (needs && warp < 8) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float* o = Cf + (4 * (lane >> 2) + j) * kOzM + 16 * warp + 4 * (lane & 3);
+                float hi[4], lo[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    hi[i] = __uint_as_float((uint32_t)(corr[i][j >> 1] >> (32 * (j & 1))));
+                    lo[i] = __uint_as_float((uint32_t)(cerr[i][j >> 1] >> (32 * (j & 1))));
+                }
+                *reinterpret_cast<float4*>(o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<float4*>(o + kOzN * kOzM) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+            }
+        }
+        __syncthreads();
+        const int q = warp & 3, h = warp >> 2;
+        const int m = 32 * q + lane, R = it.row0 + m;
+        const bool valid = warp < 8 && m < it.rows;
+        const int2 ro = s_row[valid ? R : it.row0];
+        const int fr = valid ? frow[sig_row[C.sig] + R] : 0;
+        const int nth = ro.y & 0xFF, bm = mask_rows ? ro.y >> 8 : 0;
+        const float rny = __frcp_rn((float)C.ny);
+        // rows of inflow-boundary nodes stay zero under RTG_MASK_ROWS
+        auto masked = [&](int ij) {
+            const int i = small_div(ij, rny);
+            return bm && bdry_node(bm, i, ij - i * C.ny, C.nx, C.ny);
+        };
+        double* yc = y + C.dof_off + ro.x;
+        for (int cb = 4 * h; cb < np && warp < 8; cb += 8) {
+            uint32_t d[kOzD][4];
+#pragma unroll
+            for (int k = 0; k < kOzD; ++k)
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(d[k][0]), "=r"(d[k][1]), "=r"(d[k][2]), "=r"(d[k][3])
+                             : "r"(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(k * np + cb))
+                             : "memory");
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (!valid) continue;
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj) {
+                const int n = cb + jj;
+                if (n >= it.nn || !s_E[n]) continue;
+                const int ij = s_node[n];
+                if (masked(ij)) continue;
+                long long H = 0, L = 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    H = (H << 8) + __float2int_rn(__uint_as_float(d[k][jj]));
+                    L = (L << 8) + __float2int_rn(__uint_as_float(d[k + 4][jj]));
+                }
+                double s = oz_times_pow2(oz_double(H, L), fr);
+                if (needs) s -= oz_widen16(Cf[n * kOzM + m]) + oz_widen16(Cf[(kOzN + n) * kOzM + m]);
+                atomicAdd(yc + ij * nth, s * s_g[n]);
+            }
+        }
+        if (s_bad && valid && h == 0) {
+            // nodes left out of the product: kept terms one by one (the bits of |W| against the threshold)
+            const double* Wr = v.W + v.W_off[C.sig] + (int64_t)R * Nth;
+            for (int n = 0; n < it.nn; ++n) {
+                if (s_E[n] || s_g[n] == 0.) continue;
+                const int ij = s_node[n];
+                if (masked(ij)) continue;
+                const unsigned long long tb = thr[C.node_off + ij];
+                double s = 0.;
+                for (int c = 0; c < Nth; ++c) {
+                    const unsigned long long wb = (unsigned long long)__double_as_longlong(Wr[c]);
+                    const bool keep = c != R && (wb & 0x7FFFFFFFFFFFFFFFull) >= tb;
+                    const int2 rc = s_row[c];
+                    s = fma(keep ? Wr[c] : 0., xc[rc.x + ij * (rc.y & 0xFF)], s);
+                }
+                atomicAdd(yc + ij * nth, s * s_g[n]);
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 8) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols) : "memory");
+    }
+}
+
+// One block per row of a distinct W: its digits into the row tile's image (per
+// stage of kOzK columns: digit, 8-row group, 8-column group, row, column), its
+// scale, and the range of the nonzero off-diagonal |W| per stage and 16 rows.  bad: an entry is not
+// finite, or the row's largest is outside [2^-100, 2^100].
+__global__ void oz_digits_kernel(const double* __restrict__ W, const float* __restrict__ W32,
+                                 const int64_t* __restrict__ W_off, const int2* __restrict__ rows,
+                                 const int64_t* __restrict__ sig_tile, const int64_t* __restrict__ sig_wrange,
+                                 const int32_t* __restrict__ sig_n, unsigned char* __restrict__ out,
+                                 int* __restrict__ frow, float2* __restrict__ wrange, int* __restrict__ bad) {
+    __shared__ unsigned long long s_mx[4];
+    const int sg = rows[blockIdx.x].x, R = rows[blockIdx.x].y, n = sig_n[sg];
+    const double* w = W + W_off[sg] + (int64_t)R * n;
+    unsigned long long mx = 0;
+    for (int c = threadIdx.x; c < n; c += blockDim.x)
+        if (c != R) mx = max(mx, (unsigned long long)__double_as_longlong(w[c]) & 0x7FFFFFFFFFFFFFFFull);
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) s_mx[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    for (int q = 0; q < (int)blockDim.x / 32; ++q) mx = max(mx, s_mx[q]);
+    const int E = (int)(mx >> 52);
+    const bool ok = mx == 0 || (E >= 923 && E <= 1123);
+    if (threadIdx.x == 0) {
+        if (!ok) atomicExch(bad, 1);
+        frow[blockIdx.x] = ok && mx ? E - 1056 : 0;
+    }
+    if (!ok || !mx) return;   // the digits stay zero
+    const int mt = R / kOzM, rr = R % kOzM, nch = (n + kOzK - 1) / kOzK;
+    const int rows8 = (min(kOzM, n - mt * kOzM) + 7) & ~7;
+    unsigned char* tile = out + sig_tile[sg] + (int64_t)mt * nch * kOzM * kRowBytes;
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
+        if (c == R) continue;
+        const unsigned long long u = oz_digits(oz_fixed(w[c], E));
+        unsigned char* st = tile + (int64_t)(c / kOzK) * rows8 * kRowBytes;
+        unsigned char* p = st + (rr >> 3) * 256 + ((c % kOzK) >> 3) * 128 + (rr & 7) * 16 + (c & 7) * 2;
+        for (int k = 0; k < kOzD; ++k)
+            *reinterpret_cast<uint16_t*>(p + k * rows8 * kOzK * 2) =
+                (uint16_t)oz_pair(k < 4 ? (uint32_t)(u >> 32) : (uint32_t)u, 0u, 3 - (k & 3));
+        const float w32 = W32[W_off[sg] + (int64_t)R * n + c];
+        reinterpret_cast<float*>(st + rows8 * kDigBytes)[(c % kOzK) * rows8 + rr] = w32;
+        const float a = fabsf(w32);
+        if (a > 0.f) {
+            float2* wr = wrange + sig_wrange[sg] + 8 * ((int64_t)mt * nch + c / kOzK) + (rr >> 4);
+            atomicMin(reinterpret_cast<int*>(&wr->x), __float_as_int(a));
+            atomicMax(reinterpret_cast<int*>(&wr->y), __float_as_int(a));
+        }
+    }
+}
+
+// One block per class-2 node: the FP32 threshold that decides |W| >= t as the
+// FP64 one does (rounding to FP32 is monotone, so only W that round to the
+// same value as t are in doubt); NaN when W of that value lie on both sides.
+__global__ void oz_threshold_kernel(const double* __restrict__ W, const int64_t* __restrict__ W_off,
+                                    const int32_t* __restrict__ sig_n, const int2* __restrict__ nodes,
+                                    const uint64_t* __restrict__ thr, float* __restrict__ thr32) {
+    const int node = nodes[blockIdx.x].x, sg = nodes[blockIdx.x].y, n = sig_n[sg];
+    const double t = __longlong_as_double((long long)thr[node]);
+    const float f = (float)t;
+    const double* w = W + W_off[sg];
+    bool lo = false, hi = false;
+    for (int64_t q = threadIdx.x; q < (int64_t)n * n; q += blockDim.x) {
+        const double a = fabs(w[q]);
+        if ((float)a != f || q % (n + 1) == 0) continue;   // the diagonal is not tested
+        if (a < t) lo = true;
+        else hi = true;
+    }
+    const int any_lo = __syncthreads_or(lo), any_hi = __syncthreads_or(hi);
+    if (threadIdx.x == 0)
+        thr32[node] = any_lo ? (any_hi ? __int_as_float(0x7FC00000) : __int_as_float(__float_as_int(f) + 1)) : f;
+}
+
+}  // namespace
+
+struct Scat64 {
+    OzItem* d_items = nullptr;
+    int nitems = 0;
+    unsigned char* d_digits = nullptr;
+    int* d_frow = nullptr;   // per row: exponent of its scale
+    int64_t* d_sig_row = nullptr;
+    float2* d_wrange = nullptr;
+    float* d_thr32 = nullptr;
+    uint8_t* d_perm = nullptr;
+    const uint64_t* d_thr = nullptr;
+    int* d_status = nullptr;
+    std::vector<void*> allocs;
+};
+
+bool scat64_fits(const ColDev& C) { return C.nth_col <= kOzMaxNth; }
+
+Scat64* build_scat64(const rtg_handle* h, const std::vector<char>& cols, const uint8_t* scls, const uint64_t* thr,
+                     const uint64_t* d_thr) {
+    const HostTables& t = h->host;
+    const int nsig = (int)t.sig_nth.size();
+    std::vector<char> used(nsig, 0);
+    for (size_t c = 0; c < cols.size(); ++c)
+        if (cols[c]) used[t.cols[c].sig] = 1;
+    std::vector<int64_t> sig_tile(nsig, 0), sig_wrange(nsig, 0), sig_row(nsig, 0);
+    std::vector<int2> rows;
+    int64_t bytes = 0, nw = 0;
+    for (int s = 0; s < nsig; ++s) {
+        if (!used[s]) continue;
+        const int n = t.sig_nth[s], nch = (n + kOzK - 1) / kOzK;
+        sig_tile[s] = bytes;
+        sig_wrange[s] = nw;
+        sig_row[s] = (int64_t)rows.size();
+        for (int r = 0; r < n; ++r) rows.push_back(make_int2(s, r));
+        for (int r0 = 0; r0 < n; r0 += kOzM) {
+            bytes += (int64_t)((std::min(kOzM, n - r0) + 7) & ~7) * nch * kRowBytes;
+            nw += 8 * nch;
+        }
+    }
+    std::vector<OzItem> items;
+    std::vector<int2> nodes;
+    std::vector<uint8_t> perm;
+    std::vector<int64_t> cost(nsig, 0);
+    for (int ci = 0; ci < (int)t.cols.size(); ++ci) {
+        if (!cols[ci]) continue;
+        const ColDev& C = t.cols[ci];
+        const int nij = C.nx * C.ny, nch = (C.nth_col + kOzK - 1) / kOzK;
+        // the nodes whose product is used, by threshold, those of thresholds
+        // shared by 4, 8, .. nodes first: the kernel tests four nodes at once
+        std::vector<uint8_t> ord;
+        std::map<float, int> share;
+        auto thr_f = [&](int q) {
+            double t;
+            std::memcpy(&t, &thr[C.node_off + q], 8);
+            return (float)t;
+        };
+        for (int q = 0; q < nij; ++q) {
+            const uint8_t cls = scls[C.node_off + q];
+            if (cls == 1 || cls == 2) {
+                ord.push_back((uint8_t)q);
+                ++share[thr_f(q)];
+            }
+            if (cls == 2) nodes.push_back(make_int2(C.node_off + q, C.sig));
+        }
+        std::stable_sort(ord.begin(), ord.end(), [&](uint8_t a, uint8_t b) {
+            const float ta = thr_f(a), tb = thr_f(b);
+            const bool ra = share[ta] % 4 != 0, rb = share[tb] % 4 != 0;
+            return ra != rb ? rb : ta < tb;
+        });
+        const int na = (int)ord.size(), ntl = (na + kOzN - 1) / kOzN;
+        const int per = ntl ? ((na + ntl - 1) / ntl + 3) & ~3 : 4, p0 = (int)perm.size();
+        perm.insert(perm.end(), ord.begin(), ord.end());
+        for (int n0 = 0; n0 < na; n0 += per) {
+            const int nn = std::min(per, na - n0);
+            int drops = 0;
+            for (int q = n0; q < n0 + nn; ++q) drops |= scls[C.node_off + ord[q]] == 2;
+            for (int r0 = 0; r0 < C.nth_col; r0 += kOzM) {
+                const int mt = r0 / kOzM;
+                items.push_back(OzItem{ci, r0, std::min(kOzM, C.nth_col - r0), p0 + n0, nn, drops,
+                                       sig_tile[C.sig] + (int64_t)mt * nch * kOzM * kRowBytes,
+                                       sig_wrange[C.sig] + 8 * (int64_t)mt * nch});
+                cost[C.sig] += (int64_t)nch * kOzM;
+            }
+        }
+    }
+    // the CTAs that read one row tile run next to each other, so that its
+    // digits come from L2 after the first
+    std::stable_sort(items.begin(), items.end(), [&](const OzItem& a, const OzItem& b) {
+        const int sa = t.cols[a.col].sig, sb = t.cols[b.col].sig;
+        if (cost[sa] != cost[sb]) return cost[sa] > cost[sb];
+        if (sa != sb) return sa < sb;
+        return a.row0 < b.row0;
+    });
+    Scat64* p = new Scat64();
+    try {
+        auto alloc = [&](size_t n) -> void* {
+            void* d = nullptr;
+            RTG_CUDA(cudaMalloc(&d, std::max<size_t>(n, 16)));
+            p->allocs.push_back(d);
+            return d;
+        };
+        auto up = [&](const void* src, size_t n) -> void* {
+            void* d = alloc(n);
+            if (n) RTG_CUDA(cudaMemcpy(d, src, n, cudaMemcpyHostToDevice));
+            return d;
+        };
+        p->nitems = (int)items.size();
+        p->d_items = (OzItem*)up(items.data(), sizeof(OzItem) * items.size());
+        p->d_digits = (unsigned char*)alloc((size_t)bytes);
+        p->d_frow = (int*)alloc(sizeof(int) * rows.size());
+        p->d_sig_row = (int64_t*)up(sig_row.data(), sizeof(int64_t) * nsig);
+        p->d_wrange = (float2*)alloc(sizeof(float2) * (size_t)nw);
+        p->d_thr32 = (float*)alloc(sizeof(float) * std::max<size_t>((size_t)t.nnodes, 1));
+        p->d_status = (int*)alloc(sizeof(int));
+        p->d_perm = (uint8_t*)up(perm.data(), perm.size());
+        p->d_thr = d_thr;
+        int2* d_rows = (int2*)up(rows.data(), sizeof(int2) * rows.size());
+        int2* d_nodes = (int2*)up(nodes.data(), sizeof(int2) * nodes.size());
+        int64_t* d_st = (int64_t*)up(sig_tile.data(), sizeof(int64_t) * nsig);
+        int64_t* d_sw = (int64_t*)up(sig_wrange.data(), sizeof(int64_t) * nsig);
+        int32_t* d_n = (int32_t*)up(t.sig_nth.data(), sizeof(int32_t) * nsig);
+        int* d_bad = (int*)alloc(sizeof(int));
+        RTG_CUDA(cudaMemset(p->d_status, 0, sizeof(int)));
+        RTG_CUDA(cudaMemset(d_bad, 0, sizeof(int)));
+        RTG_CUDA(cudaMemset(p->d_digits, 0, (size_t)bytes));
+        const std::vector<float2> none((size_t)nw, make_float2(3.4e38f, 0.f));
+        RTG_CUDA(cudaMemcpy(p->d_wrange, none.data(), sizeof(float2) * (size_t)nw, cudaMemcpyHostToDevice));
+        RTG_CUDA(cudaMemset(p->d_thr32, 0, sizeof(float) * (size_t)t.nnodes));
+        if (!rows.empty()) {
+            oz_digits_kernel<<<(int)rows.size(), 128>>>(h->v64.W, h->v32.W, h->v64.W_off, d_rows, d_st, d_sw, d_n,
+                                                        p->d_digits, p->d_frow, p->d_wrange, d_bad), count_launch();
+            RTG_LAUNCHED("oz_digits_kernel");
+        }
+        if (!nodes.empty()) {
+            oz_threshold_kernel<<<(int)nodes.size(), 256>>>(h->v64.W, h->v64.W_off, d_n, d_nodes, d_thr, p->d_thr32),
+                count_launch();
+            RTG_LAUNCHED("oz_threshold_kernel");
+        }
+        int bad = 0;
+        RTG_CUDA(cudaMemcpy(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost));
+        if (bad) {
+            free_scat64(p);
+            return nullptr;
+        }
+        raise_smem_limit((const void*)scat64_kernel, kOzSmem);
+    } catch (...) {
+        free_scat64(p);
+        throw;
+    }
+    return p;
+}
+
+void free_scat64(Scat64* p) {
+    if (!p) return;
+    for (void* d : p->allocs) cudaFree(d);
+    delete p;
+}
+
+void launch_scat64(const Scat64* p, const OpView<double>& v, uint32_t flags, const double* x,
+                   double* y, cudaStream_t s) {
+    if (!p->nitems) return;
+    scat64_kernel<<<p->nitems, kOzThreads + 32, kOzSmem, s>>>(v, flags, p->d_items, p->d_digits, p->d_frow,
+                                                         p->d_sig_row, p->d_wrange, p->d_perm, p->d_thr, p->d_thr32, x,
+                                                         y, p->d_status), count_launch();
+    RTG_LAUNCHED("scat64_kernel");
+}
+
+int* scat64_status(const Scat64* p) { return p->d_status; }
+
+}  // namespace rtg

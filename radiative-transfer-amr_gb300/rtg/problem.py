@@ -277,7 +277,10 @@ class DeviceOperator:
         out = None
         for f, c in terms.items():
             t = self.ctx.apply(f, x, prec=prec)
-            out = t.mul_(c) if out is None else out.add_(t, alpha=c)
+            if out is None:
+                out = t if c == 1. else t.mul_(c)
+            else:
+                out.add_(t, alpha=c)
         if out is None:
             out = torch.zeros(self.ctx.N, dtype=torch.float64, device=self.ctx.device)
         if y is not None:
