@@ -17,10 +17,10 @@
 // couplings that close it are dropped from P.  One persistent launch applies
 // P^{-1}: CTAs take elements in level order and wait on the upwind values
 // themselves (z is filled with a sentinel first).  An element whose upwind
-// map G_e = -B_e C_e (built once, FP64 with an FP32 copy) fits in shared
-// memory computes z_e = B_e rin_e + G_e z_upwind in one phase after its
-// inputs arrive; the others form the face couplings in factorised form
-// (T = Et z, c = Es T) and apply the face columns of B_e.
+// map G_e = -B_e C_e (built once, FP64 with a BF16 copy) fits in shared
+// memory computes z_e = B_e rin_e + G_e w in one phase after its inputs arrive
+// (w the upwind values, see the maps below); the others form the face couplings
+// in factorised form (T = Et z, c = Es T) and apply the face columns of B_e.
 // Applying P^{-1} is exact for the transport part of an acyclic mesh; the
 // cross-cell scattering is left to the Krylov iteration.
 #include <algorithm>
@@ -43,14 +43,26 @@ constexpr int kSweepThreads = 256;
 constexpr size_t kSweepSmemBudget = 110 * 1024;  // rhs + prefetched block inverse (2 CTAs per SM)
 constexpr size_t kSweepSmemSmall = 72 * 1024;    // the alternatives the first sweep also times (3 CTAs per SM)
 constexpr size_t kSweepSmemTiny = 54 * 1024;     // ... and 4 CTAs per SM (the register limit): more copies in flight
-constexpr int kSweepShapes = 5;
+constexpr int kSweepShapes = 7;
 // the shapes the first sweep times: (threads per CTA, shared-memory budget);
-// the 128-thread CTAs fit 6 or 8 per SM, each staging one element
-constexpr int kShapeThreads[kSweepShapes] = {kSweepThreads, kSweepThreads, kSweepThreads, 128, 128};
+// the 128-thread CTAs fit 6 or 8 per SM, each staging one element.  The last
+// two take the FP64 sweep's elements two angular nodes at a time (split lists):
+// an item's multiply-adds run at two a clock on its SM's FP64 pipe, and on
+// meshes of few elements per level the other SMs are idle meanwhile (218,581
+// DOF: 3,100 of the 4,500 cycles of a level)
+constexpr int kShapeThreads[kSweepShapes] = {kSweepThreads, kSweepThreads, kSweepThreads, 128, 128, 128, 128};
 constexpr size_t kShapeBudget[kSweepShapes] = {kSweepSmemBudget, kSweepSmemSmall, kSweepSmemTiny, 36 * 1024,
-                                               27 * 1024};
+                                               27 * 1024, 54 * 1024, 36 * 1024};
+constexpr int kWholeShapes = 5;                 // shapes of whole elements
+constexpr size_t kSplitBudget = 36 * 1024;      // the smallest of the split shapes: every part fits it
+constexpr int kSplitNth = 2;                    // angular nodes of a part (even: parts of a block inverse start on 16 bytes)
 constexpr int kMaxCplStaged = 32;               // active couplings staged per element
 constexpr int kMaxBlock = 100;  // nx*ny supported by the element-block inverse
+// elements per level below which the FP32 sweep's maps have Et folded in (see
+// the upwind maps): at 42 per level (218,581 DOF) a sweep takes 72 us folded and 80
+// with T, at 217 (1.95e6 DOF) 136 and 118, at 282 (7.95e6 DOF) 505 and 450; about one
+// per SM lies between
+constexpr int kFoldElems = 128;
 
 __device__ __forceinline__ int gofs_s(int n) { return (n - 1) * n * (2 * n - 1) / 6; }
 
@@ -220,17 +232,21 @@ constexpr int kRecNf = 11;      // face nodes with active couplings
 constexpr int kRecCplB = 12, kRecCplE = 13;   // the element's couplings (all of them)
 constexpr int kRecOk = 14;      // one-phase path: bit 0 FP32, bit 1 FP64
 constexpr int kRecReg = 15;     // one-phase staged region in values, FP32 then FP64
-constexpr int kRecNup = 17;     // upwind values of the one-phase map
+constexpr int kRecNup = 17;     // one-phase map: columns of couplings with diagonal angular mortars,
 constexpr int kRecGoff = 18;    // map offset, FP32 (two words) then FP64 (two words)
 constexpr int kRecUoff = 22;    // upwind index list offset (two words)
 constexpr int kRecDirect = 24;  // 1: every staged coupling has diagonal mortars (Es and Et)
-constexpr int kRecHead = 25;
+constexpr int kRecNupN = 25;    // ... of the others
+constexpr int kRecR0 = 26, kRecNr = 27;   // the item's angular nodes (all of them but in split lists)
+constexpr int kRecRaw = 28, kRecEt = 29;  // one-phase path: upwind values and mortar entries of the others
+constexpr int kRecHead = 30;
 // per staged coupling: face, m1, nth1, n0, stride, es, et, base (two words),
 // staging offset, coupling index, (unused); then the face nodes (ascending ij)
-constexpr int kRecCpl = 12;
+constexpr int kRecCpl = 16;
 constexpr int kCplF = 0, kCplM1 = 1, kCplNt1 = 2, kCplN0 = 3, kCplStr = 4, kCplEs = 5, kCplEt = 6, kCplBase = 7,
               kCplOff = 9, kCplK = 10,
-              kCplDiag = 11;   // bit 0: Es diagonal, bit 1: Et diagonal (off-diagonal entries below 1e-13 of the largest)
+              kCplDiag = 11,   // bit 0: Es diagonal, bit 1: Et diagonal (off-diagonal entries below 1e-13 of the largest)
+              kCplCol = 12, kCplRaw = 13, kCplEtOff = 14;   // one-phase path, Et not diagonal: column of T, offsets of line and Et
 constexpr int kRecMax = kRecHead + kRecCpl * kMaxCplStaged + kMaxFaceNodes;
 
 __device__ __forceinline__ int64_t rec64(const int* w) {
@@ -341,18 +357,33 @@ struct MapStore<double> {
     using type = double;
 };
 
-// Row length (entries) of an element's upwind map in the sweep of precision
-// T: nup rounded up so that a row is a whole number of 16-byte units of the
-// stored type and the number of units is odd (rows of consecutive outputs
-// then start in different 16-byte bank groups, so 16-byte loads of a quarter
-// warp do not conflict).
+// Row of an element's upwind map in the sweep of precision T: columns per
+// angular node, then columns shared by all of them, each part rounded up to
+// whole 16-byte units of the stored type and the number of units made odd
+// (rows of consecutive outputs then start in different 16-byte bank groups, so
+// 16-byte loads of a quarter warp do not conflict).
+struct MapRow {
+    int d, n, ld;   // entries of the parts and of the row
+};
 template <typename T>
-__host__ __device__ __forceinline__ int map_ld(int nup) {
+__host__ __device__ __forceinline__ MapRow map_row_layout(int d, int n) {
     constexpr int kVec = 16 / (int)sizeof(typename MapStore<T>::type);
-    if (nup <= 0) return 0;
-    int r = (nup + kVec - 1) / kVec * kVec;
-    if ((r / kVec) % 2 == 0) r += kVec;
-    return r;
+    MapRow m;
+    m.d = (d + kVec - 1) / kVec * kVec;
+    m.n = (n + kVec - 1) / kVec * kVec;
+    if (m.d + m.n > 0 && ((m.d + m.n) / kVec) % 2 == 0) (n > 0 ? m.n : m.d) += kVec;
+    m.ld = m.d + m.n;
+    return m;
+}
+
+// Values of T the one-phase path keeps in shared memory besides the block
+// inverse: the columns' values [nr][d] and [n], the map [nout][ld] (of the
+// stored type), upwind lines and mortars of the couplings that need T, rounded
+// up to 16 bytes
+template <typename T>
+__host__ __device__ __forceinline__ int64_t map_region(MapRow m, int nr, int nout, int raw, int et) {
+    return (int64_t)nr * m.d + m.n +
+           (int64_t)m.ld * nout * (int)sizeof(typename MapStore<T>::type) / (int)sizeof(T) + (raw + et + 3) / 4 * 4;
 }
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -365,38 +396,37 @@ __device__ __forceinline__ bool on_face(int F, int i, int j, int nx, int ny) {
     return (F == 0 && i == nx - 1) || (F == 1 && j == ny - 1) || (F == 2 && i == 0) || (F == 3 && j == 0);
 }
 
-// Upwind maps of the elements that take the one-phase path: for element e
-// with nup upwind values (the facing node lines of its active couplings, in
-// coupling order, then jj, then a), G_e = -B_e C_e maps them to the element's
-// values: z_e = B_e rin_e + G_e z_upwind.  G is stored by output row
-// (l = ij*nth + r), each row map_ld<T>(nup) values long (zero padded), each
-// element's block on a 16-byte boundary; FP32 and FP64 copies have their own
-// offsets.  Shared memory of the path (after rhs and zpre): upwind values
-// [map_ld, zero padded] | G_e [nloc * map_ld] | B_e [nth*nn*nn].
-// acc + sum over 16-byte units q0 <= q < q1 of a map row times the upwind
-// values (16-byte loads; four independent partial sums in FP32, two in FP64)
-__device__ __forceinline__ float map_row(const float* g, const float* zl, int q0, int q1, float acc) {
-    float a0 = acc, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-    const float4* g4 = reinterpret_cast<const float4*>(g);
-    const float4* z4 = reinterpret_cast<const float4*>(zl);
-    for (int q = q0; q < q1; ++q) {
-        const float4 gv = g4[q], zv = z4[q];
-        a0 = fmaf(gv.x, zv.x, a0);
-        a1 = fmaf(gv.y, zv.y, a1);
-        a2 = fmaf(gv.z, zv.z, a2);
-        a3 = fmaf(gv.w, zv.w, a3);
-    }
-    return (a0 + a1) + (a2 + a3);
-}
-// BF16 map (the FP32 sweep): a 16-byte unit holds eight entries, widened to
-// FP32 against two 16-byte units of upwind values
-__device__ __forceinline__ float map_row(const __nv_bfloat16* g, const float* zl, int q0, int q1, float acc) {
+// Upwind maps of the elements that take the one-phase path: z_e = B_e rin_e + G_e
+// w, w one value per angular node r and (coupling, jj), jj a node of the facing
+// line.  A coupling with a diagonal angular mortar (neighbouring cells of one
+// angle and degree) reaches the values of angular node r from those of node r
+// alone: w is the upwind value (jj, r) and G holds -dcoeff Et[r][r] sum_q B_r[ij][f_q]
+// Es[jj][q].  For the others w = T[jj][r] = sum_a Et[a][r] z_upwind[jj][a] is formed
+// after the wait, and G leaves Et out.  Either way a row of the map is
+// sum_couplings m1 long, nth times shorter than one over all upwind values (10
+// against 50 for 5 x 5 nodes and 5 angles): less to stage, and after the wait
+// nth times fewer multiply-adds, at which the FP64 pipe takes two a clock.  Columns of
+// the diagonal couplings come first.  T costs a barrier after the wait: where few
+// elements share a level (kFoldElems) the FP32 sweep, bound by the time from
+// level to level, folds Et into the map instead, whose rows then end with the
+// other couplings' upwind values (jj, a) themselves.  G is stored by output row
+// (l = ij*nth + r), each row map_row_layout<T> long (zero padded), each element's
+// block on a 16-byte boundary; FP32 and FP64 copies have their own offsets.
+// Shared memory of the path (after rhs and zpre): w [nr][d], [n] | G [nout][ld] |
+// upwind lines | Et | B_e.
+// acc + sum over the nvec 16-byte units of a map row times the columns' values:
+// the first nvd units meet zd, the others zn (both indexed by the unit; one
+// loop, so that what follows the wait is few instructions to fetch).  FP32: BF16
+// entries, eight to a unit, widened; four independent partial sums.
+__device__ __forceinline__ float map_row(const __nv_bfloat16* g, const float* zd, const float* zn, int nvd, int nvec,
+                                         float acc) {
     float a0 = acc, a1 = 0.f, a2 = 0.f, a3 = 0.f;
     const uint4* g4 = reinterpret_cast<const uint4*>(g);
-    const float4* z4 = reinterpret_cast<const float4*>(zl);
-    for (int q = q0; q < q1; ++q) {
+#pragma unroll 4
+    for (int q = 0; q < nvec; ++q) {
         const uint4 gv = g4[q];
-        const float4 za = z4[2 * q], zb = z4[2 * q + 1];
+        const float4* z4 = reinterpret_cast<const float4*>((q < nvd ? zd : zn) + 8 * q);
+        const float4 za = z4[0], zb = z4[1];
         const float2 g01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv.x));
         const float2 g23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv.y));
         const float2 g45 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv.z));
@@ -412,12 +442,13 @@ __device__ __forceinline__ float map_row(const __nv_bfloat16* g, const float* zl
     }
     return (a0 + a1) + (a2 + a3);
 }
-__device__ __forceinline__ double map_row(const double* g, const double* zl, int q0, int q1, double acc) {
+__device__ __forceinline__ double map_row(const double* g, const double* zd, const double* zn, int nvd, int nvec,
+                                          double acc) {
     double a0 = acc, a1 = 0.;
     const double2* g2 = reinterpret_cast<const double2*>(g);
-    const double2* z2 = reinterpret_cast<const double2*>(zl);
-    for (int q = q0; q < q1; ++q) {
-        const double2 gv = g2[q], zv = z2[q];
+#pragma unroll 2
+    for (int q = 0; q < nvec; ++q) {
+        const double2 gv = g2[q], zv = *reinterpret_cast<const double2*>((q < nvd ? zd : zn) + 2 * q);
         a0 = fma(gv.x, zv.x, a0);
         a1 = fma(gv.y, zv.y, a1);
     }
@@ -482,6 +513,7 @@ struct UpwindMap {
     int reg_cap = 0;                 // the largest one-phase region (upwind values and map) this launch takes (values)
     int stage_cap = 0;               // values of shared memory after rhs and zpre: a one-phase element whose
                                      // region and block inverse fit stages the inverse too
+    bool fold = false;               // the maps hold Et of every coupling: no T
     const int64_t* up = nullptr;     // upwind value offsets into z
     const typename MapStore<T>::type* G = nullptr;   // maps (this precision's copy)
 };
@@ -507,10 +539,12 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
     __shared__ int s_rec[kRecMax];
     __shared__ T s_dc[kMaxCplStaged];
     if (v.stop && *v.stop) return;
+    int ahead = -1;   // thread 0: the next element, claimed once this one's inputs are there
     for (;;) {
         unsigned long long t_claim = 0;
         if (threadIdx.x == 0) {
-            s_idx = (int)atomicAdd(next, 1u);
+            s_idx = ahead >= 0 ? ahead : (int)atomicAdd(next, 1u);
+            ahead = -1;
             s_abort = 0;
             if (trace) t_claim = globaltimer_ns();
         }
@@ -535,76 +569,177 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
         const int64_t dof_off = rec64(s_rec + kRecDof);
         // ---- independent of the sweep: block inverse, residual, mortars
         const TB* B = inv + rec64(s_rec + kRecInv);
-        const int bsize = nth * nn * nn;
-        if ((s_rec[kRecOk] & kOkBit) && s_rec[kRecReg + kP] <= um.reg_cap) {
+        const int r0 = s_rec[kRecR0], nr = s_rec[kRecNr];   // nr < nth: a part, which takes the one-phase path
+        const int bsize = nr * nn * nn;
+        const float rnth = __frcp_rn((float)nth), rnn = __frcp_rn((float)nn), rny = __frcp_rn((float)ny);
+        // the residual (asynchronous copies), zero at inflow-boundary nodes
+        auto stage_rin = [&] {
+            const float rnr = __frcp_rn((float)nr);
+            for (int l = threadIdx.x; l < nn * nr; l += blockDim.x) {   // rhs[ij*nr + (r - r0)]
+                const int ij = small_div(l, rnr);
+                bool bd = false;
+                if (bm) {
+                    const int i = small_div(ij, rny);
+                    bd = bdry_node_s(bm, i, ij - i * ny, nx, ny);
+                }
+                if (bd) rhs[l] = T(0);
+                else cp_async_small<sizeof(T)>(rhs + l, rin + dof_off + ij * nth + r0 + l - ij * nr);
+            }
+        };
+        if (nr < nth || ((s_rec[kRecOk] & kOkBit) && s_rec[kRecReg + kP] <= um.reg_cap)) {
             // ---- one-phase path: zpre = B rin and G_e staged before the wait,
-            // then z = zpre + G_e z_upwind once the upwind values arrive
+            // then z = zpre + G_e w once the upwind values arrive
             using TG = typename MapStore<T>::type;
             constexpr int kVec = 16 / sizeof(TG);  // map entries per 16-byte copy
-            const int nup = s_rec[kRecNup];
-            const int ld = map_ld<T>(nup);         // upwind values (T) and map row entries (TG)
-            const int gsz = ld * nloc;             // a multiple of kVec
-            T* zl = Bs;
-            TG* Gs = reinterpret_cast<TG*>(Bs + ld);
-            TB* Bg = reinterpret_cast<TB*>(Gs + gsz);
+            const bool fold = um.fold;
+            const int nd = s_rec[kRecNup], nraw = s_rec[kRecRaw];
+            const int nc = fold ? 0 : s_rec[kRecNupN], net = fold ? 0 : s_rec[kRecEt];
+            const MapRow m = map_row_layout<T>(nd + nc, fold ? nraw : 0);
+            const int ld = m.ld;                   // map entries of a row
+            const int nout = nn * nr;              // outputs of the item, l = ij*nr + (r - r0)
+            const int gsz = ld * nout;             // a multiple of kVec
+            const int region = (int)map_region<T>(m, nr, nout, fold ? 0 : nraw, net);
+            T* zl = Bs;                            // w
+            T* zc = Bs + nr * m.d;                 // ... of the columns shared by the angular nodes
+            TG* Gs = reinterpret_cast<TG*>(zc + m.n);
+            T* lines = reinterpret_cast<T*>(Gs + gsz);
+            T* ets = lines + nraw;
+            TB* Bg = reinterpret_cast<TB*>(Bs + region);
+            const int* s_cpl = s_rec + kRecHead;
+            const int ncs = s_rec[kRecNcs];
             const TG* Gg = um.G + rec64(s_rec + kRecGoff + 2 * kP);
             const int64_t* up = um.up + rec64(s_rec + kRecUoff);
-            for (int t = threadIdx.x; t < gsz / kVec; t += blockDim.x) cp_async16(Gs + t * kVec, Gg + t * kVec);
+            const float rnr = __frcp_rn((float)nr);
+            if (nr == nth) {
+                for (int t = threadIdx.x; t < gsz / kVec; t += blockDim.x) cp_async16(Gs + t * kVec, Gg + t * kVec);
+            } else {   // the part's rows of the map
+                const int nvl = ld / kVec;
+                const float rnv = __frcp_rn((float)max(nvl, 1));
+                for (int t = threadIdx.x; t < nout * nvl; t += blockDim.x) {
+                    const int l = small_div(t, rnv), ij = small_div(l, rnr);
+                    cp_async16(Gs + t * kVec,
+                               Gg + ((size_t)(ij * nth + r0 + l - ij * nr) * nvl + (t - l * nvl)) * kVec);
+                }
+            }
             // B is read once here (B rin, before the wait): staged with the map
             // when both fit, else read where it lies (coalesced over ij)
-            const bool bstaged = s_rec[kRecReg + kP] + block_units<T, TB>(bsize) <= um.stage_cap;
-            if (bstaged) stage_block(Bg, B, bsize);
-            const TB* Bv = bstaged ? Bg : B;
-            for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
-                const int ij = l / nth;
-                rhs[l] = bdry_node_s(bm, ij / ny, ij % ny, nx, ny) ? T(0) : rin[dof_off + l];
+            const bool bstaged = region + block_units<T, TB>(bsize) <= um.stage_cap;
+            const TB* Bp = B + r0 * nn * nn;
+            if (bstaged) stage_block(Bg, Bp, bsize);
+            const TB* Bv = bstaged ? Bg : Bp;
+            stage_rin();
+            for (int c = 0; c < ncs && net; ++c) {   // Et of the couplings that need T
+                const int* cp = s_cpl + kRecCpl * c;
+                if (cp[kCplDiag] & 2) continue;
+                const T* et = v.mort + cp[kCplEt];
+                for (int t = threadIdx.x; t < cp[kCplNt1] * nth; t += blockDim.x)
+                    cp_async_small<sizeof(T)>(ets + cp[kCplEtOff] + t, et + t);
             }
-            int64_t my_up = threadIdx.x < nup ? __ldg(up + threadIdx.x) : 0;
+            // upwind value t: (column, r) of the diagonal couplings, then the
+            // other couplings' lines; neighbouring threads wait on neighbouring
+            // values (in the order (r, column) the polls spread over four times as
+            // many sectors and held the publishing stores up: 62 -> 70 us a sweep
+            // at 218,581 DOF)
+            const int nzd = nr * nd, nz = nzd + nraw;
+            const int raw_at = fold ? nr * m.d : (int)(lines - zl);   // places by their offset from zl
+            auto value = [&](int t, int64_t& o) -> int {   // offset in z; place
+                if (t < nzd) {
+                    const int u = small_div(t, rnr), r = t - u * nr;
+                    o = __ldg(up + u) + r0 + r;
+                    return r * m.d + u;
+                }
+                o = __ldg(up + nd + t - nzd);
+                return raw_at + t - nzd;
+            };
+            int64_t my_o = 0;
+            int my_p = (int)threadIdx.x < nz ? value(threadIdx.x, my_o) : 0;
+            for (int t = threadIdx.x; t < nr * (m.d - nd - nc); t += blockDim.x) {   // padding
+                const int u = small_div(t, rnr);
+                zl[(t - u * nr) * m.d + nd + nc + u] = T(0);
+            }
+            if (fold && nraw + (int)threadIdx.x < m.n) zc[nraw + threadIdx.x] = T(0);
             cp_async_wait_all();
             __syncthreads();
-            for (int t = threadIdx.x; t < nloc; t += blockDim.x) {
-                const int r = t / nn, ij = t % nn;
-                zpre[ij * nth + r] = strided_dot(Bv + r * nn * nn + ij, nn, rhs + r, nth, nn);
+            for (int t = threadIdx.x; t < nout; t += blockDim.x) {
+                const int r = small_div(t, rnn), ij = t - r * nn;
+                zpre[ij * nr + r] = strided_dot(Bv + r * nn * nn + ij, nn, rhs + r, nr, nn);
             }
+            // everything but the upwind values in place for the thread's first
+            // output and item of T: what follows the wait is all on the critical path
+            const int l0 = threadIdx.x, ij0 = small_div(l0, rnr), q0 = l0 - ij0 * nr;
+            const int nvd = m.d / kVec, nvec = ld / kVec;
+            const T* zn0 = zc - m.d;               // indexed by the row's entry
+            const TG* g0 = Gs + (size_t)l0 * ld;
+            const T* zl0 = zl + q0 * m.d;
+            T* zout = z + dof_off + r0;
+            const int nT = nc * nr;
+            int tet = 0, tline = 0, tdst = 0, tn = 0;
+            auto find_T = [&](int t) {   // item t of T: its mortar column, line and place
+                for (int c = 0; c < ncs; ++c) {
+                    const int* cp = s_cpl + kRecCpl * c;
+                    if (cp[kCplDiag] & 2) continue;
+                    const int n = cp[kCplM1] * nr;
+                    if (t >= n) {
+                        t -= n;
+                        continue;
+                    }
+                    const int jj = small_div(t, rnr), r = t - jj * nr;
+                    tn = cp[kCplNt1];
+                    tet = cp[kCplEtOff] + r0 + r;
+                    tline = cp[kCplRaw] + jj * tn;
+                    tdst = r * m.d + cp[kCplCol] + jj;
+                    return;
+                }
+            };
+            if ((int)threadIdx.x < nT) find_T(threadIdx.x);
             long long ck0 = 0, ck1 = 0;
             if (trace && threadIdx.x == 0) {
                 trace[kTr * e + 1] = globaltimer_ns();
                 ck0 = clock64();
             }
-            for (int u = threadIdx.x; u < ld; u += blockDim.x) {
+            for (int t = threadIdx.x; t < nz; t += blockDim.x) {
+                if (t != (int)threadIdx.x) my_p = value(t, my_o);
                 T val = T(0);
-                if (u < nup) {
-                    const int64_t o = u == threadIdx.x ? my_up : __ldg(up + u);
-                    if (!load_published(z + o, val, status)) s_abort = 1;
-                }
-                zl[u] = val;   // padding: zero
+                if (!load_published(z + my_o, val, status)) s_abort = 1;
+                zl[my_p] = val;
             }
             __syncthreads();
             if (s_abort) break;
             if (trace && threadIdx.x == 0) ck1 = clock64();
-            // FP64 (bound by the FP64 pipe): two threads per output when the
-            // CTA has them, the second half of the upwind values through rhs
-            // (free once zpre is formed).  FP32 is latency bound and keeps one
-            // thread per output (the extra barrier costs more than it saves).
-            const bool split = sizeof(T) == 8 && 2 * nloc <= (int)blockDim.x;
-            const int nvec = ld / kVec;                 // 16-byte units per row
-            const int vh = split ? (nvec + 1) / 2 : nvec;
-            T part = T(0);
-            const int t = threadIdx.x;
-            const int l = split ? t % nloc : t;
-            const int half = split ? t / nloc : 0;
-            if (!split || t < 2 * nloc) {
-                for (int l2 = l; l2 < nloc; l2 += blockDim.x) {
-                    const int q0 = half ? vh : 0, q1 = half ? nvec : vh;
-                    part = map_row(Gs + (size_t)l2 * ld, zl, q0, q1, half ? T(0) : zpre[l2]);
-                    if (half) rhs[l2] = part;
-                    else if (!split) st_relaxed(z + dof_off + l2, part);
+            // A CTA that has spun for its values fetches what follows anew: few
+            // instructions, each loop once (with the first output peeled off and a
+            // loop for either part of the row 600 cycles, so 440 at 4 x 4 nodes)
+            if (nT) {
+                // T[jj][r] of the couplings whose angular mortar is not diagonal
+                for (int t = threadIdx.x; t < nT; t += blockDim.x) {
+                    if (t != (int)threadIdx.x) find_T(t);
+                    T a0 = T(0), a1 = T(0);
+                    int a = 0;
+                    for (; a + 2 <= tn; a += 2) {
+                        a0 = fma(ets[tet + a * nth], lines[tline + a], a0);
+                        a1 = fma(ets[tet + (a + 1) * nth], lines[tline + a + 1], a1);
+                    }
+                    if (a < tn) a0 = fma(ets[tet + a * nth], lines[tline + a], a0);
+                    zl[tdst] = a0 + a1;
+                }
+                __syncthreads();
+            }
+            {
+                int l = l0, at = ij0 * nth + q0;
+                const TG* g = g0;
+                const T* zd = zl0;
+                while (l < nout) {
+                    st_relaxed(zout + at, map_row(g, zd, zn0, nvd, nvec, zpre[l]));
+                    l += blockDim.x;
+                    const int ij = small_div(l, rnr), r = l - ij * nr;
+                    at = ij * nth + r;
+                    g = Gs + (size_t)l * ld;
+                    zd = zl + r * m.d;
                 }
             }
-            if (split) {
-                __syncthreads();
-                if (t < nloc) st_relaxed(z + dof_off + t, part + rhs[t]);
-            }
+            // the claim's round trip passes while the other warps finish (a
+            // claim before the wait would hold the next element up: 0.77 -> 0.97 ms)
+            if (threadIdx.x == 0) ahead = (int)atomicAdd(next, 1u);
             __syncthreads();
             if (trace && threadIdx.x == 0) {
                 const long long ck4 = clock64();
@@ -630,10 +765,7 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(b0 + o));
         }
         const TB* Bv = staged ? Bsb : B;
-        for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
-            const int ij = l / nth;
-            rhs[l] = bdry_node_s(bm, ij / ny, ij % ny, nx, ny) ? T(0) : rin[dof_off + l];
-        }
+        stage_rin();
         // the active couplings (in coupling order) and the face nodes they
         // reach, from the record; their mortars staged with asynchronous
         // copies, waited on with the block inverse's
@@ -655,7 +787,7 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
         __syncthreads();
         // zpre = B rin, block stored as [r][k][ij]
         for (int t = threadIdx.x; t < nloc; t += blockDim.x) {
-            const int r = t / nn, ij = t % nn;
+            const int r = small_div(t, rnn), ij = t - r * nn;
             zpre[ij * nth + r] = strided_dot(Bv + r * nn * nn + ij, nn, rhs + r, nth, nn);
         }
         // ---- couplings c on the face nodes, into rhs[ij * nth + r]
@@ -671,7 +803,7 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
             // The couplings overwrite rin at the face nodes: B rin is formed first.
             __syncthreads();
             for (int t = threadIdx.x; t < nf * nth; t += blockDim.x) {
-                const int ij = s_face[t / nth], r = t % nth, i = ij / ny, j = ij % ny;
+                const int tq = small_div(t, rnth), ij = s_face[tq], r = t - tq * nth, i = small_div(ij, rny), j = ij - i * ny;
                 T acc = T(0);
                 for (int c = 0; c < ncs; ++c) {
                     const int* cp = s_cpl + kRecCpl * c;
@@ -697,8 +829,9 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
                 T* dst = cs + cp[kCplOff] + m1 * cp[kCplN0] + nt1 * nth;
                 const T* src = z + rec64(cp + kCplBase);
                 const int str = cp[kCplStr];
+                const float rnt1 = __frcp_rn((float)nt1);
                 for (int t = threadIdx.x; t < m1 * nt1; t += blockDim.x) {
-                    const int jj = t / nt1, a = t % nt1;
+                    const int jj = small_div(t, rnt1), a = t - jj * nt1;
                     T val = T(0);
                     if (!load_published(src + (int64_t)jj * str + a, val, status)) s_abort = 1;
                     dst[t] = val;
@@ -724,7 +857,7 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
                     const T* Et = cs + cp[kCplOff] + m1 * cp[kCplN0];
                     const T* zl = Et + nt1 * nth;
                     T* Tm = cs + cp[kCplOff] + m1 * cp[kCplN0] + nt1 * nth + m1 * nt1;
-                    const int q = t - base, jj = q / nth, r = q % nth;
+                    const int q = t - base, jj = small_div(q, rnth), r = q - jj * nth;
                     T acc = T(0);
                     if (dg & 2) {
                         acc = Et[r * nth + r] * zl[jj * nt1 + r];
@@ -737,7 +870,7 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
             __syncthreads();
             if (trace && threadIdx.x == 0) ck2 = clock64();
             for (int t = threadIdx.x; t < nf * nth; t += blockDim.x) {
-                const int ij = s_face[t / nth], r = t % nth, i = ij / ny, j = ij % ny;
+                const int tq = small_div(t, rnth), ij = s_face[tq], r = t - tq * nth, i = small_div(ij, rny), j = ij - i * ny;
                 T acc = T(0);
                 for (int c = 0; c < ncs; ++c) {
                     const int* cp = s_cpl + kRecCpl * c;
@@ -763,7 +896,7 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
             }
         } else {
             for (int t = threadIdx.x; t < nf * nth; t += blockDim.x) {
-                const int ij = s_face[t / nth], r = t % nth, i = ij / ny, j = ij % ny;
+                const int tq = small_div(t, rnth), ij = s_face[tq], r = t - tq * nth, i = small_div(ij, rny), j = ij - i * ny;
                 T acc = T(0);
                 for (int k = s_rec[kRecCplB]; k < s_rec[kRecCplE]; ++k) {
                     if (!active[k]) continue;
@@ -795,7 +928,7 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
         if (trace && threadIdx.x == 0) ck3 = clock64();
         // ---- z = zpre - B c over the face columns of B
         for (int t = threadIdx.x; t < nloc; t += blockDim.x) {
-            const int r = t / nn, ij = t % nn;
+            const int r = small_div(t, rnn), ij = t - r * nn;
             const TB* col = Bv + r * nn * nn + ij;
             T a0 = zpre[ij * nth + r], a1 = T(0), a2 = T(0), a3 = T(0);
             int f = 0;
@@ -809,6 +942,7 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
             for (; f < nf; ++f) a0 -= widen(col[s_face[f] * nn]) * rhs[s_face[f] * nth + r];
             st_relaxed(z + dof_off + (int64_t)ij * nth + r, (a0 + a1) + (a2 + a3));
         }
+        if (threadIdx.x == 0) ahead = (int)atomicAdd(next, 1u);
         // the stored values are the publication (downstream elements wait on
         // the values themselves); the barrier ends this element's use of the
         // shared buffers before the next claim
@@ -833,38 +967,42 @@ __global__ void to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __re
         out[i] = __float2bfloat16_rn(in[i]);
 }
 
-// Builds the upwind maps G_e = -B_e C_e of the one-phase elements in FP64
-// (and the FP32 sweep's BF16 copies, rounded to nearest even; rows of map_ld
-// entries, padding left zero): entry
-// (u, l) with u = (coupling k, jj, a) and l = (ij, r) is -dcoeff_k Et_k[a][r] sum_q B_r[ij][f_q] Es_k[jj][q] over the
-// nodes f_q of coupling k's face that are not inflow-boundary nodes.  One CTA
-// per element.
+// Builds the upwind maps of the one-phase elements in FP64 (and the FP32
+// sweep's BF16 copies, rounded to nearest even; rows of map_row_layout entries,
+// padding left zero): entry (coupling k, jj) of the row of output l = (ij, r) is -dcoeff_k
+// sum_q B_r[ij][f_q] Es_k[jj][q] over the nodes f_q of coupling k's face that are
+// not inflow-boundary nodes, times Et_k[r][r] where diag marks the coupling's
+// angular mortar as diagonal; those columns come first.  With fold the FP32
+// sweep's rows hold, for the others, the entries times Et_k[a][r] of every (jj, a)
+// instead.  One CTA per element.
 __global__ void build_upwind_map_kernel(OpView<double> v, const uint8_t* __restrict__ active,
+                                        const uint8_t* __restrict__ diag,
                                         const double* __restrict__ inv, const int64_t* __restrict__ inv_elem_off,
                                         const int32_t* __restrict__ elems, const int32_t* __restrict__ nup_e,
-                                        const int64_t* __restrict__ goff64, const int64_t* __restrict__ goff32,
+                                        const int64_t* __restrict__ goff64, const int64_t* __restrict__ goff32, bool fold,
                                         double* __restrict__ G64, __nv_bfloat16* __restrict__ G16) {
     const int e = elems[blockIdx.x];
     const ElemDev E = v.elems[e];
     const ColDev C = v.cols[E.col];
     const int nth = E.nth, nn = C.nx * C.ny, nloc = nn * nth, bm = E.flags >> 4;
-    const int nup = nup_e[e];
+    const int nd = nup_e[3 * e], nc = nup_e[3 * e + 1], nraw = nup_e[3 * e + 2];
+    const MapRow m64 = map_row_layout<double>(nd + nc, 0);
+    const MapRow m32 = map_row_layout<float>(fold ? nd : nd + nc, fold ? nraw : 0);
     const double* B = inv + inv_elem_off[e];
-    for (int t = threadIdx.x; t < nup * nloc; t += blockDim.x) {
+    for (int t = threadIdx.x; t < (nd + nc) * nloc; t += blockDim.x) {
         const int u = t / nloc, l = t % nloc, ij = l / nth, r = l % nth;
-        int uu = u, k = E.cpl_begin;
+        const bool dg = u < nd;
+        int jj = dg ? u : u - nd, k = E.cpl_begin, line = 0;   // line: entries of the other couplings' lines before k's
         for (; k < E.cpl_end; ++k) {
-            if (!active[k]) continue;
-            const int sz = v.cgeo[k].m1 * v.cgeo[k].nth1;
-            if (uu < sz) break;
-            uu -= sz;
+            if (!active[k] || (bool)diag[k] != dg) continue;
+            if (jj < v.cgeo[k].m1) break;
+            jj -= v.cgeo[k].m1;
+            line += v.cgeo[k].m1 * v.cgeo[k].nth1;
         }
-        const CplGeo g = v.cgeo[k];
         const CplDev cp = v.cpls[k];
-        const int jj = uu / g.nth1, a = uu % g.nth1;
         const int F = cp.face;
         const int n0 = (F % 2 == 0) ? C.ny : C.nx;
-        const double et = v.mort[cp.et + a * nth + r];
+        const double et = dg ? v.mort[cp.et + r * nth + r] : 1.;
         double acc = 0.;
         for (int q = 0; q < n0; ++q) {
             const int i = (F == 0) ? C.nx - 1 : (F == 2) ? 0 : q;
@@ -873,8 +1011,16 @@ __global__ void build_upwind_map_kernel(OpView<double> v, const uint8_t* __restr
             acc += B[(int64_t)r * nn * nn + (int64_t)(i * C.ny + j) * nn + ij] * v.mort[cp.es + jj * n0 + q];
         }
         const double val = -v.cplc[k] * et * acc;
-        G64[goff64[e] + (int64_t)l * map_ld<double>(nup) + u] = val;
-        G16[goff32[e] + (int64_t)l * map_ld<float>(nup) + u] = __float2bfloat16_rn((float)val);
+        G64[goff64[e] + (int64_t)l * m64.ld + u] = val;
+        __nv_bfloat16* row = G16 + goff32[e] + (int64_t)l * m32.ld;
+        if (dg || !fold) {
+            row[u] = __float2bfloat16_rn((float)val);
+        } else {
+            const int nt1 = v.cgeo[k].nth1;
+            for (int a = 0; a < nt1; ++a)
+                row[m32.d + line + jj * nt1 + a] =
+                    __float2bfloat16_rn((float)(-v.cplc[k] * v.mort[cp.et + a * nth + r] * acc));
+        }
     }
 }
 
@@ -899,12 +1045,15 @@ struct Sweep {
     struct Shape {
         size_t smem = 0;
         int bcap = 0, grid = 0, reg_cap = 0, threads = kSweepThreads;
+        bool split = false;
     };
     Shape shape[2][kSweepShapes];
     int pick[2] = {-1, -1};
     float shape_ms[2][kSweepShapes] = {};
     int32_t *d_greg32 = nullptr, *d_greg64 = nullptr;
     int32_t* d_rec = nullptr;            // element records in claim order
+    int32_t* d_rec_split = nullptr;      // the same in parts of kSplitNth angular nodes (FP64)
+    int nsplit = 0;
     int rec_stride = 0;                  // words per record (a multiple of 32)
     int n_lagged = 0;
     std::vector<void*> allocs;
@@ -918,6 +1067,7 @@ struct Sweep {
     __nv_bfloat16* d_G16 = nullptr;     // the FP32 sweep's copy
     int64_t gmax32 = 0, gmax64 = 0;     // largest one-phase region with its block inverse (values) per precision
     int64_t g_entries = 0;
+    bool fold = false;                  // FP32 maps with Et folded in
     // per precision (FP32, FP64), the elements with a map: the region the map
     // and the upwind values take (values), map entries, upwind indices; a
     // launch shape uses the maps whose region fits it
@@ -1136,14 +1286,41 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
         max_c = std::max(max_c, c);
     }
     s->max_c = max_c;
+    // an m x n mortar block is diagonal: off-diagonal entries (rounding noise
+    // between conforming neighbours) below 1e-13 of the largest, which the
+    // preconditioner leaves out
+    auto diagonal = [&](int64_t off, int rows, int cols) {
+        if (rows != cols) return false;
+        double mx = 0.;
+        for (int q = 0; q < rows * cols; ++q) mx = std::max(mx, std::fabs(t.mort[(size_t)off + q]));
+        for (int a = 0; a < rows; ++a)
+            for (int b = 0; b < cols; ++b)
+                if (a != b && std::fabs(t.mort[(size_t)off + (size_t)a * cols + b]) > 1e-13 * mx) return false;
+        return mx > 0.;
+    };
+    // per coupling: its angular mortar is diagonal (mortars are shared: each block is looked at once)
+    std::vector<uint8_t> ediag(t.cpls.size(), 0);
+    {
+        std::unordered_map<int64_t, uint8_t> seen;
+        for (int e = 0; e < ne; ++e)
+            for (int k = t.elems[e].cpl_begin; k < t.elems[e].cpl_end; ++k) {
+                const int64_t key = ((int64_t)t.cpls[k].et * (kMaxNodes + 1) + t.cgeo[k].nth1) * (kMaxNodes + 1) + t.elems[e].nth;
+                auto f = seen.find(key);
+                if (f == seen.end())
+                    f = seen.emplace(key, diagonal(t.cpls[k].et, t.cgeo[k].nth1, t.elems[e].nth) ? 1 : 0).first;
+                ediag[k] = f->second;
+            }
+    }
     // ---- upwind maps of the elements whose map fits in shared memory.  A map
     // is a function of the element's (shared) block inverses and of its active
     // couplings' faces, sizes, mortars and dcoeff; elements that agree on them
     // share one stored map (built once, by the first of them).
     {
         const int rhs_cap = (std::max(s->max_nloc, 1) + 1) & ~1;   // even: 16-byte aligned region after rhs, zpre
+        const bool fold = ne < kFoldElems * nlev;
+        s->fold = fold;
         std::vector<uint8_t> gok(ne, 0);
-        std::vector<int32_t> gnup(ne, 0), gel, greg32(ne, 0), greg64(ne, 0);
+        std::vector<int32_t> gnup(3 * (size_t)ne, 0), graw(ne, 0), get(ne, 0), gel, greg32(ne, 0), greg64(ne, 0);
         std::vector<int64_t> goff64(ne, 0), goff32(ne, 0), uoff(ne, 0), up;
         int64_t gtot64 = 0, gtot32 = 0;
         std::unordered_map<std::vector<uint64_t>, std::pair<int64_t, int64_t>, WordsHash> gshared;
@@ -1152,17 +1329,31 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
             const ElemDev& E = t.elems[e];
             const ColDev& C = t.cols[E.col];
             const int nloc = C.nx * C.ny * E.nth;
-            int64_t nup = 0;
-            for (int k = E.cpl_begin; k < E.cpl_end; ++k)
-                if (active[k]) nup += (int64_t)t.cgeo[k].m1 * t.cgeo[k].nth1;
-            // upwind values (one map row long), G_e, then B_e
+            // columns through diagonal angular mortars and through the others;
+            // upwind values and mortar entries of the others
+            int nd = 0, nn1 = 0, raw = 0, et = 0, nact = 0;
+            for (int k = E.cpl_begin; k < E.cpl_end; ++k) {
+                if (!active[k]) continue;
+                const CplGeo& g = t.cgeo[k];
+                ++nact;
+                if (ediag[k]) {
+                    nd += g.m1;
+                } else {
+                    nn1 += g.m1;
+                    raw += g.m1 * g.nth1;
+                    et += g.nth1 * E.nth;
+                }
+            }
+            if (nact > kMaxCplStaged) continue;
             const int64_t bsize = (int64_t)E.nth * C.nx * C.ny * C.nx * C.ny;
-            const int64_t ld32 = map_ld<float>((int)nup), ld64 = map_ld<double>((int)nup);
-            // FP32 sweep: upwind values in FP32, G_e in BF16 (ld32 is a multiple
-            // of 8, so the map is a whole number of FP32 values); B_e (read
-            // once, before the wait) joins them in shared memory when it fits
-            const int64_t region32 = ld32 + ld32 * nloc / 2;
-            const int64_t region64 = ld64 + ld64 * nloc;
+            const MapRow m32 = map_row_layout<float>(fold ? nd : nd + nn1, fold ? raw : 0);
+            const MapRow m64 = map_row_layout<double>(nd + nn1, 0);
+            const int64_t ld32 = m32.ld, ld64 = m64.ld;
+            // FP32 sweep: G_e in BF16 (ld32 is a multiple of 8, so the map is a
+            // whole number of FP32 values); B_e (read once, before the wait)
+            // joins them in shared memory when it fits
+            const int64_t region32 = map_region<float>(m32, E.nth, nloc, fold ? 0 : raw, fold ? 0 : et);
+            const int64_t region64 = map_region<double>(m64, E.nth, nloc, raw, et);
             const int64_t with_b32 = region32 + block_units<float, __nv_bfloat16>((int)bsize);
             const int64_t with_b64 = region64 + block_units<double, double>((int)bsize);
             uint8_t ok = 0;
@@ -1170,7 +1361,11 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
             if (region64 * 8 + 2 * rhs_cap * 8 <= (int64_t)kSweepSmemBudget) ok |= 2;
             if (!ok) continue;
             gok[e] = ok;
-            gnup[e] = (int32_t)nup;
+            gnup[3 * (size_t)e] = nd;
+            gnup[3 * (size_t)e + 1] = nn1;
+            gnup[3 * (size_t)e + 2] = raw;
+            graw[e] = raw;
+            get[e] = et;
             greg32[e] = (int32_t)region32;
             greg64[e] = (int32_t)region64;
             uoff[e] = (int64_t)up.size();
@@ -1194,16 +1389,18 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
                 goff64[e] = ghit->second.first;
                 goff32[e] = ghit->second.second;
             }
-            for (int k = E.cpl_begin; k < E.cpl_end; ++k) {
-                if (!active[k]) continue;
-                const CplGeo& g = t.cgeo[k];
-                for (int jj = 0; jj < g.m1; ++jj)
-                    for (int a = 0; a < g.nth1; ++a) up.push_back(g.base + (int64_t)jj * g.stride + a);
-            }
+            // the diagonal couplings' columns (offsets of angular node 0), then the others' lines
+            for (int dg = 1; dg >= 0; --dg)
+                for (int k = E.cpl_begin; k < E.cpl_end; ++k) {
+                    if (!active[k] || ediag[k] != dg) continue;
+                    const CplGeo& g = t.cgeo[k];
+                    for (int jj = 0; jj < g.m1; ++jj)
+                        for (int a = 0; a < (dg ? 1 : g.nth1); ++a) up.push_back(g.base + (int64_t)jj * g.stride + a);
+                }
             if (ok & 1) s->gmax32 = std::max(s->gmax32, with_b32);
             if (ok & 2) s->gmax64 = std::max(s->gmax64, with_b64);
             for (int p = 0; p < 2; ++p)
-                if (ok & (1 << p)) s->onephase[p].push_back({p ? region64 : region32, (p ? ld64 : ld32) * nloc, nup});
+                if (ok & (1 << p)) s->onephase[p].push_back({p ? region64 : region32, (p ? ld64 : ld32) * nloc, (int64_t)nd + raw});
             if (built) gel.push_back(e);
         }
         s->g_entries = gtot64 + gtot32;
@@ -1212,7 +1409,7 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
         s->d_greg64 = sw_alloc<int32_t>(s, ne);
         RTG_CUDA(cudaMemcpy(s->d_greg32, greg32.data(), sizeof(int32_t) * ne, cudaMemcpyHostToDevice));
         RTG_CUDA(cudaMemcpy(s->d_greg64, greg64.data(), sizeof(int32_t) * ne, cudaMemcpyHostToDevice));
-        s->d_gnup = sw_alloc<int32_t>(s, ne);
+        s->d_gnup = sw_alloc<int32_t>(s, gnup.size());
         s->d_goff64 = sw_alloc<int64_t>(s, ne);
         s->d_goff32 = sw_alloc<int64_t>(s, ne);
         s->d_uoff = sw_alloc<int64_t>(s, ne);
@@ -1223,7 +1420,7 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
         RTG_CUDA(cudaMemset(s->d_G16, 0, sizeof(__nv_bfloat16) * std::max<int64_t>(gtot32, 1)));
         int32_t* d_gel = sw_alloc<int32_t>(s, gel.size());
         RTG_CUDA(cudaMemcpy(s->d_gok, gok.data(), ne, cudaMemcpyHostToDevice));
-        RTG_CUDA(cudaMemcpy(s->d_gnup, gnup.data(), sizeof(int32_t) * ne, cudaMemcpyHostToDevice));
+        RTG_CUDA(cudaMemcpy(s->d_gnup, gnup.data(), sizeof(int32_t) * gnup.size(), cudaMemcpyHostToDevice));
         RTG_CUDA(cudaMemcpy(s->d_goff64, goff64.data(), sizeof(int64_t) * ne, cudaMemcpyHostToDevice));
         RTG_CUDA(cudaMemcpy(s->d_goff32, goff32.data(), sizeof(int64_t) * ne, cudaMemcpyHostToDevice));
         RTG_CUDA(cudaMemcpy(s->d_uoff, uoff.data(), sizeof(int64_t) * ne, cudaMemcpyHostToDevice));
@@ -1231,9 +1428,11 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
             RTG_CUDA(cudaMemcpy(s->d_up, up.data(), sizeof(int64_t) * up.size(), cudaMemcpyHostToDevice));
         if (!gel.empty()) {
             RTG_CUDA(cudaMemcpy(d_gel, gel.data(), sizeof(int32_t) * gel.size(), cudaMemcpyHostToDevice));
-            build_upwind_map_kernel<<<(int)gel.size(), 256, 0, st>>>(h->v64, s->d_active, s->d_inv64, s->d_inv_off,
-                                                                    d_gel, s->d_gnup, s->d_goff64, s->d_goff32, s->d_G64,
-                                                                    s->d_G16), count_launch();
+            uint8_t* d_ediag = sw_alloc<uint8_t>(s, ediag.size());
+            RTG_CUDA(cudaMemcpy(d_ediag, ediag.data(), ediag.size(), cudaMemcpyHostToDevice));
+            build_upwind_map_kernel<<<(int)gel.size(), 256, 0, st>>>(h->v64, s->d_active, d_ediag, s->d_inv64, s->d_inv_off,
+                                                                    d_gel, s->d_gnup, s->d_goff64, s->d_goff32, fold,
+                                                                    s->d_G64, s->d_G16), count_launch();
             RTG_CUDA(cudaGetLastError());
         }
         // ---- element records in claim order (the words are listed with kRecE)
@@ -1269,7 +1468,12 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
             R[kRecOk] = gok[e];
             R[kRecReg] = greg32[e];
             R[kRecReg + 1] = greg64[e];
-            R[kRecNup] = gnup[e];
+            R[kRecNup] = gnup[3 * (size_t)e];
+            R[kRecNupN] = gnup[3 * (size_t)e + 1];
+            R[kRecRaw] = graw[e];
+            R[kRecEt] = get[e];
+            R[kRecR0] = 0;
+            R[kRecNr] = E.nth;
             put64(&R[kRecGoff], goff32[e]);
             put64(&R[kRecGoff + 2], goff64[e]);
             put64(&R[kRecUoff], uoff[e]);
@@ -1287,23 +1491,15 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
             // preconditioner leaves them out): the face value (q, r) takes only
             // the upwind value (q, r), so the couplings need no T and no sums
             bool direct = ncs > 0;
-            auto diagonal = [&](int64_t off, int rows, int cols) {
-                double mx = 0.;
-                for (int q = 0; q < rows * cols; ++q) mx = std::max(mx, std::fabs(t.mort[(size_t)off + q]));
-                for (int a = 0; a < rows; ++a)
-                    for (int b = 0; b < cols; ++b)
-                        if (a != b && std::fabs(t.mort[(size_t)off + (size_t)a * cols + b]) > 1e-13 * mx) return false;
-                return mx > 0.;
-            };
             for (int c = 0; c < ncs && direct; ++c) {
                 const int k = act[c];
                 const CplDev& cp = t.cpls[k];
                 const CplGeo& g = t.cgeo[k];
                 const int n0 = (cp.face % 2 == 0) ? C.ny : C.nx;
-                direct = g.m1 == n0 && g.nth1 == E.nth && diagonal(cp.es, g.m1, n0) && diagonal(cp.et, g.nth1, E.nth);
+                direct = diagonal(cp.es, g.m1, n0) && ediag[k];
             }
             R[kRecDirect] = direct ? 1 : 0;
-            int soff = 0;
+            int soff = 0, ccol = R[kRecNup], craw = 0, cet = 0;
             for (int c = 0; c < ncs; ++c) {
                 const int k = act[c];
                 const CplDev& cp = t.cpls[k];
@@ -1320,8 +1516,15 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
                 put64(&w[kCplBase], g.base);
                 w[kCplOff] = soff;
                 w[kCplK] = k;
-                w[kCplDiag] = (g.m1 == n0 && diagonal(cp.es, g.m1, n0) ? 1 : 0) |
-                              (g.nth1 == E.nth && diagonal(cp.et, g.nth1, E.nth) ? 2 : 0);
+                w[kCplDiag] = (diagonal(cp.es, g.m1, n0) ? 1 : 0) | (ediag[k] ? 2 : 0);
+                if (!ediag[k]) {
+                    w[kCplCol] = ccol;
+                    w[kCplRaw] = craw;
+                    w[kCplEtOff] = cet;
+                    ccol += g.m1;
+                    craw += g.m1 * g.nth1;
+                    cet += g.nth1 * E.nth;
+                }
                 R.insert(R.end(), w, w + kRecCpl);
                 soff += g.m1 * n0 + g.nth1 * E.nth + g.m1 * g.nth1 + g.m1 * E.nth;
             }
@@ -1347,6 +1550,27 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
             std::copy(recs[idx].begin(), recs[idx].end(), flat.begin() + (size_t)idx * s->rec_stride);
         s->d_rec = sw_alloc<int32_t>(s, flat.size());
         RTG_CUDA(cudaMemcpy(s->d_rec, flat.data(), sizeof(int32_t) * flat.size(), cudaMemcpyHostToDevice));
+        // the FP64 split list: elements whose parts all fit take one item per
+        // part, next to each other in the claim order
+        std::vector<int32_t> sp;
+        for (int idx = 0; idx < ne; ++idx) {
+            const std::vector<int32_t>& R = recs[idx];
+            const int nth = R[kRecNth], nn = R[kRecNx] * R[kRecNy];
+            const int64_t region = map_region<double>(map_row_layout<double>(R[kRecNup] + R[kRecNupN], 0), kSplitNth,
+                                                      nn * kSplitNth, R[kRecRaw], R[kRecEt]);
+            const bool parts = (R[kRecOk] & 2) && nth > kSplitNth &&
+                               (region + 2 * (int64_t)rhs_cap) * 8 <= (int64_t)kSplitBudget;
+            for (int r0 = 0; r0 < nth; r0 += parts ? kSplitNth : nth) {
+                const size_t at = sp.size();
+                sp.resize(at + s->rec_stride, 0);
+                std::copy(R.begin(), R.end(), sp.begin() + at);
+                sp[at + kRecR0] = r0;
+                sp[at + kRecNr] = parts ? std::min(kSplitNth, nth - r0) : nth;
+                ++s->nsplit;
+            }
+        }
+        s->d_rec_split = sw_alloc<int32_t>(s, sp.size());
+        RTG_CUDA(cudaMemcpy(s->d_rec_split, sp.data(), sizeof(int32_t) * sp.size(), cudaMemcpyHostToDevice));
     }
     return s;
 }
@@ -1374,13 +1598,17 @@ void apply_sweep(rtg_handle* h, const T* r, T* z, cudaStream_t st, unsigned long
     const int rhs_cap = (std::max(s->max_nloc, 1) + 1) & ~1;   // even: 16-byte aligned region after rhs, zpre
     UpwindMap<T> um;
     um.up = s->d_up;
+    um.fold = !f64 && s->fold;
     using TG = typename MapStore<T>::type;
     um.G = f64 ? (const TG*)(const void*)s->d_G64 : (const TG*)(const void*)s->d_G16;
+    const int ne = (int)h->host.elems.size();
+    const int nshapes = f64 ? kSweepShapes : kWholeShapes;
     auto launch = [&](const Sweep::Shape& sh) {
+        const bool split = sh.split && !trace;   // a trace has one record per element
         um.reg_cap = sh.reg_cap;
         um.stage_cap = (int)(sh.smem / sizeof(T)) - 2 * rhs_cap;
         sweep_persistent_kernel<T><<<sh.grid, sh.threads, sh.smem, st>>>(
-            v, s->d_rec, s->rec_stride, (int)h->host.elems.size(), s->d_active, inv, r, z, s->d_next, s->d_status,
+            v, split ? s->d_rec_split : s->d_rec, s->rec_stride, split ? s->nsplit : ne, s->d_active, inv, r, z, s->d_next, s->d_status,
             um, rhs_cap, sh.bcap, trace), count_launch();
     };
     if (s->pick[pi] < 0) {
@@ -1391,9 +1619,10 @@ void apply_sweep(rtg_handle* h, const T* r, T* z, cudaStream_t st, unsigned long
         int dev = 0, nsm = 0;
         RTG_CUDA(cudaGetDevice(&dev));
         RTG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        for (int q = 0; q < kSweepShapes; ++q) {
+        for (int q = 0; q < nshapes; ++q) {
             Sweep::Shape& sh = s->shape[pi][q];
             const size_t budget = kShapeBudget[q];
+            sh.split = q >= kWholeShapes;
             sh.threads = kShapeThreads[q];
             const size_t rhs_bytes = sizeof(T) * (size_t)(2 * rhs_cap + s->max_c);
             const int64_t fit = (int64_t)((budget - std::min(rhs_bytes, budget)) / sizeof(T));
@@ -1405,7 +1634,7 @@ void apply_sweep(rtg_handle* h, const T* r, T* z, cudaStream_t st, unsigned long
             int per_sm = 0;
             RTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_persistent_kernel<T>, sh.threads,
                                                                    sh.smem));
-            sh.grid = std::max(1, std::min<int>((int)h->host.elems.size(), std::max(per_sm, 1) * nsm));
+            sh.grid = std::max(1, std::min<int>(sh.split ? s->nsplit : ne, std::max(per_sm, 1) * nsm));
         }
         // time each: rounds over all shapes (so that a drift of the clocks
         // meets every shape alike), the first round a warm-up, best of the
@@ -1415,7 +1644,7 @@ void apply_sweep(rtg_handle* h, const T* r, T* z, cudaStream_t st, unsigned long
         RTG_CUDA(cudaEventCreate(&e1));
         for (int q = 0; q < kSweepShapes; ++q) s->shape_ms[pi][q] = 1e30f;
         for (int rep = 0; rep < 6; ++rep)
-            for (int q = 0; q < kSweepShapes; ++q) {
+            for (int q = 0; q < nshapes; ++q) {
                 sweep_fill_kernel<T><<<std::max(1, std::min((int)h->host.elems.size(), 152 * 8)), 256, 0, st>>>(
                     v, (int)h->host.elems.size(), z, s->d_next), count_launch();
                 RTG_CUDA(cudaEventRecord(e0, st));
@@ -1429,7 +1658,7 @@ void apply_sweep(rtg_handle* h, const T* r, T* z, cudaStream_t st, unsigned long
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         int best_q = 0;
-        for (int q = 1; q < kSweepShapes; ++q)
+        for (int q = 1; q < nshapes; ++q)
             if (s->shape_ms[pi][q] < 0.97f * s->shape_ms[pi][best_q]) best_q = q;
         s->pick[pi] = best_q;
         // the real sweep below starts from a fresh fill
