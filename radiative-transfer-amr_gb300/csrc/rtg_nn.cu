@@ -29,7 +29,7 @@
 //   loss = sum_rows o^T G o - 2 q^T o + c,  o = C(row) m(z)/s.
 // The gradient kernel recomputes the forward pass per 64-row tile, forms
 // dL/dC = (dL/do) m^T, runs the backward pass in shared memory and keeps the
-// weight gradients of its tiles in registers; per-CTA partials are summed in a
+// weight gradients of its tiles in registers, one CTA per SM; per-CTA partials are summed in a
 // fixed order, so training is deterministic.
 #include <algorithm>
 #include <cmath>
@@ -45,10 +45,12 @@ namespace {
 constexpr int kIn = RTG_NN_IN, kHid = RTG_NN_HIDDEN, kOut = RTG_NN_OUT, kMom = RTG_NN_MOM;
 constexpr int kSt = RTG_NN_STATS;
 constexpr int kTile = 64;          // rows per tile
-constexpr int kLd = kTile + 4;     // row stride of the transposed activation tiles
-constexpr int kLdo = kOut + 1;     // row stride of dL/dC in shared memory (bank spread)
-constexpr int kMlpThreads = 256;
-constexpr int kGradCtas = 2 * 152;
+constexpr int kLd = kTile + 4;     // row stride of the transposed tiles: rows 4 banks apart
+constexpr int kLd2 = kHid + 4;     // row strides of W2 and W3 in shared memory: 16 bytes of
+constexpr int kLd3 = kOut + 4;     // eight consecutive rows lie in different banks
+constexpr int kMlpThreads = 512;
+constexpr int kGradCtas = 152;     // one per SM
+constexpr int kFeat = kTile * kIn / kMlpThreads;   // features of a tile per thread
 constexpr int oW1 = 0, ob1 = oW1 + kIn * kHid, oW2 = ob1 + kHid, ob2 = oW2 + kHid * kHid, oW3 = ob2 + kHid,
               ob3 = oW3 + kHid * kOut, kNP = ob3 + kOut;
 static_assert(kNP == RTG_NN_NPARAM, "parameter layout");
@@ -56,13 +58,13 @@ static_assert(kOut == 3 * kMom, "three output moments");
 static_assert(kOut % 4 == 0, "output rows are float4-aligned");
 constexpr float kTwoPi = 6.283185307179586f;
 
-// shared-memory layout of the MLP kernels (floats); the parameter layout is
-// the shared-memory layout of the first kNP floats; float4 regions start on
-// multiples of 4 floats
-constexpr int sF = (kNP + 3) / 4 * 4, sH1 = sF + kIn * kLd, sH2 = sH1 + kHid * kLd, sO = sH2 + kHid * kLd,
-              kSmemFloats = sO + kTile * kOut;
-static_assert(sF % 4 == 0 && sH1 % 4 == 0 && sH2 % 4 == 0 && sO % 4 == 0, "alignment");
-static_assert(oW2 % 4 == 0 && oW1 % 4 == 0, "weight rows are float4-aligned");
+// shared-memory layout of the MLP kernels (floats): parameters, then the
+// transposed tiles [feature or unit][row]; every region starts on 16 bytes
+constexpr int sW1 = 0, sB1 = sW1 + kIn * kHid, sW2 = sB1 + kHid, sB2 = sW2 + kHid * kLd2, sW3 = sB2 + kHid,
+              sB3 = sW3 + kHid * kLd3, sF = sB3 + (kOut + 3) / 4 * 4, sH1 = sF + kIn * kLd, sH2 = sH1 + kHid * kLd,
+              sD = sH2 + kHid * kLd, sO = sD + kHid * kLd, sG = sO + kOut * kLd, kSmemFloats = sG + kTile;
+static_assert(kLd % 4 == 0 && kLd2 % 4 == 0 && kLd3 % 4 == 0, "float4 rows");
+static_assert(kIn == 16 && kHid == 128 && kOut == 24 && kTile == 64 && kMlpThreads == 512, "thread tiles below");
 constexpr size_t kMlpSmem = sizeof(float) * kSmemFloats;
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
@@ -73,45 +75,71 @@ __device__ __forceinline__ bool bdry_node_n(int bm, int i, int j, int nx, int ny
 }
 
 __device__ void stage_params(const float* __restrict__ P, float* sm) {
-    for (int t = threadIdx.x; t < kNP; t += blockDim.x) {
-        const bool weight = t < ob1 || (t >= oW2 && t < ob2) || (t >= oW3 && t < ob3);
-        const float val = P[t];
-        sm[t] = weight ? bf16r(val) : val;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < kIn * kHid; t += kMlpThreads) sm[sW1 + t] = bf16r(P[oW1 + t]);
+#pragma unroll 8
+    for (int t = threadIdx.x; t < kHid * kHid; t += kMlpThreads)
+        sm[sW2 + t / kHid * kLd2 + t % kHid] = bf16r(P[oW2 + t]);
+#pragma unroll 6
+    for (int t = threadIdx.x; t < kHid * kOut; t += kMlpThreads)
+        sm[sW3 + t / kOut * kLd3 + t % kOut] = bf16r(P[oW3 + t]);
+    if (threadIdx.x < kHid) {
+        sm[sB1 + threadIdx.x] = P[ob1 + threadIdx.x];
+        sm[sB2 + threadIdx.x] = P[ob2 + threadIdx.x];
     }
+    if (threadIdx.x < kOut) sm[sB3 + threadIdx.x] = P[ob3 + threadIdx.x];
 }
 
-// outT[c][r] = relu(sum_k inT[k][r] W[k][c] + b[c]) for the 64-row tile;
-// thread: rows 4tr..4tr+3, columns 8tc..8tc+7
-template <int K>
+// Products of the 64-row tile with 128-wide layers: warp w takes rows
+// 16 (w & 3).. and columns 32 (w >> 2)..; its lanes 4 row groups of 4 (lane4) by
+// 8 columns or column groups (lane8).  Lanes that read the same 16 bytes differ in
+// lane bit 0 or 1: a float4 load then takes 2 passes of the shared memory, and 4
+// where neighbouring lanes read different ones (measured 2.2 and 4.0 clocks).
+__device__ __forceinline__ int lane4() { return (threadIdx.x >> 1) & 3; }
+__device__ __forceinline__ int lane8() { return (threadIdx.x & 1) | ((threadIdx.x >> 3) & 3) << 1; }
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// two FP32 multiply-adds in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<uint64_t&>(d))
+        : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+    return d;
+}
+__device__ __forceinline__ float2 lo2(const float4& a) { return make_float2(a.x, a.y); }
+__device__ __forceinline__ float2 hi2(const float4& a) { return make_float2(a.z, a.w); }
+
+__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+
+// outT[c][r] = relu(sum_k inT[k][r] W[k][c] + b[c]); thread: 4 rows x 4 columns
+template <int K, int LDW>
 __device__ __forceinline__ void layer_relu(const float* __restrict__ inT, const float* __restrict__ W,
                                            const float* __restrict__ b, float* __restrict__ outT) {
-    const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;
-    float acc[4][8];
+    const int w = threadIdx.x >> 5;
+    const int r0 = 16 * (w & 3) + 4 * lane4(), c0 = 32 * (w >> 2) + 4 * lane8();
+    float2 acc[2][4];   // [row pair][column]
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-#pragma unroll 4
+    for (int j = 0; j < 4; ++j) acc[0][j] = acc[1][j] = make_float2(0.f, 0.f);
+#pragma unroll 8
     for (int k = 0; k < K; ++k) {
-        const float4 a = *reinterpret_cast<const float4*>(inT + k * kLd + 4 * tr);
-        const float4 w0 = *reinterpret_cast<const float4*>(W + k * kHid + 8 * tc);
-        const float4 w1 = *reinterpret_cast<const float4*>(W + k * kHid + 8 * tc + 4);
-        const float av[4] = {a.x, a.y, a.z, a.w};
-        const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        const float4 a = ld4(inT + k * kLd + r0), x = ld4(W + k * LDW + c0);
+        const float wv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) {
+            const float2 ww = make_float2(wv[j], wv[j]);
+            acc[0][j] = fma2(lo2(a), ww, acc[0][j]);
+            acc[1][j] = fma2(hi2(a), ww, acc[1][j]);
+        }
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const float bj = b[8 * tc + j];
+    for (int j = 0; j < 4; ++j) {
+        const float bj = b[c0 + j];
         float4 o;
-        o.x = fmaxf(acc[0][j] + bj, 0.f);
-        o.y = fmaxf(acc[1][j] + bj, 0.f);
-        o.z = fmaxf(acc[2][j] + bj, 0.f);
-        o.w = fmaxf(acc[3][j] + bj, 0.f);
-        *reinterpret_cast<float4*>(outT + (8 * tc + j) * kLd + 4 * tr) = o;
+        o.x = fmaxf(acc[0][j].x + bj, 0.f);
+        o.y = fmaxf(acc[0][j].y + bj, 0.f);
+        o.z = fmaxf(acc[1][j].x + bj, 0.f);
+        o.w = fmaxf(acc[1][j].y + bj, 0.f);
+        *reinterpret_cast<float4*>(outT + (c0 + j) * kLd + r0) = o;
     }
 }
 
@@ -122,33 +150,52 @@ __device__ __forceinline__ float row_gate(float f0, float f1) {
 }
 
 // Forward pass of one tile: features into Ft, then h1T, h2T and the gated
-// outputs in sO[r][kOut] (thread: row t/4, outputs t%4 + 4u).
-__device__ __forceinline__ void forward_tile(const float* __restrict__ F, int64_t r0, int nr, float* sm) {
+// outputs in sO[c][r].
+// f holds this thread's features of the tile (load_features), which are loaded a
+// tile ahead.
+__device__ __forceinline__ void load_features(float (&f)[kFeat], const float* __restrict__ F, int64_t r0, int64_t rows) {
+#pragma unroll
+    for (int u = 0; u < kFeat; ++u) {
+        const int t = threadIdx.x + u * kMlpThreads;
+        f[u] = r0 + t / kIn < rows ? F[r0 * kIn + t] : 0.f;
+    }
+}
+__device__ __forceinline__ void forward_tile(const float (&f)[kFeat], float* sm) {
     float* Ft = sm + sF;
-    for (int t = threadIdx.x; t < kTile * kIn; t += blockDim.x) {
-        const int r = t / kIn, k = t % kIn;
-        Ft[k * kLd + r] = r < nr ? F[(r0 + r) * kIn + k] : 0.f;
+#pragma unroll
+    for (int u = 0; u < kFeat; ++u) {
+        const int t = threadIdx.x + u * kMlpThreads;
+        Ft[t % kIn * kLd + t / kIn] = f[u];
     }
     __syncthreads();
-    layer_relu<kIn>(Ft, sm + oW1, sm + ob1, sm + sH1);
+    if (threadIdx.x < kTile) sm[sG + threadIdx.x] = row_gate(Ft[threadIdx.x], Ft[kLd + threadIdx.x]);
+    layer_relu<kIn, kHid>(Ft, sm + sW1, sm + sB1, sm + sH1);
     __syncthreads();
-    layer_relu<kHid>(sm + sH1, sm + oW2, sm + ob2, sm + sH2);
+    layer_relu<kHid, kLd2>(sm + sH1, sm + sW2, sm + sB2, sm + sH2);
     __syncthreads();
-    const int r = threadIdx.x >> 2, c0 = threadIdx.x & 3;
-    const float* h2T = sm + sH2;
-    const float* W3 = sm + oW3;
-    float acc[kOut / 4];
+    if (threadIdx.x < 128) {   // one warp per scheduler, 6 columns each; lanes of 2 rows
+        const int r = 2 * (threadIdx.x & 31), c0 = 6 * (threadIdx.x >> 5);
+        float2 acc[2][3];   // [row][column pair]
 #pragma unroll
-    for (int u = 0; u < kOut / 4; ++u) acc[u] = sm[ob3 + c0 + 4 * u];
-#pragma unroll 4
-    for (int k = 0; k < kHid; ++k) {
-        const float hv = h2T[k * kLd + r];
+        for (int j = 0; j < 3; ++j) acc[0][j] = acc[1][j] = ld2(sm + sB3 + c0 + 2 * j);
+#pragma unroll 8
+        for (int k = 0; k < kHid; ++k) {
+            const float2 a = ld2(sm + sH2 + k * kLd + r);
 #pragma unroll
-        for (int u = 0; u < kOut / 4; ++u) acc[u] = fmaf(hv, W3[k * kOut + c0 + 4 * u], acc[u]);
+            for (int j = 0; j < 3; ++j) {
+                const float2 x = ld2(sm + sW3 + k * kLd3 + c0 + 2 * j);
+                acc[0][j] = fma2(make_float2(a.x, a.x), x, acc[0][j]);
+                acc[1][j] = fma2(make_float2(a.y, a.y), x, acc[1][j]);
+            }
+        }
+        const float2 g = ld2(sm + sG + r);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            float* o = sm + sO + (c0 + 2 * j) * kLd + r;
+            *reinterpret_cast<float2*>(o) = make_float2(g.x * acc[0][j].x, g.y * acc[1][j].x);
+            *reinterpret_cast<float2*>(o + kLd) = make_float2(g.x * acc[0][j].y, g.y * acc[1][j].y);
+        }
     }
-    const float g = row_gate(Ft[r], Ft[kLd + r]);
-#pragma unroll
-    for (int u = 0; u < kOut / 4; ++u) sm[sO + r * kOut + c0 + 4 * u] = g * acc[u];
     __syncthreads();
 }
 
@@ -156,67 +203,89 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
 nn_forward_kernel(const float* __restrict__ P, const float* __restrict__ F, int64_t rows, float* __restrict__ O) {
     extern __shared__ float4 smem4[];
     float* sm = reinterpret_cast<float*>(smem4);
+    float f[kFeat];
+    load_features(f, F, (int64_t)blockIdx.x * kTile, rows);
     stage_params(P, sm);
     __syncthreads();
     const int64_t ntiles = (rows + kTile - 1) / kTile;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t r0 = tile * kTile;
         const int nr = (int)(rows - r0 < kTile ? rows - r0 : kTile);
-        forward_tile(F, r0, nr, sm);
-        for (int t = threadIdx.x; t < nr * kOut; t += blockDim.x) O[r0 * kOut + t] = sm[sO + t];
+        forward_tile(f, sm);
+        load_features(f, F, (tile + gridDim.x) * kTile, rows);
+        for (int t = threadIdx.x; t < nr * kOut; t += blockDim.x) O[r0 * kOut + t] = sm[sO + t % kOut * kLd + t / kOut];
         __syncthreads();
     }
 }
 
 // Loss and gradient over all rows.  work[b][kNP] gets CTA b's gradient,
-// lossw[b] its loss.
+// lossw[b] its loss.  FP32 throughout (weights are BF16 values): 62e3
+// multiply-adds per row are 31e3 cycles of an SM's FP32 pipe per tile, and what
+// bounds it besides is the operands from shared memory.  Register tiles of 4 x 4
+// (forward, dh) and 4 x 8 (dW2) outputs per thread, lanes that share operands next
+// to each other, 16 warps in one CTA per SM, and dh2 and dh1 in buffers of their
+// own, so that two products run between barriers: 110 us at 32,768 rows (54e3
+// cycles per tile, 46e3 of them in the four 128-wide products), 182 us with 256
+// threads, scalar reads of dO, W3 and W2 and two CTAs in turn on half of the SMs.
+// The chains of the forward pass keep their order of k, so the loss does not
+// depend on the tiling.
 __global__ void __launch_bounds__(kMlpThreads, 1)
 nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const float* __restrict__ Mo,
                const float* __restrict__ S, int64_t rows, float* __restrict__ work, double* __restrict__ lossw) {
     extern __shared__ float4 smem4[];
     float* sm = reinterpret_cast<float*>(smem4);
-    __shared__ float dO[kTile * kLdo];
-    __shared__ double red[kMlpThreads / 32];
+    __shared__ double red[kTile / 32];
+    float f[kFeat];
+    load_features(f, F, (int64_t)blockIdx.x * kTile, rows);
     stage_params(P, sm);
     __syncthreads();
-    const int t = threadIdx.x;
-    constexpr int kW3PerThread = kHid * kOut / kMlpThreads;
-    float gW2[8][8], gW1[8], gW3[kW3PerThread], gb1 = 0.f, gb2 = 0.f, gb3 = 0.f;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int l4 = lane4(), l8 = lane8();
+    // gradients of this thread, over the CTA's tiles
+    float gW2[4][8];                 // k = 32 (w & 3) + l8 + 8p, c = 32 (w >> 2) + l4 + 4q
+    float gW1[2][2];                 // k = l8 + 8p, c = 8w + l4 + 4q
+    float gW3[2][3];                 // k = 16 (w >> 1) + l8 + 8p, c = 12 (w & 1) + 3 l4 + q
+    float gb1[4], gb2[4], gb3[3];    // units 32 (w >> 2) + l8 + 8j over 4 rows; outputs as gW3
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-        gW1[p] = 0.f;
+    for (int p = 0; p < 4; ++p) {
+        gb1[p] = gb2[p] = 0.f;
 #pragma unroll
         for (int q = 0; q < 8; ++q) gW2[p][q] = 0.f;
     }
 #pragma unroll
-    for (int u = 0; u < kW3PerThread; ++u) gW3[u] = 0.f;
+    for (int p = 0; p < 2; ++p) {
+        gW1[p][0] = gW1[p][1] = 0.f;
+        gW3[p][0] = gW3[p][1] = gW3[p][2] = 0.f;
+    }
+    gb3[0] = gb3[1] = gb3[2] = 0.f;
     double loss = 0.;
     float* Ft = sm + sF;
     float* h1T = sm + sH1;
     float* h2T = sm + sH2;
-    const float* W2 = sm + oW2;
-    const float* W3 = sm + oW3;
+    float* dT = sm + sD;
+    float* dOT = sm + sO;
     const int64_t ntiles = (rows + kTile - 1) / kTile;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t r0 = tile * kTile;
         const int nr = (int)(rows - r0 < kTile ? rows - r0 : kTile);
-        forward_tile(F, r0, nr, sm);
-        // o = C m, loss, dL/dC = (dL/do) m^T
+        // the row's moments and statistics, in flight during the forward pass
+        float m[kMom], s[10];
+#pragma unroll
+        for (int l = 0; l < kMom; ++l) m[l] = t < nr ? Mo[(r0 + t) * kMom + l] : 0.f;
+#pragma unroll
+        for (int l = 0; l < 10; ++l) s[l] = t < nr ? S[(r0 + t) * kSt + l] : 0.f;
+        forward_tile(f, sm);
+        load_features(f, F, (tile + gridDim.x) * kTile, rows);
+        // o = C m, loss, dL/dC = (dL/do) m^T, and dL/d(pre-gate outputs) = g dL/dC in place of C
         if (t < kTile) {
-            float m[kMom], d[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-            for (int l = 0; l < kMom; ++l) m[l] = 0.f;
+            float d[3] = {0.f, 0.f, 0.f};
             if (t < nr) {
-                const float* s = S + (r0 + t) * kSt;
-                const float* mg = Mo + (r0 + t) * kMom;
-#pragma unroll
-                for (int l = 0; l < kMom; ++l) m[l] = mg[l];
                 float o[3];
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     float a = 0.f;
 #pragma unroll
-                    for (int l = 0; l < kMom; ++l) a = fmaf(sm[sO + t * kOut + kMom * k + l], m[l], a);
+                    for (int l = 0; l < kMom; ++l) a = fmaf(dOT[(kMom * k + l) * kLd + t], m[l], a);
                     o[k] = a;
                 }
                 const float g0 = s[0] * o[0] + s[1] * o[1] + s[2] * o[2];
@@ -228,153 +297,214 @@ nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const f
                 d[1] = 2.f * (g1 - s[7]);
                 d[2] = 2.f * (g2 - s[8]);
             }
-            // dL/d(pre-gate outputs) = g dL/dC
-            const float g = row_gate(Ft[t], Ft[kLd + t]);
+            const float g = sm[sG + t];
 #pragma unroll
             for (int k = 0; k < 3; ++k)
 #pragma unroll
-                for (int l = 0; l < kMom; ++l) dO[t * kLdo + kMom * k + l] = g * d[k] * m[l];
+                for (int l = 0; l < kMom; ++l) dOT[(kMom * k + l) * kLd + t] = g * d[k] * m[l];
         }
         __syncthreads();
-        // dW3, db3
-#pragma unroll
-        for (int u = 0; u < kW3PerThread; ++u) {
-            const int idx = t + kMlpThreads * u, k = idx / kOut, c = idx % kOut;
-            float a = 0.f;
-            for (int r = 0; r < kTile; ++r) a = fmaf(h2T[k * kLd + r], dO[r * kLdo + c], a);
-            gW3[u] += a;
-        }
-        if (t < kOut)
-            for (int r = 0; r < kTile; ++r) gb3 += dO[r * kLdo + t];
-        __syncthreads();
-        // dh2 = (dO W3^T) * [h2 > 0], in place
+        // dW3[k][c] += sum_r h2[r][k] dO[r][c], db3[c] += sum_r dO[r][c]
         {
-            const int tr = t & 15, tc = t >> 4;
-#pragma unroll 2
-            for (int j = 0; j < 8; ++j) {
-                const int k = 8 * tc + j;
-                float4 hv = *reinterpret_cast<float4*>(h2T + k * kLd + 4 * tr);
-                float* hp = &hv.x;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = 4 * tr + i;
-                    float dsum = 0.f;
-#pragma unroll
-                    for (int c = 0; c < kOut; ++c) dsum = fmaf(dO[r * kLdo + c], W3[k * kOut + c], dsum);
-                    hp[i] = hp[i] > 0.f ? dsum : 0.f;
-                }
-                *reinterpret_cast<float4*>(h2T + k * kLd + 4 * tr) = hv;
-            }
-        }
-        __syncthreads();
-        if (t < kHid)
-            for (int r = 0; r < kTile; ++r) gb2 += h2T[t * kLd + r];
-        // dW2[k][c] += sum_r h1[r][k] dh2[r][c]; k = tk + 16p, c = 8tc + q
-        {
-            const int tk = t & 15, tc = t >> 4;
+            const float* hp = h2T + (16 * (w >> 1) + l8) * kLd;
+            const float* dp = dOT + (12 * (w & 1) + 3 * l4) * kLd;
+#pragma unroll 4
             for (int r = 0; r < kTile; r += 4) {
-                float4 a[8], b[8];
+                float4 a[2], b[3];
 #pragma unroll
-                for (int p = 0; p < 8; ++p) a[p] = *reinterpret_cast<const float4*>(h1T + (tk + 16 * p) * kLd + r);
+                for (int p = 0; p < 2; ++p) a[p] = ld4(hp + 8 * p * kLd + r);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) b[q] = *reinterpret_cast<const float4*>(h2T + (8 * tc + q) * kLd + r);
+                for (int q = 0; q < 3; ++q) b[q] = ld4(dp + q * kLd + r);
 #pragma unroll
-                for (int p = 0; p < 8; ++p)
+                for (int p = 0; p < 2; ++p)
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        gW2[p][q] = fmaf(a[p].x, b[q].x,
-                                         fmaf(a[p].y, b[q].y, fmaf(a[p].z, b[q].z, fmaf(a[p].w, b[q].w, gW2[p][q]))));
+                    for (int q = 0; q < 3; ++q)
+                        gW3[p][q] = fmaf(a[p].x, b[q].x,
+                                         fmaf(a[p].y, b[q].y, fmaf(a[p].z, b[q].z, fmaf(a[p].w, b[q].w, gW3[p][q]))));
+                if (w < 2)
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) gb3[q] += (b[q].x + b[q].y) + (b[q].z + b[q].w);
             }
         }
-        __syncthreads();
-        // dh1 = (dh2 W2^T) * [h1 > 0], in place; rows 4tr.., k = tk + 16p
+        // dh2[r][k] = [h2 > 0] sum_c dO[r][c] W3[k][c], and db2
+        const int rr = 16 * (w & 3) + 4 * l4, kk = 32 * (w >> 2) + l8;   // 4 rows, units kk + 8j
         {
-            const int tr = t & 15, tk = t >> 4;
-            float acc[8][4];
+            float2 acc[4][2];   // [unit][row pair]
 #pragma unroll
-            for (int p = 0; p < 8; ++p)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[p][i] = 0.f;
+            for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_float2(0.f, 0.f);
 #pragma unroll 2
-            for (int c = 0; c < kHid; ++c) {
-                const float4 d = *reinterpret_cast<const float4*>(h2T + c * kLd + 4 * tr);
+            for (int c = 0; c < kOut; c += 4) {
+                float4 d[4];
 #pragma unroll
-                for (int p = 0; p < 8; ++p) {
-                    const float w = W2[(tk + 16 * p) * kHid + c];
-                    acc[p][0] = fmaf(d.x, w, acc[p][0]);
-                    acc[p][1] = fmaf(d.y, w, acc[p][1]);
-                    acc[p][2] = fmaf(d.z, w, acc[p][2]);
-                    acc[p][3] = fmaf(d.w, w, acc[p][3]);
+                for (int u = 0; u < 4; ++u) d[u] = ld4(dOT + (c + u) * kLd + rr);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 x = ld4(sm + sW3 + (kk + 8 * j) * kLd3 + c);
+                    const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float2 xx = make_float2(xv[u], xv[u]);
+                        acc[j][0] = fma2(lo2(d[u]), xx, acc[j][0]);
+                        acc[j][1] = fma2(hi2(d[u]), xx, acc[j][1]);
+                    }
                 }
             }
 #pragma unroll
-            for (int p = 0; p < 8; ++p) {
-                float4 hv = *reinterpret_cast<float4*>(h1T + (tk + 16 * p) * kLd + 4 * tr);
-                hv.x = hv.x > 0.f ? acc[p][0] : 0.f;
-                hv.y = hv.y > 0.f ? acc[p][1] : 0.f;
-                hv.z = hv.z > 0.f ? acc[p][2] : 0.f;
-                hv.w = hv.w > 0.f ? acc[p][3] : 0.f;
-                *reinterpret_cast<float4*>(h1T + (tk + 16 * p) * kLd + 4 * tr) = hv;
+            for (int j = 0; j < 4; ++j) {
+                const int at = (kk + 8 * j) * kLd + rr;
+                float4 hv = ld4(h2T + at);
+                hv.x = hv.x > 0.f ? acc[j][0].x : 0.f;
+                hv.y = hv.y > 0.f ? acc[j][0].y : 0.f;
+                hv.z = hv.z > 0.f ? acc[j][1].x : 0.f;
+                hv.w = hv.w > 0.f ? acc[j][1].y : 0.f;
+                *reinterpret_cast<float4*>(dT + at) = hv;
+                gb2[j] += (hv.x + hv.y) + (hv.z + hv.w);
             }
         }
         __syncthreads();
-        if (t < kHid)
-            for (int r = 0; r < kTile; ++r) gb1 += h1T[t * kLd + r];
-        // dW1[k][c] += sum_r F[r][k] dh1[r][c]; k = t & 15, c = 8 (t >> 4) + q
+        // dW2[k][c] += sum_r h1[r][k] dh2[r][c]
         {
-            const int k = t & 15, c0 = 8 * (t >> 4);
+            const float* hp = h1T + (32 * (w & 3) + l8) * kLd;
+            const float* dp = dT + (32 * (w >> 2) + l4) * kLd;
+#pragma unroll 1
             for (int r = 0; r < kTile; r += 4) {
-                const float4 a = *reinterpret_cast<const float4*>(Ft + k * kLd + r);
+                float4 a[4];
+#pragma unroll
+                for (int p = 0; p < 4; ++p) a[p] = ld4(hp + 8 * p * kLd + r);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const float4 b = *reinterpret_cast<const float4*>(h1T + (c0 + q) * kLd + r);
-                    gW1[q] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, gW1[q]))));
+                    const float4 b = ld4(dp + 4 * q * kLd + r);
+#pragma unroll
+                    for (int p = 0; p < 4; ++p)
+                        gW2[p][q] = fmaf(a[p].x, b.x,
+                                         fmaf(a[p].y, b.y, fmaf(a[p].z, b.z, fmaf(a[p].w, b.w, gW2[p][q]))));
                 }
+            }
+        }
+        // dh1[r][k] = [h1 > 0] sum_c dh2[r][c] W2[k][c] in place of h2, and db1
+        {
+            float2 acc[4][2];   // [unit][row pair]
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_float2(0.f, 0.f);
+#pragma unroll 2
+            for (int c = 0; c < kHid; c += 4) {
+                float4 d[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) d[u] = ld4(dT + (c + u) * kLd + rr);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 x = ld4(sm + sW2 + (kk + 8 * j) * kLd2 + c);
+                    const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float2 xx = make_float2(xv[u], xv[u]);
+                        acc[j][0] = fma2(lo2(d[u]), xx, acc[j][0]);
+                        acc[j][1] = fma2(hi2(d[u]), xx, acc[j][1]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int at = (kk + 8 * j) * kLd + rr;
+                float4 hv = ld4(h1T + at);
+                hv.x = hv.x > 0.f ? acc[j][0].x : 0.f;
+                hv.y = hv.y > 0.f ? acc[j][0].y : 0.f;
+                hv.z = hv.z > 0.f ? acc[j][1].x : 0.f;
+                hv.w = hv.w > 0.f ? acc[j][1].y : 0.f;
+                *reinterpret_cast<float4*>(h2T + at) = hv;
+                gb1[j] += (hv.x + hv.y) + (hv.z + hv.w);
+            }
+        }
+        __syncthreads();
+        // dW1[k][c] += sum_r F[r][k] dh1[r][c]
+        {
+            const float* fp = Ft + l8 * kLd;
+            const float* dp = h2T + (8 * w + l4) * kLd;
+#pragma unroll 4
+            for (int r = 0; r < kTile; r += 4) {
+                float4 a[2], b[2];
+#pragma unroll
+                for (int p = 0; p < 2; ++p) a[p] = ld4(fp + 8 * p * kLd + r), b[p] = ld4(dp + 4 * p * kLd + r);
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        gW1[p][q] = fmaf(a[p].x, b[q].x,
+                                         fmaf(a[p].y, b[q].y, fmaf(a[p].z, b[q].z, fmaf(a[p].w, b[q].w, gW1[p][q]))));
             }
         }
         __syncthreads();
     }
-    // per-CTA partials
+    // per-CTA partials; the bias partials of the 16 row groups meet in shared memory
     float* g = work + (int64_t)blockIdx.x * kNP;
     {
-        const int tk = t & 15, tc = t >> 4;
 #pragma unroll
-        for (int p = 0; p < 8; ++p)
+        for (int p = 0; p < 4; ++p)
 #pragma unroll
-            for (int q = 0; q < 8; ++q) g[oW2 + (tk + 16 * p) * kHid + 8 * tc + q] = gW2[p][q];
-        const int k = t & 15, c0 = 8 * (t >> 4);
+            for (int q = 0; q < 8; ++q)
+                sm[sW2 + (32 * (w & 3) + l8 + 8 * p) * kLd2 + 32 * (w >> 2) + l4 + 4 * q] = gW2[p][q];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) g[oW1 + k * kHid + c0 + q] = gW1[q];
+        for (int p = 0; p < 2; ++p) {
 #pragma unroll
-        for (int u = 0; u < kW3PerThread; ++u) g[oW3 + t + kMlpThreads * u] = gW3[u];
-        if (t < kHid) {
-            g[ob1 + t] = gb1;
-            g[ob2 + t] = gb2;
+            for (int q = 0; q < 2; ++q) g[oW1 + (l8 + 8 * p) * kHid + 8 * w + l4 + 4 * q] = gW1[p][q];
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                g[oW3 + (16 * (w >> 1) + l8 + 8 * p) * kOut + 12 * (w & 1) + 3 * l4 + q] = gW3[p][q];
         }
-        if (t < kOut) g[ob3 + t] = gb3;
+        if (w < 2 && l8 == 0)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) g[ob3 + 12 * w + 3 * l4 + q] = gb3[q];
+        float* b1 = sm + sH1;   // [unit][row group]
+        float* b2 = sm + sH2;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int at = (32 * (w >> 2) + l8 + 8 * j) * kLd + 4 * (w & 3) + l4;
+            b1[at] = gb1[j];
+            b2[at] = gb2[j];
+        }
     }
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, o);
-    if ((t & 31) == 0) red[t >> 5] = loss;
+    if (t < kTile && lane == 0) red[w] = loss;
     __syncthreads();
-    if (t == 0) {
-        double s = 0.;
-        for (int w = 0; w < kMlpThreads / 32; ++w) s += red[w];
-        lossw[blockIdx.x] = s;
+#pragma unroll 8
+    for (int i = t; i < kHid * kHid; i += kMlpThreads) g[oW2 + i] = sm[sW2 + i / kHid * kLd2 + i % kHid];
+    if (t < 2 * kHid) {
+        const int u = t % kHid;
+        const float* b = sm + (t < kHid ? sH1 : sH2) + u * kLd;
+        float a = 0.f;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) a += b[r];
+        g[(t < kHid ? ob1 : ob2) + u] = a;
     }
+    if (t == 0) lossw[blockIdx.x] = red[0] + red[1];
 }
 
-__global__ void nn_reduce_grad_kernel(const float* __restrict__ work, int nb, const double* __restrict__ lossw,
-                                      float* __restrict__ grad, double* __restrict__ loss) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < kNP) {
-        float s = 0.f;
-        for (int b = 0; b < nb; ++b) s += work[(int64_t)b * kNP + p];
-        grad[p] = s;
+// grad[p] = sum over the nb partials, in kRedSlices interleaved sums: one warp
+// reads 32 neighbouring parameters of a partial, and a block's slices read as many
+// partials at once (304 partials summed by one thread per parameter took 34 us, this
+// takes 4).
+constexpr int kRedParams = 32, kRedSlices = 8;
+__global__ void __launch_bounds__(kRedParams * kRedSlices)
+nn_reduce_grad_kernel(const float* __restrict__ work, int nb, const double* __restrict__ lossw,
+                      float* __restrict__ grad, double* __restrict__ loss) {
+    __shared__ float part[kRedSlices][kRedParams];
+    const int l = threadIdx.x % kRedParams, sl = threadIdx.x / kRedParams, p = blockIdx.x * kRedParams + l;
+    float s = 0.f;
+    if (p < kNP)
+#pragma unroll 8
+        for (int b = sl; b < nb; b += kRedSlices) s += work[(int64_t)b * kNP + p];
+    part[sl][l] = s;
+    if (blockIdx.x == 0 && sl == kRedSlices - 1 && loss) {
+        double a = 0.;
+        for (int b = l; b < nb; b += 32) a += lossw[b];
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+        if (l == 0) *loss = a;
     }
-    if (p == 0 && loss) {
-        double s = 0.;
-        for (int b = 0; b < nb; ++b) s += lossw[b];
-        *loss = s;
+    __syncthreads();
+    if (sl == 0 && p < kNP) {
+#pragma unroll
+        for (int k = 1; k < kRedSlices; ++k) s += part[k][l];
+        grad[p] = s;
     }
 }
 
@@ -807,7 +937,7 @@ void nn_forward(const float* params, const float* feat, int64_t rows, float* coe
     if (rows <= 0) return;
     mlp_attributes();
     const int64_t ntiles = (rows + kTile - 1) / kTile;
-    const int grid = (int)std::min<int64_t>(ntiles, 152);
+    const int grid = (int)std::min<int64_t>(ntiles, kGradCtas);
     nn_forward_kernel<<<grid, kMlpThreads, kMlpSmem, s>>>(params, feat, rows, coef), count_launch();
     RTG_CUDA(cudaGetLastError());
 }
@@ -885,7 +1015,7 @@ void nn_loss_grad(const float* params, const float* feat, const float* mom, cons
     double* lossw = reinterpret_cast<double*>(work + (int64_t)kGradCtas * kNP);
     nn_grad_kernel<<<grid, kMlpThreads, kMlpSmem, s>>>(params, feat, mom, stats, std::max<int64_t>(rows, 0), work,
                                                        lossw), count_launch();
-    nn_reduce_grad_kernel<<<(kNP + 255) / 256, 256, 0, s>>>(work, grid, lossw, grad, loss), count_launch();
+    nn_reduce_grad_kernel<<<(kNP + kRedParams - 1) / kRedParams, kRedParams * kRedSlices, 0, s>>>(work, grid, lossw, grad, loss), count_launch();
     RTG_CUDA(cudaGetLastError());
 }
 
