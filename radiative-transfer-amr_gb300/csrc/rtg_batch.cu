@@ -6,9 +6,13 @@
 // inner products are segmented by instance, the Hessenberg matrix, Givens
 // rotations and convergence flags of each instance live on the device and
 // are updated by one thread per instance, and a converged instance's basis is
-// frozen.  One GMRES restart cycle (m Arnoldi steps, the correction and its
-// sweep) is a fixed kernel sequence, captured once in a CUDA graph and
-// replayed; the host reads the per-instance flags once per cycle.
+// frozen.  The start of a GMRES restart cycle, each Arnoldi step and the end
+// (the correction and its sweep) are fixed kernel sequences, captured once in
+// CUDA graphs and replayed; the host queues step j + 1, then reads whether step j
+// finished the last instance, so the GPU never waits for it and a cycle runs at
+// most one step (whose launches return at once) too many.  A cycle that always ran its
+// m = 30 steps spent 40 % of the solve of 64 instances of 72,000 DOF on steps with
+// nothing left to do.
 //
 // method 1 (the batched workload's method): FP64 iterative refinement around
 // FP32 sweep-preconditioned GMRES; method 0: FP64 GMRES.
@@ -73,11 +77,9 @@ __global__ void bdot_kernel(const BChunk* __restrict__ ch, const T* __restrict__
     }
 }
 
-// out[b*ldo + q] = sum of the partials of instance b; with add, also
-// out_sum[b*ldo + q] = out + add.
+// out[b*ldo + q] = sum of the partials of instance b
 __global__ void breduce_kernel(const int32_t* __restrict__ cbeg, const double* __restrict__ partial, int k,
-                               double* __restrict__ out, int ldo, const double* __restrict__ add,
-                               double* __restrict__ out_sum) {
+                               double* __restrict__ out, int ldo) {
     const int b = blockIdx.x, q = blockIdx.y;
     double s = 0.;
     for (int c = cbeg[b] + threadIdx.x; c < cbeg[b + 1]; c += blockDim.x) s += partial[(int64_t)c * k + q];
@@ -89,56 +91,207 @@ __global__ void breduce_kernel(const int32_t* __restrict__ cbeg, const double* _
         double t = 0.;
         for (int wq = 0; wq < (int)(blockDim.x + 31) / 32; ++wq) t += red[wq];
         out[b * ldo + q] = t;
-        if (add) out_sum[b * ldo + q] = t + add[b * ldo + q];
     }
 }
 
-// w -= sum_{q<k} h[b][q] V_q on the chunk's instance b
-template <typename T>
-__global__ void baxpy_kernel(const BChunk* __restrict__ ch, T* __restrict__ w, const T* __restrict__ V, int64_t ldv,
-                             int k, const double* __restrict__ h, int ldh, const int32_t* __restrict__ done) {
-    __shared__ T hs[64];
-    const BChunk c = ch[blockIdx.x];
-    if (done && done[c.inst]) return;
-    if (threadIdx.x < k) hs[threadIdx.x] = (T)h[c.inst * ldh + threadIdx.x];
+// The partials of an Arnoldi step's sums: k values each, those of instance b from
+// beg[b] to beg[b + 1].  Every block that needs an instance's sums adds them itself (in one
+// order, so all get the same), which saves a launch of 4.5 us between two passes of
+// 10; above kOwnSums partials per instance breduce_kernel leaves one.
+struct BSums {
+    const double* partial;
+    const int32_t* beg;
+};
+constexpr int kOwnSums = 64;
+
+// out[q] = the sums of instance b, for the block's threads
+__device__ __forceinline__ void inst_sums(BSums sums, int b, int k, double* out) {
+    const int lane = threadIdx.x & 31, c0 = sums.beg[b], c1 = sums.beg[b + 1];
+    for (int q = threadIdx.x >> 5; q < k; q += kBThreads / 32) {
+        double s = 0.;
+        for (int c = c0 + lane; c < c1; c += 32) s += sums.partial[(int64_t)c * k + q];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) out[q] = s;
+    }
     __syncthreads();
-    for (int64_t i = c.begin + threadIdx.x; i < c.end; i += blockDim.x) {
-        T sv = w[i];
-        for (int q = 0; q < k; ++q) sv = fma(-hs[q], V[(int64_t)q * ldv + i], sv);
-        w[i] = sv;
+}
+
+// A chunk of a vector in the block's registers
+constexpr int kBPer = kBChunk / kBThreads;
+__device__ __forceinline__ void load_chunk(float (&w)[kBPer], const float* __restrict__ p, int n) {
+#pragma unroll
+    for (int u = 0; u < kBPer; ++u) w[u] = (int)threadIdx.x + u * kBThreads < n ? p[threadIdx.x + u * kBThreads] : 0.f;
+}
+__device__ __forceinline__ void store_chunk(const float (&w)[kBPer], float* __restrict__ p, int n) {
+#pragma unroll
+    for (int u = 0; u < kBPer; ++u)
+        if ((int)threadIdx.x + u * kBThreads < n) p[threadIdx.x + u * kBThreads] = w[u];
+}
+// w -= sum_{q<k} h[q] V_q
+__device__ __forceinline__ void axpy_chunk(float (&w)[kBPer], const float* __restrict__ V, int64_t ldv, int k,
+                                           const double* h, int n) {
+    for (int q = 0; q < k; ++q) {
+        float v[kBPer];
+        load_chunk(v, V + (int64_t)q * ldv, n);
+        const float hq = (float)h[q];
+#pragma unroll
+        for (int u = 0; u < kBPer; ++u) w[u] = fmaf(-hq, v[u], w[u]);
+    }
+}
+// partial of <w, w>: per element and warp in FP32, double from the warps' sums on
+__device__ __forceinline__ void norm_chunk(const float (&w)[kBPer], double* partial) {
+    __shared__ double red[kBThreads / 32];
+    float s = 0.f;
+#pragma unroll
+    for (int u = 0; u < kBPer; ++u) s = fmaf(w[u], w[u], s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (double)s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.;
+        for (int wq = 0; wq < kBThreads / 32; ++wq) t += red[wq];
+        *partial = t;
+    }
+}
+// partials of <V_q, w>, q < k
+__device__ __forceinline__ void dot_chunk(const float (&w)[kBPer], const float* __restrict__ V, int64_t ldv, int k,
+                                          int n, double* partial) {
+    __shared__ double red[kBGroup][kBThreads / 32];
+    for (int g0 = 0; g0 < k; g0 += kBGroup) {
+        const int gk = min(kBGroup, k - g0);
+        float acc[kBGroup];
+#pragma unroll
+        for (int q = 0; q < kBGroup; ++q) {
+            acc[q] = 0.f;
+            if (q < gk) {
+                float v[kBPer];
+                load_chunk(v, V + (int64_t)(g0 + q) * ldv, n);
+#pragma unroll
+                for (int u = 0; u < kBPer; ++u) acc[q] = fmaf(v[u], w[u], acc[q]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kBGroup; ++q) {
+            float sw = acc[q];
+            for (int o = 16; o > 0; o >>= 1) sw += __shfl_down_sync(0xffffffffu, sw, o);
+            if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = (double)sw;
+        }
+        __syncthreads();
+        if (threadIdx.x < gk) {
+            double s = 0.;
+            for (int wq = 0; wq < kBThreads / 32; ++wq) s += red[threadIdx.x][wq];
+            partial[g0 + threadIdx.x] = s;
+        }
+        __syncthreads();
     }
 }
 
-// out = w / sqrt(nsq[b]); hcol[b*ldh + jcol] = sqrt(nsq[b]) (first chunk of b)
-template <typename T>
-__global__ void bnormalize_kernel(const BChunk* __restrict__ ch, const int32_t* __restrict__ cbeg,
-                                  const T* __restrict__ w, T* __restrict__ out, const double* __restrict__ nsq,
-                                  int ldn, double* __restrict__ hcol, int ldh, int jcol,
-                                  const int32_t* __restrict__ done) {
+// w = rhs - s and its norm's partials
+__global__ void __launch_bounds__(kBThreads)
+bresid_kernel(const BChunk* __restrict__ ch, const float* __restrict__ rhs, const float* __restrict__ sv,
+              float* __restrict__ w, double* __restrict__ partial) {
     const BChunk c = ch[blockIdx.x];
-    if (done && done[c.inst]) return;
-    const double nr = sqrt(nsq[c.inst * ldn]);
-    if (hcol && threadIdx.x == 0 && cbeg[c.inst] == (int)blockIdx.x) hcol[c.inst * ldh + jcol] = nr;
-    const T inv = (T)(nr > 0. ? 1. / nr : 0.);
-    for (int64_t i = c.begin + threadIdx.x; i < c.end; i += blockDim.x) out[i] = w[i] * inv;
+    const int n = (int)(c.end - c.begin);
+    float a[kBPer], b[kBPer];
+    load_chunk(a, rhs + c.begin, n);
+    load_chunk(b, sv + c.begin, n);
+#pragma unroll
+    for (int u = 0; u < kBPer; ++u) a[u] -= b[u];
+    store_chunk(a, w + c.begin, n);
+    norm_chunk(a, partial + blockIdx.x);
 }
 
-// x += scale[b] * sum_{q < kb[b]} y[b][q] V_q
-template <typename TV, typename TX>
-__global__ void bcombine_kernel(const BChunk* __restrict__ ch, TX* __restrict__ x, const TV* __restrict__ V,
-                                int64_t ldv, const int32_t* __restrict__ kb, const double* __restrict__ y, int ldy) {
-    using A = typename std::conditional<sizeof(TV) == 4 && sizeof(TX) == 4, float, double>::type;
-    __shared__ A ys[64];
-    __shared__ int s_k;
+// The passes of classical Gram-Schmidt with reorthogonalisation over the k basis
+// vectors of the chunk's instance, w in registers: <V, w>; then w -= V h1 and
+// <V, w> again; then w -= V h2 and <w, w>.  Each is bound by reading V (twice in
+// the second, the second time from L2 or L1).
+__global__ void __launch_bounds__(kBThreads)
+bdots_kernel(const BChunk* __restrict__ ch, const float* __restrict__ V, int64_t ldv, int k,
+             const float* __restrict__ w, double* __restrict__ partial, const int32_t* __restrict__ done) {
     const BChunk c = ch[blockIdx.x];
-    if (threadIdx.x == 0) s_k = kb[c.inst];
-    if (threadIdx.x < 64) ys[threadIdx.x] = (A)y[c.inst * ldy + min((int)threadIdx.x, ldy - 1)];
+    if (done[c.inst]) return;
+    const int n = (int)(c.end - c.begin);
+    float wr[kBPer];
+    load_chunk(wr, w + c.begin, n);
+    dot_chunk(wr, V + c.begin, ldv, k, n, partial + (int64_t)blockIdx.x * k);
+}
+
+__global__ void __launch_bounds__(kBThreads)
+baxpy_dots_kernel(const BChunk* __restrict__ ch, const int32_t* __restrict__ cbeg, BSums sums,
+                  const float* __restrict__ V, int64_t ldv, int k, float* __restrict__ w, double* __restrict__ h1,
+                  int ldh, double* __restrict__ partial, const int32_t* __restrict__ done) {
+    __shared__ double h[64];
+    const BChunk c = ch[blockIdx.x];
+    if (done[c.inst]) return;
+    const int n = (int)(c.end - c.begin);
+    float wr[kBPer];
+    load_chunk(wr, w + c.begin, n);
+    inst_sums(sums, c.inst, k, h);
+    if (cbeg[c.inst] == (int)blockIdx.x && threadIdx.x < k) h1[c.inst * ldh + threadIdx.x] = h[threadIdx.x];
+    axpy_chunk(wr, V + c.begin, ldv, k, h, n);
+    store_chunk(wr, w + c.begin, n);
+    dot_chunk(wr, V + c.begin, ldv, k, n, partial + (int64_t)blockIdx.x * k);
+}
+
+// ho = h1 + h2
+__global__ void __launch_bounds__(kBThreads)
+baxpy_norm_kernel(const BChunk* __restrict__ ch, const int32_t* __restrict__ cbeg, BSums sums,
+                  const float* __restrict__ V, int64_t ldv, int k, float* __restrict__ w,
+                  const double* __restrict__ h1, double* __restrict__ ho, int ldh, double* __restrict__ partial,
+                  const int32_t* __restrict__ done) {
+    __shared__ double h[64];
+    const BChunk c = ch[blockIdx.x];
+    if (done[c.inst]) return;
+    const int n = (int)(c.end - c.begin);
+    float wr[kBPer];
+    load_chunk(wr, w + c.begin, n);
+    inst_sums(sums, c.inst, k, h);
+    if (cbeg[c.inst] == (int)blockIdx.x && threadIdx.x < k)
+        ho[c.inst * ldh + threadIdx.x] = h[threadIdx.x] + h1[c.inst * ldh + threadIdx.x];
+    axpy_chunk(wr, V + c.begin, ldv, k, h, n);
+    store_chunk(wr, w + c.begin, n);
+    norm_chunk(wr, partial + blockIdx.x);
+}
+
+// out = w / ||w||, the norm into nrm[b*ldn] (first chunk of b), and the sentinel
+// over z, the output of the sweep that follows (its claim counter is reset by the
+// step kernels below)
+__global__ void __launch_bounds__(kBThreads)
+bnormalize_kernel(const BChunk* __restrict__ ch, const int32_t* __restrict__ cbeg, BSums sums,
+                  const float* __restrict__ w, float* __restrict__ out, double* __restrict__ nrm, int ldn,
+                  float* __restrict__ z, const int32_t* __restrict__ done) {
+    __shared__ double s_sq;
+    __shared__ float s_inv;
+    const BChunk c = ch[blockIdx.x];
+    if (done && done[c.inst]) return;
+    inst_sums(sums, c.inst, 1, &s_sq);
+    if (threadIdx.x == 0) {
+        const double nr = sqrt(s_sq);
+        s_inv = (float)(nr > 0. ? 1. / nr : 0.);
+        if (cbeg[c.inst] == (int)blockIdx.x) nrm[c.inst * ldn] = nr;
+    }
     __syncthreads();
-    const int k = s_k;
+    const float inv = s_inv;
+    Sentinel<float>::U* zq = reinterpret_cast<Sentinel<float>::U*>(z);
     for (int64_t i = c.begin + threadIdx.x; i < c.end; i += blockDim.x) {
-        A sv = A(0);
-        for (int q = 0; q < k; ++q) sv = fma(ys[q], (A)V[(int64_t)q * ldv + i], sv);
-        x[i] = (TX)((A)x[i] + sv);
+        out[i] = w[i] * inv;
+        zq[i] = Sentinel<float>::bits;
+    }
+}
+
+// x = sum_{q < kb[b]} y[b][q] V_q, and the sentinel over z for the sweep of x
+__global__ void __launch_bounds__(kBThreads)
+bcombine_kernel(const BChunk* __restrict__ ch, float* __restrict__ x, const float* __restrict__ V, int64_t ldv,
+                const int32_t* __restrict__ kb, const double* __restrict__ y, int ldy, float* __restrict__ z) {
+    const BChunk c = ch[blockIdx.x];
+    const int k = kb[c.inst];
+    if (k == 0) return;
+    Sentinel<float>::U* zq = reinterpret_cast<Sentinel<float>::U*>(z);
+    for (int64_t i = c.begin + threadIdx.x; i < c.end; i += blockDim.x) {
+        float sv = 0.f;
+        for (int q = 0; q < k; ++q) sv = fmaf((float)y[c.inst * ldy + q], V[(int64_t)q * ldv + i], sv);
+        x[i] = sv;
+        zq[i] = Sentinel<float>::bits;
     }
 }
 
@@ -155,77 +308,97 @@ __global__ void bscale_kernel(const BChunk* __restrict__ ch, const TX* __restric
         y[i] = (TY)((s == 0. ? A(0) : sa * (A)x[i]) + (beta == 0. ? A(0) : ba * (A)y[i]));
 }
 
-// Start of a restart cycle, one thread per instance: beta = ||r||, g = (beta, 0...).
-__global__ void bstart_kernel(int nb, int m, const double* __restrict__ nsq, int ldn, double* __restrict__ g,
-                              const double* __restrict__ tol, int32_t* __restrict__ kvalid,
-                              int32_t* __restrict__ done) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const double beta = sqrt(nsq[b * ldn]);
-    for (int q = 0; q <= m; ++q) g[b * (m + 1) + q] = 0.;
-    g[b * (m + 1)] = beta;
-    kvalid[b] = 0;
-    done[b] = (beta <= tol[b]) ? 1 : 0;
+// What one restart cycle knows of its instances, on the device
+struct BState {
+    double *H, *cs, *sn, *g, *est, *y;
+    const double* tol;
+    int32_t *kvalid, *done;
+    int32_t* ndone;                // instances that are done, then 1 once all are (stop): [2]
+    unsigned int* next;            // the sweep's claim counter
+    const int32_t* col_beg;        // first column of instance b (columns of an instance are contiguous)
+    int32_t* skip;                 // columns that products and sweeps leave out
+    int nb, m;
+};
+
+// Columns of instance b skipped or not; the block's threads
+__device__ __forceinline__ void set_skip(const BState& st, int b, int skip) {
+    for (int c = st.col_beg[b] + threadIdx.x; c < st.col_beg[b + 1]; c += blockDim.x) st.skip[c] = skip;
+}
+__device__ __forceinline__ void count_done(const BState& st, int b) {
+    st.done[b] = 1;
+    if (atomicAdd(st.ndone, 1) == st.nb - 1) st.ndone[1] = 1;
 }
 
-// Arnoldi step j of every instance, one thread per instance: store the new
-// Hessenberg column, apply the previous Givens rotations, form the new one,
-// update g and the residual estimate; freeze the instance once converged.
-__global__ void barnoldi_kernel(int nb, int m, int j, const double* __restrict__ ho, int ldh, double* __restrict__ H,
-                                double* __restrict__ cs, double* __restrict__ sn, double* __restrict__ g,
-                                const double* __restrict__ tol, int32_t* __restrict__ kvalid,
-                                int32_t* __restrict__ done, double* __restrict__ est) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb || done[b]) return;
-    double* hc = H + (int64_t)b * (m + 1) * m + (int64_t)j * (m + 1);
-    for (int q = 0; q <= j + 1; ++q) hc[q] = ho[b * ldh + q];
-    double* c = cs + b * m;
-    double* s = sn + b * m;
-    for (int q = 0; q < j; ++q) {
-        const double a0 = hc[q], a1 = hc[q + 1];
-        hc[q] = c[q] * a0 + s[q] * a1;
-        hc[q + 1] = -s[q] * a0 + c[q] * a1;
+// Start of a restart cycle, one block per instance: beta = ||r||, g = (beta, 0...).
+__global__ void bstart_kernel(BState st, const double* __restrict__ nrm) {
+    const int b = blockIdx.x, m = st.m;
+    const double beta = nrm[b];
+    const bool fin = beta <= st.tol[b];
+    for (int q = threadIdx.x; q <= m; q += blockDim.x) st.g[b * (m + 1) + q] = q ? 0. : beta;
+    set_skip(st, b, fin);
+    if (threadIdx.x == 0) {
+        if (b == 0) *st.next = 0u;
+        st.kvalid[b] = 0;
+        st.done[b] = 0;
+        if (fin) count_done(st, b);
     }
-    const double a0 = hc[j], a1 = hc[j + 1];
-    const double rr = hypot(a0, a1);
-    c[j] = rr > 0. ? a0 / rr : 1.;
-    s[j] = rr > 0. ? a1 / rr : 0.;
-    hc[j] = rr;
-    hc[j + 1] = 0.;
-    double* gg = g + b * (m + 1);
-    gg[j + 1] = -s[j] * gg[j];
-    gg[j] = c[j] * gg[j];
-    const double e = fabs(gg[j + 1]);
-    est[b] = e;
-    kvalid[b] = j + 1;
-    if (e <= tol[b] || rr == 0. || !isfinite(e)) done[b] = 1;
 }
 
-// y = H^{-1} g on the kvalid columns of each instance (back substitution)
-__global__ void bsolve_kernel(int nb, int m, const double* __restrict__ H, const double* __restrict__ g,
-                              const int32_t* __restrict__ kvalid, double* __restrict__ y) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const int k = kvalid[b];
-    const double* Hb = H + (int64_t)b * (m + 1) * m;
-    double* yb = y + b * m;
+// Arnoldi step j, one block per instance: store the new Hessenberg column, apply the
+// previous Givens rotations, form the new one, update g and the residual estimate;
+// freeze the instance and skip its columns once converged.
+__global__ void barnoldi_kernel(BState st, int j, const double* __restrict__ ho, int ldh) {
+    const int b = blockIdx.x, m = st.m;
+    if (b == 0 && threadIdx.x == 0) *st.next = 0u;
+    if (st.done[b]) return;
+    __shared__ int s_fin;
+    if (threadIdx.x == 0) {
+        double* hc = st.H + (int64_t)b * (m + 1) * m + (int64_t)j * (m + 1);
+        const double* hb = ho + b * ldh;
+        double* c = st.cs + b * m;
+        double* s = st.sn + b * m;
+        double a0 = hb[0];
+        for (int q = 0; q < j; ++q) {
+            const double a1 = hb[q + 1];
+            hc[q] = c[q] * a0 + s[q] * a1;
+            a0 = -s[q] * a0 + c[q] * a1;
+        }
+        const double a1 = hb[j + 1];
+        const double rr = hypot(a0, a1);
+        c[j] = rr > 0. ? a0 / rr : 1.;
+        s[j] = rr > 0. ? a1 / rr : 0.;
+        hc[j] = rr;
+        hc[j + 1] = 0.;
+        double* gg = st.g + b * (m + 1);
+        const double gj = gg[j];
+        gg[j + 1] = -s[j] * gj;
+        gg[j] = c[j] * gj;
+        const double e = fabs(gg[j + 1]);
+        st.est[b] = e;
+        st.kvalid[b] = j + 1;
+        s_fin = e <= st.tol[b] || rr == 0. || !isfinite(e);
+        if (s_fin) count_done(st, b);
+    }
+    __syncthreads();
+    if (s_fin) set_skip(st, b, 1);
+}
+
+// y = H^{-1} g on the kvalid columns of each instance (back substitution), and
+// the columns of instances without a correction skipped
+__global__ void bsolve_kernel(BState st) {
+    const int b = blockIdx.x, m = st.m;
+    const int k = st.kvalid[b];
+    set_skip(st, b, k == 0);
+    if (threadIdx.x) return;
+    if (b == 0) *st.next = 0u;
+    const double* Hb = st.H + (int64_t)b * (m + 1) * m;
+    double* yb = st.y + b * m;
     for (int q = k - 1; q >= 0; --q) {
-        double acc = g[b * (m + 1) + q];
+        double acc = st.g[b * (m + 1) + q];
         for (int cc = q + 1; cc < k; ++cc) acc -= Hb[(int64_t)cc * (m + 1) + q] * yb[cc];
         const double d = Hb[(int64_t)q * (m + 1) + q];
         yb[q] = d != 0. ? acc / d : 0.;
     }
-    for (int q = k; q < m; ++q) yb[q] = 0.;
-}
-
-// Per-column skip flags from the per-instance state: mode 0 skips finished
-// instances (done), mode 1 skips instances without a correction (kvalid 0).
-__global__ void bskip_kernel(int ncols, const int32_t* __restrict__ col_inst, const int32_t* __restrict__ done,
-                             const int32_t* __restrict__ kvalid, int mode, int32_t* __restrict__ skip) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncols) return;
-    const int b = col_inst[c];
-    skip[c] = mode == 0 ? (done[b] != 0) : (kvalid[b] == 0);
 }
 
 // d += z on the chunks of instances that formed a correction this cycle
@@ -236,24 +409,25 @@ __global__ void badd_kernel(const BChunk* __restrict__ ch, const float* __restri
     for (int64_t i = c.begin + threadIdx.x; i < c.end; i += blockDim.x) d[i] += z[i];
 }
 
-inline int grid1(int n) { return (n + 127) / 128; }
-
 }  // namespace
 
 struct BatchWs {
     int nb = 0, m = 0, nchunks = 0;
     int64_t N = 0;
+    std::vector<int64_t> off;      // instance offsets
     BChunk* d_ch = nullptr;
     int32_t* d_cbeg = nullptr;
     double *b = nullptr, *r = nullptr, *x = nullptr, *t = nullptr, *gb = nullptr;
     float *V32 = nullptr, *w32 = nullptr, *z32 = nullptr, *s32 = nullptr, *d32 = nullptr, *rhs32 = nullptr;
-    double *partial = nullptr, *h1 = nullptr, *h2 = nullptr, *ho = nullptr, *nsq = nullptr;
-    double *H = nullptr, *cs = nullptr, *sn = nullptr, *g = nullptr, *y = nullptr, *est = nullptr;
-    double *tol = nullptr, *tin = nullptr, *scale = nullptr, *vnorm = nullptr;
-    int32_t *kvalid = nullptr, *done = nullptr;
-    int32_t *col_inst = nullptr, *col_skip = nullptr;   // per column: instance, skip flag
-    cudaGraphExec_t cycle = nullptr;
-    long long cycle_kernels = 0;   // kernels one replay of the cycle runs
+    double *partial = nullptr, *partial2 = nullptr, *rsum = nullptr, *h1 = nullptr, *ho = nullptr, *nsq = nullptr;
+    double *tin = nullptr, *scale = nullptr, *vnorm = nullptr;
+    int32_t* d_one = nullptr;      // 0, 1, .., nb: one partial per instance
+    bool own_sums = true;          // blocks add their instance's partials (kOwnSums)
+    BState st{};
+    int32_t* hstop = nullptr;      // per step, pinned: every instance is done
+    cudaEvent_t ev[2] = {};
+    std::vector<cudaGraphExec_t> graphs;   // start, m steps, end
+    std::vector<long long> graph_kernels;  // kernels one replay runs
     std::vector<void*> allocs;
 };
 
@@ -267,9 +441,18 @@ T* balloc(BatchWs* w, size_t n) {
     return (T*)p;
 }
 
+void drop_graphs(BatchWs* w) {
+    for (cudaGraphExec_t g : w->graphs) cudaGraphExecDestroy(g);
+    w->graphs.clear();
+    w->graph_kernels.clear();
+}
+
 void free_bws(BatchWs* w) {
     if (!w) return;
-    if (w->cycle) cudaGraphExecDestroy(w->cycle);
+    drop_graphs(w);
+    for (cudaEvent_t e : w->ev)
+        if (e) cudaEventDestroy(e);
+    if (w->hstop) cudaFreeHost(w->hstop);
     for (void* p : w->allocs) cudaFree(p);
     delete w;
 }
@@ -278,52 +461,103 @@ void free_bws(BatchWs* w) {
 template <typename T>
 void bnorm2(const BatchWs* w, const T* v, double* out, int ldo, cudaStream_t s, const int32_t* done = nullptr) {
     bdot_kernel<T><<<w->nchunks, kBThreads, 0, s>>>(w->d_ch, v, 0, 1, v, w->partial, done), count_launch();
-    breduce_kernel<<<dim3(w->nb, 1), 128, 0, s>>>(w->d_cbeg, w->partial, 1, out, ldo, nullptr, nullptr), count_launch();
+    breduce_kernel<<<dim3(w->nb, 1), 128, 0, s>>>(w->d_cbeg, w->partial, 1, out, ldo), count_launch();
 }
 
-// One restart cycle of batched FP32 GMRES for A d = rhs32, sweep right
-// preconditioned, d updated in place; the kernel sequence is fixed.
-void record_cycle(rtg_handle* h, BatchWs* w, cudaStream_t s) {
+// the sums of the partials p (k per chunk), for blocks that need one instance's
+BSums sums_of(const BatchWs* w, const double* p, int k, cudaStream_t s) {
+    if (w->own_sums) return {p, w->d_cbeg};
+    breduce_kernel<<<dim3(w->nb, k), 128, 0, s>>>(w->d_cbeg, p, k, w->rsum, k), count_launch();
+    return {w->rsum, w->d_one};
+}
+
+// Part of one restart cycle of batched FP32 GMRES for A d = rhs32, sweep right
+// preconditioned, d updated in place: 0 the start, 1 + j Arnoldi step j, m + 1 the
+// end; each a fixed kernel sequence.
+void record_part(rtg_handle* h, BatchWs* w, int part, cudaStream_t s) {
     const int m = w->m, nb = w->nb, nc = w->nchunks;
     const int64_t N = w->N;
     const int ldh = m + 2;
-    const int ncols = h->v32.ncols;
-    OpView<float> v = h->v32;       // the operator with the batch's column skip flags
-    v.skip = w->col_skip;
-    // w = rhs - A d ; V0 = w / ||w|| ; start
-    launch_apply<float>(h, h->v32, RTG_SYSTEM | RTG_MASK_ROWS, w->d32, w->s32, s);
-    bscale_kernel<float, float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->rhs32, w->w32, nullptr, 0, 1., 0.), count_launch();
-    bscale_kernel<float, float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->s32, w->w32, nullptr, 0, -1., 1.), count_launch();
-    bnorm2<float>(w, w->w32, w->nsq, 1, s);
-    bnormalize_kernel<float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, w->w32, w->V32, w->nsq, 1, nullptr, 0, 0,
-                                                      nullptr), count_launch();
-    bstart_kernel<<<grid1(nb), 128, 0, s>>>(nb, m, w->nsq, 1, w->g, w->tin, w->kvalid, w->done), count_launch();
-    for (int j = 0; j < m; ++j) {
+    const int* stop = w->st.ndone + 1;
+    if (part == 0) {
+        // w = rhs - A d ; V0 = w / ||w|| ; start
+        launch_apply<float>(h, h->v32, RTG_SYSTEM | RTG_MASK_ROWS, w->d32, w->s32, s);
+        RTG_CUDA(cudaMemsetAsync(w->st.ndone, 0, 2 * sizeof(int32_t), s));
+        bresid_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->rhs32, w->s32, w->w32, w->partial), count_launch();
+        const BSums sums = sums_of(w, w->partial, 1, s);
+        bnormalize_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, sums, w->w32, w->V32, w->nsq, 1, w->z32,
+                                                   nullptr), count_launch();
+        bstart_kernel<<<nb, 128, 0, s>>>(w->st, w->nsq), count_launch();
+    } else if (part <= m) {
+        const int j = part - 1, k = j + 1;
         float* vj = w->V32 + (int64_t)j * N;
-        float* vn = w->V32 + (int64_t)(j + 1) * N;
-        bskip_kernel<<<grid1(ncols), 128, 0, s>>>(ncols, w->col_inst, w->done, w->kvalid, 0, w->col_skip), count_launch();
-        apply_sweep<float>(h, vj, w->z32, s, nullptr, w->col_skip);
+        OpView<float> v = h->v32;       // the operator with the batch's column skip flags
+        v.skip = w->st.skip;
+        v.stop = stop;
+        apply_sweep<float>(h, vj, w->z32, s, nullptr, w->st.skip, stop, true);
         launch_apply<float>(h, v, RTG_SYSTEM | RTG_MASK_ROWS, w->z32, w->w32, s);
         // CGS2 with per-instance coefficients; ho = h1 + h2
-        bdot_kernel<float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->V32, N, j + 1, w->w32, w->partial, w->done), count_launch();
-        breduce_kernel<<<dim3(nb, j + 1), 128, 0, s>>>(w->d_cbeg, w->partial, j + 1, w->h1, ldh, nullptr, nullptr), count_launch();
-        baxpy_kernel<float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->w32, w->V32, N, j + 1, w->h1, ldh, w->done), count_launch();
-        bdot_kernel<float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->V32, N, j + 1, w->w32, w->partial, w->done), count_launch();
-        breduce_kernel<<<dim3(nb, j + 1), 128, 0, s>>>(w->d_cbeg, w->partial, j + 1, w->h2, ldh, w->h1, w->ho), count_launch();
-        baxpy_kernel<float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->w32, w->V32, N, j + 1, w->h2, ldh, w->done), count_launch();
-        bnorm2<float>(w, w->w32, w->nsq, 1, s, w->done);
-        bnormalize_kernel<float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, w->w32, vn, w->nsq, 1, w->ho, ldh, j + 1,
-                                                          w->done), count_launch();
-        barnoldi_kernel<<<grid1(nb), 128, 0, s>>>(nb, m, j, w->ho, ldh, w->H, w->cs, w->sn, w->g, w->tin, w->kvalid,
-                                                   w->done, w->est), count_launch();
+        bdots_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->V32, N, k, w->w32, w->partial, w->st.done), count_launch();
+        BSums sums = sums_of(w, w->partial, k, s);
+        baxpy_dots_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, sums, w->V32, N, k, w->w32, w->h1, ldh,
+                                                   w->partial2, w->st.done), count_launch();
+        sums = sums_of(w, w->partial2, k, s);
+        baxpy_norm_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, sums, w->V32, N, k, w->w32, w->h1, w->ho, ldh,
+                                                   w->partial, w->st.done), count_launch();
+        sums = sums_of(w, w->partial, 1, s);
+        bnormalize_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, sums, w->w32, vj + N, w->ho + k, ldh, w->z32,
+                                                   w->st.done), count_launch();
+        barnoldi_kernel<<<nb, 128, 0, s>>>(w->st, j, w->ho, ldh), count_launch();
+        RTG_CUDA(cudaMemcpyAsync(w->hstop + j, stop, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    } else {
+        // d += P^{-1} (V y), for the instances that formed a correction
+        bsolve_kernel<<<nb, 128, 0, s>>>(w->st), count_launch();
+        bcombine_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->s32, w->V32, N, w->st.kvalid, w->st.y, m, w->z32), count_launch();
+        apply_sweep<float>(h, w->s32, w->z32, s, nullptr, w->st.skip, nullptr, true);
+        badd_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->z32, w->d32, w->st.kvalid), count_launch();
     }
-    // d += P^{-1} (V y), for the instances that formed a correction
-    bsolve_kernel<<<grid1(nb), 128, 0, s>>>(nb, m, w->H, w->g, w->kvalid, w->y), count_launch();
-    bscale_kernel<float, float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->s32, w->s32, nullptr, 0, 0., 0.), count_launch();
-    bcombine_kernel<float, float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->s32, w->V32, N, w->kvalid, w->y, m), count_launch();
-    bskip_kernel<<<grid1(ncols), 128, 0, s>>>(ncols, w->col_inst, w->done, w->kvalid, 1, w->col_skip), count_launch();
-    apply_sweep<float>(h, w->s32, w->z32, s, nullptr, w->col_skip);
-    badd_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->z32, w->d32, w->kvalid), count_launch();
+}
+
+void capture_parts(rtg_handle* h, BatchWs* w) {
+    cudaStream_t cap;
+    RTG_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+    for (int part = 0; part <= w->m + 1; ++part) {
+        cudaGraph_t graph;
+        const long long n0 = launch_counter().load();
+        RTG_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
+        record_part(h, w, part, cap);
+        RTG_CUDA(cudaStreamEndCapture(cap, &graph));
+        // recorded launches are counted when the graph runs
+        w->graph_kernels.push_back(launch_counter().load() - n0);
+        launch_counter().fetch_sub(w->graph_kernels.back());
+        cudaGraphExec_t exec;
+        RTG_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+        w->graphs.push_back(exec);
+        RTG_CUDA(cudaGraphDestroy(graph));
+    }
+    RTG_CUDA(cudaStreamDestroy(cap));
+}
+
+void replay_part(BatchWs* w, int part, cudaStream_t s) {
+    RTG_CUDA(cudaGraphLaunch(w->graphs[part], s));
+    launch_counter().fetch_add(w->graph_kernels[part]);
+}
+
+// One restart cycle; returns the Arnoldi steps it took.
+int run_cycle(BatchWs* w, cudaStream_t s) {
+    replay_part(w, 0, s);
+    int steps = 0;
+    for (int j = 0; j < w->m; ++j) {
+        replay_part(w, 1 + j, s);
+        RTG_CUDA(cudaEventRecord(w->ev[j & 1], s));
+        if (j > 0) {
+            RTG_CUDA(cudaEventSynchronize(w->ev[(j - 1) & 1]));
+            if (w->hstop[j - 1]) break;
+        }
+        steps = j + 1;
+    }
+    replay_part(w, w->m + 1, s);
+    return steps;
 }
 
 }  // namespace
@@ -346,7 +580,8 @@ int solve_batched(rtg_handle* h, int nb, const int64_t* inst_off, const double* 
     get_sweep(h, s);
     // (re)build the workspace when the instance split or restart changes
     BatchWs* w = h->bws;
-    bool same = w && w->nb == nb && w->m == m && w->N == N;
+    const std::vector<int64_t> off(inst_off, inst_off + nb + 1);
+    const bool same = w && w->off == off && w->m == m && w->N == N;
     std::vector<BChunk> chunks;
     std::vector<int32_t> cbeg(nb + 1, 0);
     for (int b = 0; b < nb; ++b) {
@@ -355,12 +590,17 @@ int solve_batched(rtg_handle* h, int nb, const int64_t* inst_off, const double* 
             chunks.push_back(BChunk{i, std::min(inst_off[b + 1], i + kBChunk), b, 0});
     }
     cbeg[nb] = (int32_t)chunks.size();
-    if (same) {
-        std::vector<int32_t> old(nb + 1);
-        RTG_CUDA(cudaMemcpy(old.data(), w->d_cbeg, sizeof(int32_t) * (nb + 1), cudaMemcpyDeviceToHost));
-        same = old == cbeg;
-    }
     if (!same) {
+        // columns of every instance (contiguous in DOF order)
+        const HostTables& t = h->host;
+        std::vector<int32_t> cb(nb + 1, (int32_t)t.cols.size());
+        cb[0] = 0;
+        int b = 0;
+        for (size_t c = 0; c < t.cols.size(); ++c) {
+            while (b + 1 < nb && t.cols[c].dof_off >= inst_off[b + 1]) cb[++b] = (int32_t)c;
+            if (t.cols[c].dof_off < inst_off[b] || t.cols[c].dof_off + t.cols[c].ndof > inst_off[b + 1])
+                throw RtgError{RTG_ERR_ARG, "an instance boundary splits a column"};
+        }
         free_bws(w);
         w = new BatchWs();
         h->bws = w;
@@ -384,37 +624,42 @@ int solve_batched(rtg_handle* h, int nb, const int64_t* inst_off, const double* 
         w->d32 = balloc<float>(w, N);
         w->rhs32 = balloc<float>(w, N);
         w->partial = balloc<double>(w, (size_t)chunks.size() * (m + 2));
+        w->partial2 = balloc<double>(w, (size_t)chunks.size() * (m + 2));
         const int ldh = m + 2;
+        w->rsum = balloc<double>(w, (size_t)nb * ldh);
         w->h1 = balloc<double>(w, (size_t)nb * ldh);
-        w->h2 = balloc<double>(w, (size_t)nb * ldh);
         w->ho = balloc<double>(w, (size_t)nb * ldh);
         w->nsq = balloc<double>(w, nb);
-        w->H = balloc<double>(w, (size_t)nb * (m + 1) * m);
-        w->cs = balloc<double>(w, (size_t)nb * m);
-        w->sn = balloc<double>(w, (size_t)nb * m);
-        w->g = balloc<double>(w, (size_t)nb * (m + 1));
-        w->y = balloc<double>(w, (size_t)nb * m);
-        w->est = balloc<double>(w, nb);
-        w->tol = balloc<double>(w, nb);
         w->tin = balloc<double>(w, nb);
         w->scale = balloc<double>(w, nb);
         w->vnorm = balloc<double>(w, nb);
-        w->kvalid = balloc<int32_t>(w, nb);
-        w->done = balloc<int32_t>(w, nb);
-        // instance of every column (columns are contiguous in DOF order)
-        const HostTables& t = h->host;
-        std::vector<int32_t> ci(t.cols.size());
-        int b = 0;
-        for (size_t c = 0; c < t.cols.size(); ++c) {
-            while (b + 1 < nb && t.cols[c].dof_off >= inst_off[b + 1]) ++b;
-            if (t.cols[c].dof_off < inst_off[b] || t.cols[c].dof_off + t.cols[c].ndof > inst_off[b + 1])
-                throw RtgError{RTG_ERR_ARG, "an instance boundary splits a column"};
-            ci[c] = b;
-        }
-        w->col_inst = balloc<int32_t>(w, ci.size());
-        w->col_skip = balloc<int32_t>(w, ci.size());
-        RTG_CUDA(cudaMemcpy(w->col_inst, ci.data(), sizeof(int32_t) * ci.size(), cudaMemcpyHostToDevice));
-        RTG_CUDA(cudaMemset(w->col_skip, 0, sizeof(int32_t) * ci.size()));
+        std::vector<int32_t> one(nb + 1);
+        for (int b = 0; b <= nb; ++b) one[b] = b;
+        for (int b = 0; b < nb; ++b) w->own_sums = w->own_sums && cbeg[b + 1] - cbeg[b] <= kOwnSums;
+        w->d_one = balloc<int32_t>(w, nb + 1);
+        RTG_CUDA(cudaMemcpy(w->d_one, one.data(), sizeof(int32_t) * (nb + 1), cudaMemcpyHostToDevice));
+        BState& st = w->st;
+        st.nb = nb;
+        st.m = m;
+        st.H = balloc<double>(w, (size_t)nb * (m + 1) * m);
+        st.cs = balloc<double>(w, (size_t)nb * m);
+        st.sn = balloc<double>(w, (size_t)nb * m);
+        st.g = balloc<double>(w, (size_t)nb * (m + 1));
+        st.y = balloc<double>(w, (size_t)nb * m);
+        st.est = balloc<double>(w, nb);
+        st.tol = w->tin;
+        st.kvalid = balloc<int32_t>(w, nb);
+        st.done = balloc<int32_t>(w, nb);
+        st.ndone = balloc<int32_t>(w, 2);
+        st.next = sweep_counter(h, s);
+        RTG_CUDA(cudaMallocHost(&w->hstop, sizeof(int32_t) * m));
+        for (cudaEvent_t& e : w->ev) RTG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        int32_t* d_cb = balloc<int32_t>(w, nb + 1);
+        st.col_beg = d_cb;
+        st.skip = balloc<int32_t>(w, t.cols.size());
+        RTG_CUDA(cudaMemcpy(d_cb, cb.data(), sizeof(int32_t) * (nb + 1), cudaMemcpyHostToDevice));
+        RTG_CUDA(cudaMemset(st.skip, 0, sizeof(int32_t) * t.cols.size()));
+        w->off = off;   // complete from here on
     }
     const int nc = w->nchunks;
     // b = mask_I (f - A mask_B g); x = 0
@@ -458,32 +703,20 @@ int solve_batched(rtg_handle* h, int nb, const int64_t* inst_off, const double* 
         RTG_CUDA(cudaMemcpyAsync(w->tin, tin.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, s));
         bscale_kernel<double, float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->r, w->rhs32, w->scale, 1, 0., 0.), count_launch();
         bscale_kernel<float, float><<<nc, kBThreads, 0, s>>>(w->d_ch, w->d32, w->d32, nullptr, 0, 0., 0.), count_launch();
-        if (!w->cycle) {
+        if ((int)w->graphs.size() != m + 2) {
             // build the FP32 apply plan and sweep launch shape before capture
             launch_apply<float>(h, h->v32, RTG_SYSTEM | RTG_MASK_ROWS, w->d32, w->s32, s);
             apply_sweep<float>(h, w->s32, w->z32, s);
             RTG_CUDA(cudaStreamSynchronize(s));
-            cudaStream_t cap;
-            RTG_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-            cudaGraph_t graph;
-            const long long n0 = launch_counter().load();
-            RTG_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-            record_cycle(h, w, cap);
-            RTG_CUDA(cudaStreamEndCapture(cap, &graph));
-            // recorded launches are counted when the graph runs
-            w->cycle_kernels = launch_counter().load() - n0;
-            launch_counter().fetch_sub(w->cycle_kernels);
-            RTG_CUDA(cudaGraphInstantiate(&w->cycle, graph, 0));
-            RTG_CUDA(cudaGraphDestroy(graph));
-            RTG_CUDA(cudaStreamDestroy(cap));
+            drop_graphs(w);   // of a capture that failed half-way
+            capture_parts(h, w);
         }
         for (int cyc = 0; cyc < max_cycles; ++cyc) {
-            RTG_CUDA(cudaGraphLaunch(w->cycle, s));
-            launch_counter().fetch_add(w->cycle_kernels);
-            fp32_applies += m + 1;
-            sweeps += m + 1;
-            RTG_CUDA(cudaMemcpyAsync(done.data(), w->done, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, s));
-            RTG_CUDA(cudaMemcpyAsync(kv.data(), w->kvalid, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, s));
+            const int steps = run_cycle(w, s);
+            fp32_applies += steps + 1;
+            sweeps += steps + 1;
+            RTG_CUDA(cudaMemcpyAsync(done.data(), w->st.done, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, s));
+            RTG_CUDA(cudaMemcpyAsync(kv.data(), w->st.kvalid, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, s));
             RTG_CUDA(cudaStreamSynchronize(s));
             bool all = true;
             for (int b = 0; b < nb; ++b) {
