@@ -85,9 +85,7 @@ class ErrorIndicator:
                                                  C.c_void_p(col_lp.data_ptr()), C.c_void_p(cell_lp.data_ptr()),
                                                  None))
             col_keys, elem_keys = self._keys()
-            cl, el = col_lp.cpu().numpy(), cell_lp.cpu().numpy()
-            self._lp = ({ck: float(cl[i]) for i, ck in enumerate(col_keys)},
-                        {ek: float(el[e]) for e, ek in enumerate(elem_keys)})
+            self._lp = (dict(zip(col_keys, col_lp.tolist())), dict(zip(elem_keys, cell_lp.tolist())))
         return self._lp
 
     # ---------------------------------------------------------- hp steering
@@ -110,21 +108,21 @@ class ErrorIndicator:
         ce = torch.empty(lay.nelem, dtype=torch.float64, device=self.ctx.device)
         _lib.check(self.ctx.lib.rtg_error_angular_jump(self.ctx.h, C.c_void_p(self._u_dev().data_ptr()),
                                                        C.c_void_p(ce.data_ptr()), None, None))
-        ce = ce.cpu().numpy()
+        ce = ce.tolist()
+        err = list(map(math.sqrt, ce))
         col_keys, elem_keys = self._keys()
-        cols, col_max, cell_max, mesh_err = {}, -INF, -INF, 0.
-        e = 0
-        for ck in col_keys:
-            cells, s = {}, 0.
-            while e < len(elem_keys) and elem_keys[e][0] == ck:
-                s += ce[e]
-                mesh_err += ce[e]
-                cells[elem_keys[e][1]] = ErrorIndicatorCell(math.sqrt(ce[e]))
-                cell_max = max(cell_max, math.sqrt(ce[e]))
-                e += 1
-            cols[ck] = ErrorIndicatorColumn(math.sqrt(s), cells)
-            col_max = max(col_max, math.sqrt(s))
-        self._finish(cols, col_max, cell_max, mesh_err)
+        start = lay.col_elem_start.tolist()
+        cols, col_err, mesh_err = {}, [], 0.
+        for i, ck in enumerate(col_keys):
+            e0, e1 = start[i], start[i + 1]
+            s = 0.
+            for v in ce[e0:e1]:
+                s += v
+                mesh_err += v
+            col_err.append(math.sqrt(s))
+            cols[ck] = ErrorIndicatorColumn(col_err[i], {elem_keys[e][1]: ErrorIndicatorCell(err[e])
+                                                         for e in range(e0, e1)})
+        self._finish(cols, col_err, err, mesh_err)
 
     def error_spatial_jump(self):
         torch = self.ctx.torch
@@ -132,44 +130,45 @@ class ErrorIndicator:
         cc = torch.empty(lay.ncols, dtype=torch.float64, device=self.ctx.device)
         _lib.check(self.ctx.lib.rtg_error_spatial_jump(self.ctx.h, C.c_void_p(self._u_dev().data_ptr()),
                                                        C.c_void_p(cc.data_ptr()), None))
-        cc = cc.cpu().numpy()
+        cc = cc.tolist()
+        col_err = list(map(math.sqrt, cc))
         col_keys, elem_keys = self._keys()
-        cols, col_max, mesh_err = {}, -INF, 0.
+        start = lay.col_elem_start.tolist()
+        cols, mesh_err = {}, 0.
         for i, ck in enumerate(col_keys):
-            cells = {kk: ErrorIndicatorCell(-INF) for kk in sorted(self.proj.mesh.cols[ck].cells.keys())}
             mesh_err += cc[i]
-            cols[ck] = ErrorIndicatorColumn(math.sqrt(cc[i]), cells)
-            col_max = max(col_max, math.sqrt(cc[i]))
-        self._finish(cols, col_max, -INF, mesh_err)
+            cols[ck] = ErrorIndicatorColumn(col_err[i], {elem_keys[e][1]: ErrorIndicatorCell(-INF)
+                                                         for e in range(start[i], start[i + 1])})
+        self._finish(cols, col_err, [-INF] * lay.nelem, mesh_err)
 
-    def _finish(self, cols, col_max, cell_max, mesh_err):
+    def _finish(self, cols, col_err, cell_err, mesh_err):
         """Maxima, mesh error and the refinement flags in the reference's
-        loop order (error_angular_jump.py:84-137)."""
+        loop order (error_angular_jump.py:84-137).  Columns and cells are new, their
+        do_ref False: only those over a threshold are visited."""
         self.cols = cols
-        self.col_max_error = col_max
-        self.cell_max_error = cell_max
+        self.col_max_error = max([-INF, *col_err])
+        self.cell_max_error = max([-INF, *cell_err])
         self.error = math.sqrt(mesh_err)
         self.error_to_resolve = 0.
         ang_thr = self.ang_ref_tol * self.cell_max_error
         spt_thr = self.spt_ref_tol * self.col_max_error
-        for ck in sorted(cols.keys()):
-            col = cols[ck]
-            if self.ref_kind in ("spt", "all"):
-                if col.error >= spt_thr:
-                    col.do_ref = True
-                    self.error_to_resolve += col.error
-                    col.ref_form = self.col_hp_steer(ck) if self.ref_form == "hp" else self.ref_form
-                else:
-                    col.do_ref = False
-            if self.ref_kind in ("ang", "all"):
-                for kk in sorted(col.cells.keys()):
-                    cell = col.cells[kk]
-                    if cell.error >= ang_thr:
-                        cell.do_ref = True
-                        self.error_to_resolve += cell.error
-                        cell.ref_form = self.cell_hp_steer(ck, kk) if self.ref_form == "hp" else self.ref_form
-                    else:
-                        cell.do_ref = False
+        lay = self.ctx.layout
+        col_keys, elem_keys = self._keys()
+        hits = []      # (column index, -1 or element index): a column, then its cells
+        if self.ref_kind in ("spt", "all"):
+            hits += [(i, -1) for i, v in enumerate(col_err) if v >= spt_thr]
+        if self.ref_kind in ("ang", "all"):
+            hits += [(int(lay.elem_col[e]), e) for e, v in enumerate(cell_err) if v >= ang_thr]
+        for i, e in sorted(hits):
+            ck = col_keys[i]
+            if e < 0:
+                it, steer = cols[ck], lambda: self.col_hp_steer(ck)
+            else:
+                kk = elem_keys[e][1]
+                it, steer = cols[ck].cells[kk], lambda: self.cell_hp_steer(ck, kk)
+            it.do_ref = True
+            self.error_to_resolve += it.error
+            it.ref_form = steer() if self.ref_form == "hp" else self.ref_form
 
     def close(self):
         if self._own and self.ctx is not None:

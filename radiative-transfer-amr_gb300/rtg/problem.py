@@ -404,8 +404,7 @@ class Problem:
                             max_it=int(opts["max_it"]), rtol=float(opts["rtol"]),
                             atol=float(opts["atol"]), x0=x0, inner_rtol=float(opts["inner_rtol"]),
                             precond=precond)
-        uh = Projection(mesh)
-        uh.from_vector(u.cpu().numpy())
+        uh = Projection._of_vector(mesh, u.cpu().numpy())
         hist = info["history"]
         converged_reason = 2 if info["converged"] else -3      # PETSc RTOL / DIVERGED_ITS
         convergence_info = {"converged_reason": converged_reason,

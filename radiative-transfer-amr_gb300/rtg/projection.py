@@ -7,6 +7,7 @@ an [nx, ny, nth] array; ``to_vector``/``from_vector`` use the global DOF order
 vector as raw float64 plus the mesh JSON (dg/projection/to_file.py:10-19)."""
 
 import copy
+import operator
 
 import numpy as np
 
@@ -47,10 +48,7 @@ class ProjectionColumn:
 
 class Projection:
     def __init__(self, mesh, func=None):
-        self.mesh = copy.deepcopy(mesh)
-        self.Ls = self.mesh.Ls
-        self.pbcs = self.mesh.pbcs
-        self.has_th = self.mesh.has_th
+        self._set_mesh(mesh)
         lay = MeshLayout(self.mesh)
         if func is None:
             vec = np.zeros(lay.N)
@@ -62,27 +60,49 @@ class Projection:
                 vec = np.array(_eval(lambda x, y, th: func(x, y), X, Y, T), dtype=np.float64)
         self._build(lay, vec)
 
+    @classmethod
+    def _of_vector(cls, mesh, vec):
+        """Projection(mesh).from_vector(vec), built once"""
+        self = cls.__new__(cls)
+        self._set_mesh(mesh)
+        return self.from_vector(vec)
+
+    def _set_mesh(self, mesh):
+        self.mesh = copy.deepcopy(mesh)
+        self.Ls = self.mesh.Ls
+        self.pbcs = self.mesh.pbcs
+        self.has_th = self.mesh.has_th
+
     def _build(self, lay, vec):
+        """The cells' values are views of one vector in global order."""
+        vec = np.array(vec[:lay.N], order="C")
+        start, off = lay.col_elem_start.tolist(), lay.elem_off.tolist()
         self.cols = {}
+        views = []
         for ci, ck in enumerate(lay.col_keys):
             col = self.mesh.cols[ck]
             nx, ny = col.ndofs[0], col.ndofs[1]
             cells = {}
-            for e in range(int(lay.col_elem_start[ci]), int(lay.col_elem_start[ci + 1])):
+            for e in range(start[ci], start[ci + 1]):
                 kk = lay.elem_keys[e][1]
                 cell = col.cells[kk]
-                o = int(lay.elem_off[e])
-                n = nx * ny * cell.ndofs[0]
-                cells[kk] = ProjectionCell(cell, np.array(vec[o:o + n]).reshape(nx, ny, cell.ndofs[0]))
+                vals = vec[off[e]:off[e + 1]].reshape(nx, ny, cell.ndofs[0])
+                views.append(vals)
+                cells[kk] = ProjectionCell(cell, vals)
             self.cols[ck] = ProjectionColumn(col, cells)
+        self._flat = (vec, views)
 
     def to_vector(self):
         out = []
         for ck in sorted(self.cols.keys()):
-            col = self.cols[ck]
-            for kk in sorted(col.cells.keys()):
-                out.append(col.cells[kk].vals.reshape(-1))
-        return np.concatenate(out)
+            cells = self.cols[ck].cells
+            out += [cells[kk].vals for kk in sorted(cells.keys())]
+        # as built: every cell still holds its own view of the vector (a copied or
+        # unpickled projection's arrays are no views)
+        vec, views = self._flat
+        if len(out) == len(views) and all(map(operator.is_, out, views)) and all(v.base is vec for v in views):
+            return vec.reshape(-1).copy()
+        return np.concatenate([a.reshape(-1) for a in out])
 
     def from_vector(self, vec):
         self._build(MeshLayout(self.mesh), np.asarray(vec, dtype=np.float64))
