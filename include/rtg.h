@@ -192,11 +192,13 @@ int  rtg_get_info(const rtg_handle* h, rtg_info* info);
 int rtg_apply(rtg_handle* h, uint32_t flags, int prec, const void* x, void* y,
               void* stream);
 /* Each precision's apply is autotuned on its first use: every plan shape of
- * the candidate list (16, 32 or 64 angular rows per work item; one CTA per
- * column or per work item; one launch, or one launch per shared-memory class
- * of the CTAs; FP32 also, with one CTA per column and 32 or 64 rows, with the
- * scattering product on the tensor cores, the scattering CTAs of one angular
- * mesh next to each other) is built and the whole apply timed; the fastest
+ * the candidate list (FP32: 16, 32 or 64 angular rows per work item; one CTA per
+ * column or per work item; on small meshes one launch, or one launch per
+ * shared-memory class of the CTAs; and 16 to 128 rows with the scattering
+ * product on the tensor cores, the scattering CTAs of one angular mesh next to
+ * each other.  FP64: one CTA per work item of 4 to 64 rows, and from 4e6
+ * multiply-adds in the product 16 to 64 rows with the product on the tensor
+ * cores, these alone from 1e8) is built and the whole apply timed; the fastest
  * is kept.  This returns the FP32 table (host, cap_rows rows of 9 int32: rows
  * per item, items per CTA (0: the whole column), split launches (0/1),
  * tensor-core scattering (0: none; 1: scattering CTAs heaviest first; 2:

@@ -24,6 +24,7 @@
 #include <map>
 #include <string>
 #include <tuple>
+#include <type_traits>
 
 #include "rtg_apply_common.cuh"
 #include "rtg_internal.h"
@@ -392,10 +393,13 @@ __device__ __forceinline__ void store4(double* p, const double v[4]) {
 // W[R][R], a pad (an odd stride: rows in different banks)
 constexpr int kRowVals = 9;
 
-// threads of a tiled CTA: FP32 items are latency bound (more warps per SM),
-// FP64 ones register bound
-template <typename T>
-__host__ __device__ constexpr int tiled_threads() { return sizeof(T) == 8 ? 256 : 512; }
+// Threads of a tiled CTA.  A CTA walks phases with barriers between them and
+// waits in each for loads; what hides them is other CTAs on the SM, so four (with the
+// product) to six of 256 threads, not two or three of 512: 20 against 24 us at 218,581
+// DOF in FP32, 238 against 266 at 7.95e6 (without the product).
+constexpr int kTiledThreads = 256;
+template <typename T, bool kProduct>
+__host__ __device__ constexpr int tiled_ctas() { return sizeof(T) == 8 ? (kProduct ? 3 : 4) : (kProduct ? 4 : 6); }
 
 // |v| > tol (false for NaN) by the bits: no work for the FP64 pipe
 __device__ __forceinline__ bool above(double v, double tol) {
@@ -414,10 +418,13 @@ __host__ __device__ __forceinline__ int col_int_words(int ncell, int nth_col) {
     return (4 * ncell + 2 + nth_col + 7) & ~7;
 }
 
-// kProduct = false: the tensor-core kernel does the scattering product (FP32),
-// so the CTA neither stages W nor runs the product and fits three per SM
+// kProduct = false: a tensor-core kernel does the scattering product, so the CTA
+// neither stages W nor runs the product, and forms the flux sums T while its rows
+// of x arrive.  FP32, which is not bound by a pipe, walks its outputs node by node
+// (below): at 7.95e6 DOF the whole apply, with scat_tc_kernel beside this one, 298
+// -> 270 us by that, 238 with six CTAs of 256 threads.
 template <typename T, bool kParity, bool kProduct = true>
-__global__ void __launch_bounds__(tiled_threads<T>(), sizeof(T) == 8 ? (kProduct ? 3 : 4) : (kProduct ? 2 : 3))
+__global__ void __launch_bounds__(kTiledThreads, tiled_ctas<T, kProduct>())
 apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* __restrict__ groups,
                    const TileItem* __restrict__ items, const TileCpl* __restrict__ cpl_ent, const T* __restrict__ x,
                    T* __restrict__ y) {
@@ -541,6 +548,38 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
             for (int q = threadIdx.x; q < nent * (int)(sizeof(TileCpl) / 16); q += blockDim.x)
                 cp_async16(dst + 16 * q, src + 16 * q);
         }
+        cp_async_commit();
+        // T[jj][r] = sum_a Et[a][r] x_line[jj][a] of every coupling: one warp
+        // per coupling, its lanes over (jj, r).  Couplings whose Es and Et
+        // are both diagonal (conforming neighbours) have no T: the flux
+        // phase reads their line values directly.  With a diagonal Et the
+        // sum is its one nonzero term (the others add exact zeros).
+        auto form_T = [&]() {
+            const int lane = threadIdx.x & 31, nwarp = (int)blockDim.x >> 5;
+            const int nent = it.cpl_end - it.cpl_begin;
+            for (int c = (int)threadIdx.x >> 5; c < nent; c += nwarp) {
+                const TileCpl& en = sc[c];
+                if ((kParity && en.tested) || en.diag == 3) continue;   // tested: summed term by term below
+                const int nth = en.nth, nt1 = en.nt1, cnt = en.m1 * nth;
+                const bool dt = en.diag & 2;
+                const T* Et = (kParity ? par.mortc : v.mort) + en.et;
+                for (int q = lane; q < cnt; q += 32) {
+                    const int jj = small_div(q, s_rcp[nth]), r = q - jj * nth;
+                    const T* xl = x + en.base + (int64_t)jj * en.stride;
+                    T acc = T(0);
+                    if (dt) {
+                        acc = Et[r * nth + r] * xl[r];
+                    } else {
+                        // the loads of up to 8 line values issued before their sum
+#pragma unroll
+                        for (int a = 0; a < 8; ++a)
+                            if (a < nt1) acc = fma(Et[a * nth + r], xl[a], acc);
+                        for (int a = 8; a < nt1; ++a) acc = fma(Et[a * nth + r], xl[a], acc);
+                    }
+                    Tb[en.toff + q] = acc;
+                }
+            }
+        };
         if (scat) {
             // W^T staged by rows of W^T, so consecutive threads read consecutive values
             const T* WTg = v.WT + v.W_off[C.sig];
@@ -567,6 +606,14 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
                 const int l = d - nij * crow[k];
                 const int ij = small_div(l, s_rcp[nth]);
                 cp_async_small<sizeof(T)>(Xs + (crow[k] - it.row0 + l - ij * nth) * nijp + ij, xc + d);
+            }
+            // the flux sums T while the rows arrive (there is no W in their place)
+            if (fl.bc) {
+                cp_async_commit();
+                cp_async_wait_prior();
+                __syncthreads();
+                for (int t = threadIdx.x; t < Mp * nijp; t += blockDim.x) Fy[t] = T(0);
+                form_T();
             }
         }
         cp_async_wait_all();
@@ -688,39 +735,10 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
         __syncthreads();
         // inflow face fluxes of the item's elements into Fy (the W region is free)
         if (fl.bc) {
-            for (int t = threadIdx.x; t < Mp * nijp; t += blockDim.x) Fy[t] = T(0);
-            // T[jj][r] = sum_a Et[a][r] x_line[jj][a] of every coupling: one warp
-            // per coupling, its lanes over (jj, r).  Couplings whose Es and Et
-            // are both diagonal (conforming neighbours) have no T: the flux
-            // phase reads their line values directly.  With a diagonal Et the
-            // sum is its one nonzero term (the others add exact zeros).
-            {
-                const int lane = threadIdx.x & 31, nwarp = (int)blockDim.x >> 5;
-                const int nent = it.cpl_end - it.cpl_begin;
-                for (int c = (int)threadIdx.x >> 5; c < nent; c += nwarp) {
-                    const TileCpl& en = sc[c];
-                    if ((kParity && en.tested) || en.diag == 3) continue;   // tested: summed term by term below
-                    const int nth = en.nth, nt1 = en.nt1, cnt = en.m1 * nth;
-                    const bool dt = en.diag & 2;
-                    const T* Et = (kParity ? par.mortc : v.mort) + en.et;
-                    for (int q = lane; q < cnt; q += 32) {
-                        const int jj = small_div(q, s_rcp[nth]), r = q - jj * nth;
-                        const T* xl = x + en.base + (int64_t)jj * en.stride;
-                        T acc = T(0);
-                        if (dt) {
-                            acc = Et[r * nth + r] * xl[r];
-                        } else {
-                            // the loads of up to 8 line values issued before their sum
-#pragma unroll
-                            for (int a = 0; a < 8; ++a)
-                                if (a < nt1) acc = fma(Et[a * nth + r], xl[a], acc);
-                            for (int a = 8; a < nt1; ++a) acc = fma(Et[a * nth + r], xl[a], acc);
-                        }
-                        Tb[en.toff + q] = acc;
-                    }
-                }
-            }
-            __syncthreads();
+            if constexpr (kProduct)
+                for (int t = threadIdx.x; t < Mp * nijp; t += blockDim.x) Fy[t] = T(0);
+            if constexpr (kProduct) form_T();
+            if constexpr (kProduct) __syncthreads();
             // one thread per (boundary node, row): the element's couplings on the
             // node's faces in a fixed order, so the sum is deterministic
             {
@@ -778,27 +796,114 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
             }
             __syncthreads();
         }
-        const int d0 = nij * it.row0, d1 = nij * (it.row0 + M);
-        int k = it.cell_begin;
-        for (int d = d0 + threadIdx.x; d < d1; d += blockDim.x) {
-            while (d >= nij * crow[k + 1]) ++k;
-            const int nth = crow[k + 1] - crow[k];
-            const int l = d - nij * crow[k];
-            const int ij = small_div(l, s_rcp[nth]), r = l - ij * nth;
-            const int i = small_div(ij, rny), j = ij - i * C.ny;
-            const int flg = cflg[k];
-            if (fl.mask_rows && bdry_node(flg >> 4, i, j, C.nx, C.ny)) {
-                if constexpr (kStore) yc[d] = T(0);   // FP32 tensor-core path: y was zeroed
-                continue;
+        if constexpr (!kParity) {
+            // FP32: one thread per (cell, node) walks the cell's angular rows with the
+            // node's derivative rows in registers, unrolled for equal degrees, and the
+            // finished values replace the flux values Fy, from which they go out in
+            // global order
+            const int ntask = (it.cell_end - it.cell_begin) * nij;
+            const float rnij = __frcp_rn((float)nij);
+            auto outputs = [&](auto deg) {
+                constexpr int N = decltype(deg)::value;   // nodes per direction, 0: any
+                const int ny = N ? N : C.ny, nx = N ? N : C.nx;
+                for (int t = threadIdx.x; t < ntask; t += blockDim.x) {
+                    const int kk = small_div(t, rnij), ij = t - kk * nij, k = it.cell_begin + kk;
+                    const int i = small_div(ij, rny), j = ij - i * ny;
+                    const int nth = crow[k + 1] - crow[k], m0 = crow[k] - it.row0, flg = cflg[k];
+                    T* out = Fy + m0 * nijp + ij;
+                    if (fl.mask_rows && bdry_node(flg >> 4, i, j, nx, ny)) {
+                        for (int r = 0; r < nth; ++r) out[r * nijp] = T(0);
+                        continue;
+                    }
+                    const bool edge = fl.bc && (i == 0 || j == 0 || i == nx - 1 || j == ny - 1);
+                    // outflow faces of the node
+                    const int of = edge ? flg & ((i == nx - 1 ? 1 : 0) | (j == ny - 1 ? 2 : 0) | (i == 0 ? 4 : 0) |
+                                                 (j == 0 ? 8 : 0))
+                                        : 0;
+                    const T kw = kwn[ij], cw = cwn[ij], wx = wxs[i], wy = wys[j];
+                    T gx[N ? N : 1], gy[N ? N : 1];
+                    if constexpr (N > 0) {
+#pragma unroll
+                        for (int q = 0; q < N; ++q) gx[q] = Gxs[i * N + q], gy[q] = Gys[j * N + q];
+                    }
+                    const T* rw = rowt + (kProduct ? crow[k] : m0) * kRowVals;
+                    const T* xr = Xs + (kProduct ? crow[k] : m0) * nijp;
+                    const T* ys = Ys + m0 * nijp + ij;
+                    for (int r = 0; r < nth; ++r, rw += kRowVals, xr += nijp) {
+                        const T xself = xr[ij], mterm = rw[0] * kw;
+                        T acc = T(0);
+                        if (scat) acc = -cw * ys[r * nijp];
+                        if (fl.mass) acc = fma(mterm, xself, acc);
+                        if (fl.ic) {
+                            T t1 = T(0), t2 = T(0);
+                            const T *xi = xr + i * ny, *xj = xr + j;
+                            if constexpr (N > 0) {
+#pragma unroll
+                                for (int q = 0; q < N; ++q) t1 = fma(gy[q], xi[q], t1), t2 = fma(gx[q], xj[q * N], t2);
+                            } else {
+                                for (int q = 0; q < ny; ++q) t1 = fma(Gys[j * ny + q], xi[q], t1);
+                                for (int q = 0; q < nx; ++q) t2 = fma(Gxs[i * nx + q], xj[q * ny], t2);
+                            }
+                            acc = fma(rw[1], wx * t1, acc);
+                            acc = fma(rw[2], wy * t2, acc);
+                        }
+                        if (edge) {
+                            acc += out[r * nijp];
+                            // the diagonal terms (rt/boundary_convection_matrix.py:276-346)
+                            if (of & 1) acc = fma(rw[3] * wy, xself, acc);
+                            if (of & 2) acc = fma(rw[4] * wx, xself, acc);
+                            if (of & 4) acc = fma(rw[5] * wy, xself, acc);
+                            if (of & 8) acc = fma(rw[6] * wx, xself, acc);
+                        }
+                        out[r * nijp] = acc;
+                    }
+                }
+            };
+            switch (C.nx == C.ny ? C.nx : 0) {
+                case 3: outputs(std::integral_constant<int, 3>{}); break;
+                case 4: outputs(std::integral_constant<int, 4>{}); break;
+                case 5: outputs(std::integral_constant<int, 5>{}); break;
+                case 6: outputs(std::integral_constant<int, 6>{}); break;
+                case 7: outputs(std::integral_constant<int, 7>{}); break;
+                case 8: outputs(std::integral_constant<int, 8>{}); break;
+                default: outputs(std::integral_constant<int, 0>{});
             }
-            const int R = crow[k] + r;
-            const int m = R - it.row0;   // row within the item
-            const int xr0 = kProduct ? R : m;   // row of Xs
-            const T* rw = rowt + xr0 * kRowVals;
-            const T xself = Xs[xr0 * nijp + ij];
-            const T mterm = rw[0] * kwn[ij];
-            T acc = T(0);
-            if constexpr (kParity) {
+            __syncthreads();
+            int k = it.cell_begin;
+            for (int d = nij * it.row0 + threadIdx.x; d < nij * (it.row0 + M); d += blockDim.x) {
+                while (d >= nij * crow[k + 1]) ++k;
+                const int nth = crow[k + 1] - crow[k], l = d - nij * crow[k];
+                const int ij = small_div(l, s_rcp[nth]);
+                const T val = Fy[(crow[k] - it.row0 + l - ij * nth) * nijp + ij];
+                // tensor-core path: the scattering kernel adds its part to the
+                // same zeroed y concurrently; two terms on zero sum the same in
+                // either order
+                if constexpr (kStore)
+                    yc[d] = val;
+                else if (val != T(0))
+                    atomicAdd(yc + d, val);
+            }
+        } else {
+            const int d0 = nij * it.row0, d1 = nij * (it.row0 + M);
+            int k = it.cell_begin;
+            for (int d = d0 + threadIdx.x; d < d1; d += blockDim.x) {
+                while (d >= nij * crow[k + 1]) ++k;
+                const int nth = crow[k + 1] - crow[k];
+                const int l = d - nij * crow[k];
+                const int ij = small_div(l, s_rcp[nth]), r = l - ij * nth;
+                const int i = small_div(ij, rny), j = ij - i * C.ny;
+                const int flg = cflg[k];
+                if (fl.mask_rows && bdry_node(flg >> 4, i, j, C.nx, C.ny)) {
+                    yc[d] = T(0);
+                    continue;
+                }
+                const int R = crow[k] + r;
+                const int m = R - it.row0;   // row within the item
+                const int xr0 = kProduct ? R : m;   // row of Xs
+                const T* rw = rowt + xr0 * kRowVals;
+                const T xself = Xs[xr0 * nijp + ij];
+                const T mterm = rw[0] * kwn[ij];
+                T acc = T(0);
                 if (fl.scat) {
                     const T cw = cwn[ij];
                     const T vd = fma(-cw, rw[7], fl.merged ? mterm : T(0));
@@ -823,31 +928,26 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
                     }
                 }
                 if (fl.mass && !fl.merged) acc = fma(mterm, xself, acc);
-            } else {
-                if (scat) acc = -cwn[ij] * Ys[m * nijp + ij];
-                if (fl.mass) acc = fma(mterm, xself, acc);
-            }
-            if (fl.ic) {
-                const T* xr = Xs + xr0 * nijp;
-                T t1 = T(0), t2 = T(0);
-                const T* gy = Gys + j * C.ny;
-                for (int jj = 0; jj < C.ny; ++jj) t1 = fma(gy[jj], xr[i * C.ny + jj], t1);
-                const T* gx = Gxs + i * C.nx;
-                for (int ii = 0; ii < C.nx; ++ii) t2 = fma(gx[ii], xr[ii * C.ny + j], t2);
-                acc = fma(rw[1], wxs[i] * t1, acc);
-                acc = fma(rw[2], wys[j] * t2, acc);
-            }
-            if (fl.bc && (i == 0 || j == 0 || i == C.nx - 1 || j == C.ny - 1)) {
-                acc += Fy[m * nijp + ij];
-                // outflow faces: the diagonal term (rt/boundary_convection_matrix.py:276-346)
-                for (int F = 0; F < 4; ++F) {
-                    if (!(flg & (1 << F))) continue;
-                    const bool on = (F == 0 && i == C.nx - 1) || (F == 1 && j == C.ny - 1) || (F == 2 && i == 0) ||
-                                    (F == 3 && j == 0);
-                    if (!on) continue;
-                    const T w = (F % 2 == 0) ? wys[j] : wxs[i];
-                    T val = rw[3 + F] * w;
-                    if constexpr (kParity) {
+                if (fl.ic) {
+                    const T* xr = Xs + xr0 * nijp;
+                    T t1 = T(0), t2 = T(0);
+                    const T* gy = Gys + j * C.ny;
+                    for (int jj = 0; jj < C.ny; ++jj) t1 = fma(gy[jj], xr[i * C.ny + jj], t1);
+                    const T* gx = Gxs + i * C.nx;
+                    for (int ii = 0; ii < C.nx; ++ii) t2 = fma(gx[ii], xr[ii * C.ny + j], t2);
+                    acc = fma(rw[1], wxs[i] * t1, acc);
+                    acc = fma(rw[2], wys[j] * t2, acc);
+                }
+                if (fl.bc && (i == 0 || j == 0 || i == C.nx - 1 || j == C.ny - 1)) {
+                    acc += Fy[m * nijp + ij];
+                    // outflow faces: the diagonal term (rt/boundary_convection_matrix.py:276-346)
+                    for (int F = 0; F < 4; ++F) {
+                        if (!(flg & (1 << F))) continue;
+                        const bool on = (F == 0 && i == C.nx - 1) || (F == 1 && j == C.ny - 1) || (F == 2 && i == 0) ||
+                                        (F == 3 && j == 0);
+                        if (!on) continue;
+                        const T w = (F % 2 == 0) ? wys[j] : wxs[i];
+                        T val = rw[3 + F] * w;
                         // |value| > 1e-15, near it in the reference's order of the product
                         if (!above(val, 2. * kBcTol)) {
                             const int e = C.elem_begin + k;
@@ -856,17 +956,11 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
                                   A[(3 + F) * nth + r];
                             if (!(tabs(val) > T(kBcTol))) continue;
                         }
+                        acc = fma(val, xself, acc);
                     }
-                    acc = fma(val, xself, acc);
                 }
-            }
-            // tensor-core path: the scattering kernel adds its part to the
-            // same zeroed y concurrently; two terms on zero sum the same in
-            // either order
-            if constexpr (kStore)
                 yc[d] = acc;
-            else
-                atomicAdd(yc + d, acc);
+            }
         }
         // the next item overwrites the couplings and the item region
         __syncthreads();
@@ -1556,7 +1650,7 @@ static void smem_class_limits(size_t lim[kSmemClasses]) {
     // CTAs per SM that registers and threads allow
     int maxb = 0;
     RTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, apply_tiled_kernel<T, sizeof(T) == 8, kProduct>,
-                                                           tiled_threads<T>(), 0));
+                                                           kTiledThreads, 0));
     for (int q = 0; q < kSmemClasses; ++q) {
         const int per = kSmemClasses - q;
         const long long l = (long long)per_sm / per - resv - (long long)fa.sharedSizeBytes;
@@ -1901,10 +1995,10 @@ static void run_plan(const ApplyPlan* plan, const OpView<T>& v, const OpView<flo
             if (!n) continue;
             const int4* grp = plan->d_tgroups + plan->tg_begin[q];
             if (plan->tc)
-                apply_tiled_kernel<T, f64, false><<<n, tiled_threads<T>(), plan->tg_smem[q], s>>>(
+                apply_tiled_kernel<T, f64, false><<<n, kTiledThreads, plan->tg_smem[q], s>>>(
                     v, tp, flags, grp, plan->d_tiles, plan->d_tile_cpl, x, y), count_launch();
             else
-                apply_tiled_kernel<T, f64><<<n, tiled_threads<T>(), plan->tg_smem[q], s>>>(
+                apply_tiled_kernel<T, f64><<<n, kTiledThreads, plan->tg_smem[q], s>>>(
                     v, tp, flags, grp, plan->d_tiles, plan->d_tile_cpl, x, y), count_launch();
             const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) {
@@ -1943,13 +2037,13 @@ static int plan_launches(const ApplyPlan* p) {
     return n;
 }
 
-// FP64 multiply-adds of the scattering product from which plans with the
-// tensor cores (rtg_scat64.cu) are timed beside those of the FP64 pipe, and from
+// Multiply-adds of the scattering product from which FP64 plans with the
+// tensor cores (rtg_scat64.cu; FP32 plans: more shapes, tune_plan) are timed beside those of the FP64 pipe, and from
 // which they alone are.  Whole applies, FP64 pipe against tensor cores, in us: 19.8
 // and 27.9 at 1.2e6 (33,056 DOF adaptive: an extra launch), 51.6 and 49.9 at 8.6e6
 // (218,581 DOF adaptive), 73 and 38 at 2.1e7, 459 and 103 at 1.6e8, 4067 and 870 at
 // 1.5e9 (7.95e6 DOF, two scatterers).
-constexpr int64_t kTc64Offer = 4'000'000, kTc64Alone = 100'000'000;
+constexpr int64_t kTcOffer = 4'000'000, kTc64Alone = 100'000'000;
 
 // where the tensor-core kernel of a plan reports a wait that gave up
 static int* plan_status(const ApplyPlan* p) { return p->par ? scat64_status(p->par->s64) : p->d_status; }
@@ -2035,7 +2129,7 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
             prod += (int64_t)C.nx * C.ny * C.nth_col * C.nth_col;
             all_fit &= scat64_fits(C);
         }
-        if (f64 && all_fit && prod >= kTc64Offer) {
+        if (f64 && all_fit && prod >= kTcOffer) {
             std::vector<int> cap(h->host.cols.size(), kTileRows);
             ApplyPlan* probe = make_plan<T>(h, &cap, nullptr, kChunk64, par, 0, 0, 1);
             try {
@@ -2054,17 +2148,28 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
             // of a small mesh's other SMs idle (84.6 against 51.6 us at 218,581 DOF)
             for (int rows : {4, 8, 16, 32, 64}) shapes.push_back(PlanShape{rows, 1, 0, 0});
         } else if (!tc64) {
+            // launches split by shared-memory class only matter where a launch does
+            // (none differed by 2 % at 218,581 DOF and above)
             for (int rows : {16, 32, 64})
                 for (int gcap : {0, 1})
-                    for (int split : {0, 1}) shapes.push_back(PlanShape{rows, gcap, split, 0});
+                    for (int split : {0, 1})
+                        if (!split || f64 || prod < kTcOffer) shapes.push_back(PlanShape{rows, gcap, split, 0});
         }
-        // tensor-core scattering, FP32: one CTA per column, items of 32 or 64
-        // rows, the scattering CTAs of one angular mesh next to each other
-        // (one CTA per item ties with these on the two-scatterer problem, and
-        // the heaviest-first order of the scattering CTAs is 1.7 % slower there;
-        // both are left out of the list, rtg_apply_shape can still pin them)
-        if (!f64)
-            for (int rows : {32, 64}) shapes.push_back(PlanShape{rows, 0, 0, 2});
+        // tensor-core scattering, FP32, the scattering CTAs of one angular mesh next
+        // to each other (their heaviest-first order is 1.7 % slower on the
+        // two-scatterer problem).  Below kTcOffer multiply-adds a launch decides (10 us
+        // without, 14 to 16 with, at 4,096 DOF).  Above, one CTA per item is the best at
+        // 1.95e6 DOF (two scatterers, 128 rows: 75 against 98 us for a column per CTA
+        // of 64) and on uniform 8-node meshes (16 rows: 25 against 42 to 53),
+        // one per column, of 128 rows, at 7.95e6 (250 against 252 to 307).
+        if (!f64) {
+            if (prod < kTcOffer) {
+                for (int rows : {32, 64}) shapes.push_back(PlanShape{rows, 0, 0, 2});
+            } else {
+                for (int rows : {16, 32, 128}) shapes.push_back(PlanShape{rows, 1, 0, 2});
+                for (int rows : {64, 128}) shapes.push_back(PlanShape{rows, 0, 0, 2});
+            }
+        }
         // FP64: one CTA per item (one per column leaves SMs idle at its end)
         if (tc64)
             for (int rows : {16, 32, 64}) shapes.push_back(PlanShape{rows, 1, 0, 1});

@@ -155,6 +155,10 @@ __device__ __forceinline__ void cp_async_small(void* dst, const void* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(kBytes) : "memory");
 }
+// closes the group of the copies issued so far; cp_async_wait_prior() waits for
+// every group but the last
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_prior() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // a / b for 0 <= a < 2^22, given rb = 1/b rounded to nearest float: (a + 1/2)/b
