@@ -377,14 +377,6 @@ __device__ __forceinline__ void load4(const double* p, double o[4]) {
     o[2] = b.x;
     o[3] = b.y;
 }
-__device__ __forceinline__ void store4(float* p, const float v[4]) {
-    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-__device__ __forceinline__ void store4(double* p, const double v[4]) {
-    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
-    *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
-}
-
 // values of the per-row table, every product of row constants made once per
 // row (an output then takes nx + ny + 7 FP64 operations and two per outflow
 // face; the FP64 kernel without the product is bound by them): dxdydth/8 wth_r,
@@ -433,10 +425,9 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
     __shared__ float s_rcp[kMaxNodes + 1];    // 1/n rounded to float
     __shared__ uint8_t s_cls[kParity ? kMaxNodes * kMaxNodes : 1];   // scattering class per node
     T* smt = reinterpret_cast<T*>(smt4);
-    if (v.stop && *v.stop) return;
+    after_trigger();
     const int4 grp = groups[blockIdx.x];      // column, first item, end item
     const int ci = grp.x;
-    if (v.skip && v.skip[ci]) return;
     const ColDev C = v.cols[ci];
     const ApplyFlags fl = decode(flags);
     const bool scat = kProduct && fl.scat;
@@ -492,6 +483,12 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
                                     : Gy + (q - o5);
             cp_async_small<sizeof(T)>(colt + q, src);
         }
+    }
+    // the tables above are constant; x, the flags and y are not
+    after_wait();
+    if ((v.stop && *v.stop) || (v.skip && v.skip[ci])) {
+        cp_async_wait_all();
+        return;
     }
     __syncthreads();
     const T* xc = x + C.dof_off;
@@ -1999,12 +1996,17 @@ static void run_plan(const ApplyPlan* plan, const OpView<T>& v, const OpView<flo
             const int n = plan->tg_begin[q + 1] - plan->tg_begin[q];
             if (!n) continue;
             const int4* grp = plan->d_tgroups + plan->tg_begin[q];
-            if (plan->tc)
-                apply_tiled_kernel<T, f64, false><<<n, kTiledThreads, plan->tg_smem[q], s>>>(
-                    v, tp, flags, grp, plan->d_tiles, plan->d_tile_cpl, x, y), count_launch();
-            else
-                apply_tiled_kernel<T, f64><<<n, kTiledThreads, plan->tg_smem[q], s>>>(
-                    v, tp, flags, grp, plan->d_tiles, plan->d_tile_cpl, x, y), count_launch();
+            if (plan->tc) {
+                if (tc_run)   // beside the side stream's kernel, after a fill
+                    apply_tiled_kernel<T, f64, false><<<n, kTiledThreads, plan->tg_smem[q], s>>>(
+                        v, tp, flags, grp, plan->d_tiles, plan->d_tile_cpl, x, y), count_launch();
+                else
+                    launch_after(apply_tiled_kernel<T, f64, false>, n, kTiledThreads, plan->tg_smem[q], s, v, tp, flags,
+                                 grp, plan->d_tiles, plan->d_tile_cpl, x, y);
+            } else {
+                launch_after(apply_tiled_kernel<T, f64>, n, kTiledThreads, plan->tg_smem[q], s, v, tp, flags, grp,
+                             plan->d_tiles, plan->d_tile_cpl, x, y);
+            }
             const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) {
                 cudaFuncAttributes fa{};
@@ -2261,6 +2263,11 @@ static void force_shape(rtg_handle* h, const PlanShape& sh) {
     ApplyPlan*& slot = f64 ? h->plan64 : h->plan32;
     free_plan(slot);
     slot = p;
+}
+
+bool apply_chains(const rtg_handle* h, int prec) {
+    const ApplyPlan* p = prec == RTG_FP64 ? h->plan64 : h->plan32;
+    return p && !p->ntc;
 }
 
 int apply_shape(rtg_handle* h, int prec, const int32_t* shape) {

@@ -57,6 +57,31 @@ struct RtgError {
                                                     cudaGetErrorString(e_)};                 \
     } while (0)
 
+// Programmatic dependent launch: a kernel launched with launch_after() may have its
+// blocks resident before the kernel ahead of it in the stream has ended, from when every
+// block of that one has passed after_trigger(); after_wait() returns once it has ended and
+// its writes are there.  Every kernel so launched waits before it reads or writes
+// anything another kernel writes or reads (stop flags included), so the order of a stream's
+// kernels stays that of plain launches.  It hides the launch and, where a kernel reads
+// constant tables first, those.
+__device__ __forceinline__ void after_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    RTG_CUDA(cudaLaunchKernelEx(&c, kernel, P(args)...));
+    count_launch();
+}
+
 // Per column.
 struct ColDev {
     double dx, dy;
@@ -251,6 +276,9 @@ int apply_status(rtg_handle* h, cudaStream_t s);
 // FP32 apply autotuning table (tunes on first use): rows of [nx, ny, nth_b,
 // cap, ns per candidate cap]; returns the number of degree classes
 int apply_tuning(rtg_handle* h, int32_t* out, int cap_rows, cudaStream_t s);
+// true when an apply in this precision ends with kernels on its own stream only
+// (no side stream joined): the kernel after it may be launched with launch_after()
+bool apply_chains(const rtg_handle* h, int prec);
 int apply_shape(rtg_handle* h, int prec, const int32_t* shape);
 
 // Sweep preconditioner (rtg_sweep.cu): z = P^{-1} r

@@ -538,6 +538,8 @@ sweep_persistent_kernel(OpView<T> v, const int32_t* __restrict__ rec, int rstrid
     __shared__ int s_abort;
     __shared__ int s_rec[kRecMax];
     __shared__ T s_dc[kMaxCplStaged];
+    after_trigger();
+    after_wait();
     if (v.stop && *v.stop) return;
     int ahead = -1;   // thread 0: the next element, claimed once this one's inputs are there
     for (;;) {
@@ -1607,9 +1609,9 @@ void apply_sweep(rtg_handle* h, const T* r, T* z, cudaStream_t st, unsigned long
         const bool split = sh.split && !trace;   // a trace has one record per element
         um.reg_cap = sh.reg_cap;
         um.stage_cap = (int)(sh.smem / sizeof(T)) - 2 * rhs_cap;
-        sweep_persistent_kernel<T><<<sh.grid, sh.threads, sh.smem, st>>>(
-            v, split ? s->d_rec_split : s->d_rec, s->rec_stride, split ? s->nsplit : ne, s->d_active, inv, r, z, s->d_next, s->d_status,
-            um, rhs_cap, sh.bcap, trace), count_launch();
+        launch_after(sweep_persistent_kernel<T>, sh.grid, sh.threads, sh.smem, st, v, split ? s->d_rec_split : s->d_rec,
+                     s->rec_stride, split ? s->nsplit : ne, s->d_active, inv, r, z, s->d_next, s->d_status, um, rhs_cap,
+                     sh.bcap, trace);
     };
     if (s->pick[pi] < 0) {
         // the launch shapes: larger per-CTA shared memory (more one-phase
