@@ -2155,12 +2155,14 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
             // of a small mesh's other SMs idle (84.6 against 51.6 us at 218,581 DOF)
             for (int rows : {4, 8, 16, 32, 64}) shapes.push_back(PlanShape{rows, 1, 0, 0});
         } else if (!tc64) {
-            // launches split by shared-memory class only matter where a launch does
-            // (none differed by 2 % at 218,581 DOF and above)
+            // on larger meshes launches split by shared-memory class (none differed by 2 %
+            // at 218,581 DOF and above) and a column of 16 or 32 rows per CTA (never the
+            // best there) are left out
             for (int rows : {16, 32, 64})
                 for (int gcap : {0, 1})
                     for (int split : {0, 1})
-                        if (!split || f64 || prod < kTcOffer) shapes.push_back(PlanShape{rows, gcap, split, 0});
+                        if (f64 || prod < kTcOffer || (!split && (gcap || rows == 64)))
+                            shapes.push_back(PlanShape{rows, gcap, split, 0});
         }
         // tensor-core scattering, FP32, the scattering CTAs of one angular mesh next
         // to each other (their heaviest-first order is 1.7 % slower on the
@@ -2173,8 +2175,8 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
             if (prod < kTcOffer) {
                 for (int rows : {32, 64}) shapes.push_back(PlanShape{rows, 0, 0, 2});
             } else {
-                for (int rows : {16, 32, 128}) shapes.push_back(PlanShape{rows, 1, 0, 2});
-                for (int rows : {64, 128}) shapes.push_back(PlanShape{rows, 0, 0, 2});
+                for (int rows : {16, 128}) shapes.push_back(PlanShape{rows, 1, 0, 2});
+                shapes.push_back(PlanShape{128, 0, 0, 2});
             }
         }
         // FP64: one CTA per item (one per column leaves SMs idle at its end)

@@ -1640,13 +1640,16 @@ void apply_sweep(rtg_handle* h, const T* r, T* z, cudaStream_t st, unsigned long
         }
         // time each: rounds over all shapes (so that a drift of the clocks
         // meets every shape alike), the first round a warm-up, best of the
-        // other five; a smaller budget must win by 3 %
+        // other five, of which a shape 1.25 times slower than the best so far takes
+        // one; a smaller budget must win by 3 %
         cudaEvent_t e0, e1;
         RTG_CUDA(cudaEventCreate(&e0));
         RTG_CUDA(cudaEventCreate(&e1));
         for (int q = 0; q < kSweepShapes; ++q) s->shape_ms[pi][q] = 1e30f;
         for (int rep = 0; rep < 6; ++rep)
             for (int q = 0; q < nshapes; ++q) {
+                if (rep > 1 && s->shape_ms[pi][q] > 1.25f * *std::min_element(s->shape_ms[pi], s->shape_ms[pi] + nshapes))
+                    continue;
                 sweep_fill_kernel<T><<<std::max(1, std::min((int)h->host.elems.size(), 152 * 8)), 256, 0, st>>>(
                     v, (int)h->host.elems.size(), z, s->d_next), count_launch();
                 RTG_CUDA(cudaEventRecord(e0, st));
