@@ -42,38 +42,22 @@ struct BChunk {
     int32_t inst, pad;
 };
 
-template <typename T>
-__global__ void bdot_kernel(const BChunk* __restrict__ ch, const T* __restrict__ V, int64_t ldv, int k,
-                            const T* __restrict__ w, double* __restrict__ partial, const int32_t* __restrict__ done) {
-    __shared__ double red[kBGroup][kBThreads / 32];
+// partials of <v, v> per chunk (FP64), bound by reading v; the general kernel's
+// reductions for eight products took 103 us at 4.65e6 values
+__global__ void __launch_bounds__(kBThreads)
+bnorm_kernel(const BChunk* __restrict__ ch, const double* __restrict__ v, double* __restrict__ partial) {
+    __shared__ double red[kBThreads / 32];
     const BChunk c = ch[blockIdx.x];
-    if (done && done[c.inst]) return;
-    for (int g0 = 0; g0 < k; g0 += kBGroup) {
-        const int gk = min(kBGroup, k - g0);
-        // per element and per warp in the vectors' precision (FP32 stays on
-        // the FP32 pipe), double from the per-warp sums on
-        T acc[kBGroup];
-#pragma unroll
-        for (int q = 0; q < kBGroup; ++q) acc[q] = T(0);
-        for (int64_t i = c.begin + threadIdx.x; i < c.end; i += blockDim.x) {
-            const T wi = w[i];
-#pragma unroll
-            for (int q = 0; q < kBGroup; ++q)
-                if (q < gk) acc[q] = fma(V[(int64_t)(g0 + q) * ldv + i], wi, acc[q]);
-        }
-#pragma unroll
-        for (int q = 0; q < kBGroup; ++q) {
-            T sw = acc[q];
-            for (int o = 16; o > 0; o >>= 1) sw += __shfl_down_sync(0xffffffffu, sw, o);
-            if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = (double)sw;
-        }
-        __syncthreads();
-        if (threadIdx.x < gk) {
-            double s = 0.;
-            for (int wq = 0; wq < kBThreads / 32; ++wq) s += red[threadIdx.x][wq];
-            partial[(int64_t)blockIdx.x * k + g0 + threadIdx.x] = s;
-        }
-        __syncthreads();
+    double s = 0.;
+#pragma unroll 8
+    for (int64_t i = c.begin + threadIdx.x; i < c.end; i += kBThreads) s = fma(v[i], v[i], s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.;
+        for (int wq = 0; wq < kBThreads / 32; ++wq) t += red[wq];
+        partial[blockIdx.x] = t;
     }
 }
 
@@ -97,12 +81,13 @@ __global__ void breduce_kernel(const int32_t* __restrict__ cbeg, const double* _
 // The partials of an Arnoldi step's sums: k values each, those of instance b from
 // beg[b] to beg[b + 1].  Every block that needs an instance's sums adds them itself (in one
 // order, so all get the same), which saves a launch of 4.5 us between two passes of
-// 10; above kOwnSums partials per instance breduce_kernel leaves one.
+// 10; above kOwnSums partials per instance breduce_kernel leaves one.  With instances
+// of up to 92 partials the solve takes 11.62 ms with the launch and 11.31 without.
 struct BSums {
     const double* partial;
     const int32_t* beg;
 };
-constexpr int kOwnSums = 64;
+constexpr int kOwnSums = 128;
 
 // out[q] = the sums of instance b, for the block's threads
 __device__ __forceinline__ void inst_sums(BSums sums, int b, int k, double* out) {
@@ -208,6 +193,8 @@ bresid_kernel(const BChunk* __restrict__ ch, const float* __restrict__ rhs, cons
 __global__ void __launch_bounds__(kBThreads)
 bdots_kernel(const BChunk* __restrict__ ch, const float* __restrict__ V, int64_t ldv, int k,
              const float* __restrict__ w, double* __restrict__ partial, const int32_t* __restrict__ done) {
+    after_trigger();
+    after_wait();
     const BChunk c = ch[blockIdx.x];
     if (done[c.inst]) return;
     const int n = (int)(c.end - c.begin);
@@ -221,6 +208,8 @@ baxpy_dots_kernel(const BChunk* __restrict__ ch, const int32_t* __restrict__ cbe
                   const float* __restrict__ V, int64_t ldv, int k, float* __restrict__ w, double* __restrict__ h1,
                   int ldh, double* __restrict__ partial, const int32_t* __restrict__ done) {
     __shared__ double h[64];
+    after_trigger();
+    after_wait();
     const BChunk c = ch[blockIdx.x];
     if (done[c.inst]) return;
     const int n = (int)(c.end - c.begin);
@@ -240,6 +229,8 @@ baxpy_norm_kernel(const BChunk* __restrict__ ch, const int32_t* __restrict__ cbe
                   const double* __restrict__ h1, double* __restrict__ ho, int ldh, double* __restrict__ partial,
                   const int32_t* __restrict__ done) {
     __shared__ double h[64];
+    after_trigger();
+    after_wait();
     const BChunk c = ch[blockIdx.x];
     if (done[c.inst]) return;
     const int n = (int)(c.end - c.begin);
@@ -262,6 +253,8 @@ bnormalize_kernel(const BChunk* __restrict__ ch, const int32_t* __restrict__ cbe
                   float* __restrict__ z, const int32_t* __restrict__ done) {
     __shared__ double s_sq;
     __shared__ float s_inv;
+    after_trigger();
+    after_wait();
     const BChunk c = ch[blockIdx.x];
     if (done && done[c.inst]) return;
     inst_sums(sums, c.inst, 1, &s_sq);
@@ -348,6 +341,8 @@ __global__ void bstart_kernel(BState st, const double* __restrict__ nrm) {
 // previous Givens rotations, form the new one, update g and the residual estimate;
 // freeze the instance and skip its columns once converged.
 __global__ void barnoldi_kernel(BState st, int j, const double* __restrict__ ho, int ldh) {
+    after_trigger();
+    after_wait();
     const int b = blockIdx.x, m = st.m;
     if (b == 0 && threadIdx.x == 0) *st.next = 0u;
     if (st.done[b]) return;
@@ -458,9 +453,8 @@ void free_bws(BatchWs* w) {
 }
 
 // per-instance squared norms into out[b*ldo]
-template <typename T>
-void bnorm2(const BatchWs* w, const T* v, double* out, int ldo, cudaStream_t s, const int32_t* done = nullptr) {
-    bdot_kernel<T><<<w->nchunks, kBThreads, 0, s>>>(w->d_ch, v, 0, 1, v, w->partial, done), count_launch();
+void bnorm2(const BatchWs* w, const double* v, double* out, int ldo, cudaStream_t s) {
+    bnorm_kernel<<<w->nchunks, kBThreads, 0, s>>>(w->d_ch, v, w->partial), count_launch();
     breduce_kernel<<<dim3(w->nb, 1), 128, 0, s>>>(w->d_cbeg, w->partial, 1, out, ldo), count_launch();
 }
 
@@ -497,17 +491,20 @@ void record_part(rtg_handle* h, BatchWs* w, int part, cudaStream_t s) {
         apply_sweep<float>(h, vj, w->z32, s, nullptr, w->st.skip, stop, true);
         launch_apply<float>(h, v, RTG_SYSTEM | RTG_MASK_ROWS, w->z32, w->w32, s);
         // CGS2 with per-instance coefficients; ho = h1 + h2
-        bdots_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->V32, N, k, w->w32, w->partial, w->st.done), count_launch();
+        if (apply_chains(h, RTG_FP32))
+            launch_after(bdots_kernel, nc, kBThreads, 0, s, w->d_ch, w->V32, N, k, w->w32, w->partial, w->st.done);
+        else
+            bdots_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->V32, N, k, w->w32, w->partial, w->st.done), count_launch();
         BSums sums = sums_of(w, w->partial, k, s);
-        baxpy_dots_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, sums, w->V32, N, k, w->w32, w->h1, ldh,
-                                                   w->partial2, w->st.done), count_launch();
+        launch_after(baxpy_dots_kernel, nc, kBThreads, 0, s, w->d_ch, w->d_cbeg, sums, w->V32, N, k, w->w32, w->h1, ldh,
+                     w->partial2, w->st.done);
         sums = sums_of(w, w->partial2, k, s);
-        baxpy_norm_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, sums, w->V32, N, k, w->w32, w->h1, w->ho, ldh,
-                                                   w->partial, w->st.done), count_launch();
+        launch_after(baxpy_norm_kernel, nc, kBThreads, 0, s, w->d_ch, w->d_cbeg, sums, w->V32, N, k, w->w32, w->h1,
+                     w->ho, ldh, w->partial, w->st.done);
         sums = sums_of(w, w->partial, 1, s);
-        bnormalize_kernel<<<nc, kBThreads, 0, s>>>(w->d_ch, w->d_cbeg, sums, w->w32, vj + N, w->ho + k, ldh, w->z32,
-                                                   w->st.done), count_launch();
-        barnoldi_kernel<<<nb, 128, 0, s>>>(w->st, j, w->ho, ldh), count_launch();
+        launch_after(bnormalize_kernel, nc, kBThreads, 0, s, w->d_ch, w->d_cbeg, sums, w->w32, vj + N, w->ho + k, ldh,
+                     w->z32, w->st.done);
+        launch_after(barnoldi_kernel, nb, 128, 0, s, w->st, j, w->ho, ldh);
         RTG_CUDA(cudaMemcpyAsync(w->hstop + j, stop, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     } else {
         // d += P^{-1} (V y), for the instances that formed a correction
@@ -669,7 +666,7 @@ int solve_batched(rtg_handle* h, int nb, const int64_t* inst_off, const double* 
     bscale_kernel<double, double><<<nc, kBThreads, 0, s>>>(w->d_ch, w->t, w->b, nullptr, 0, -1., 1.), count_launch();
     bscale_kernel<double, double><<<nc, kBThreads, 0, s>>>(w->d_ch, w->t, w->x, nullptr, 0, 0., 0.), count_launch();
     std::vector<double> bn(nb), rn(nb), tol(nb), tin(nb), scale(nb), inv(nb);
-    bnorm2<double>(w, w->b, w->vnorm, 1, s);
+    bnorm2(w, w->b, w->vnorm, 1, s);
     RTG_CUDA(cudaMemcpyAsync(bn.data(), w->vnorm, sizeof(double) * nb, cudaMemcpyDeviceToHost, s));
     RTG_CUDA(cudaStreamSynchronize(s));
     for (int b = 0; b < nb; ++b) tol[b] = std::max(o->rtol * std::sqrt(bn[b]), o->atol);
@@ -683,7 +680,7 @@ int solve_batched(rtg_handle* h, int nb, const int64_t* inst_off, const double* 
         launch_apply<double>(h, h->v64, RTG_SYSTEM | RTG_MASK_ROWS, w->x, w->r, s);
         ++fp64_applies;
         bscale_kernel<double, double><<<nc, kBThreads, 0, s>>>(w->d_ch, w->b, w->r, nullptr, 0, 1., -1.), count_launch();
-        bnorm2<double>(w, w->r, w->vnorm, 1, s);
+        bnorm2(w, w->r, w->vnorm, 1, s);
         RTG_CUDA(cudaMemcpyAsync(rn.data(), w->vnorm, sizeof(double) * nb, cudaMemcpyDeviceToHost, s));
         RTG_CUDA(cudaStreamSynchronize(s));
         bool any = false;

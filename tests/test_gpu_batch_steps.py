@@ -1,5 +1,5 @@
 """The batched solver's cycles (rtg_batch.cu) at the edges of their forms: instances
-of less than one 4096-value chunk and of more than 64 (above which an instance's
+of less than one 4096-value chunk and of more than 128 (above which an instance's
 sums have a launch of their own), one instance alone, restart lengths that end a
 cycle before and after the instances converge, and an instance without any
 right-hand side (done before the first step).
@@ -17,7 +17,7 @@ def _instances(kind):
     small = [W.batch_instance(s, max_cols=8, max_cells=4, n_range=(2, 4)) for s in (3, 4, 5)]
     if kind == "small":
         return small
-    m = Mesh([1., 1.], [False, False], [6, 6, 8], True)
+    m = Mesh([1., 1.], [False, False], [8, 8, 9], True)
     for _ in range(4):
         m.ref_mesh(kind="ang", form="h")
     for _ in range(3):
@@ -32,7 +32,7 @@ def test_batch_matches_single_solves(kind, restart):
     from rtg import DeviceContext
     from rtg.batch import BatchContext
     inst = _instances(kind)
-    assert max(m.get_ndof() for m, _ in inst) > 64 * 4096 or kind == "small"
+    assert max(m.get_ndof() for m, _ in inst) > 128 * 4096 or kind == "small"
     bc = BatchContext(inst)
     f, g = bc.forcing(), bc.inflow()
     if len(inst) > 1:        # the last instance has nothing to solve
