@@ -648,7 +648,7 @@ def run_ours(args):
                    "kernels_us": {"sweep_fp32": 1e6 * t_sweep, "sweep_fp64": 1e6 * t_sweep64,
                                   "apply_fp32": 1e6 * t_apply, "apply_fp64": 1e6 * t_apply64},
                    "apply_fp64": {"flops": int(ctx.info["flops_per_apply"]),
-                                  "note": "FP64-pipe bound (GB300 FP64 rate is 1/64 of FP32)"},
+                                  "note": "tiled kernel FP64-pipe bound (GB300 FP64 rate is 1/64 of FP32), the product on the tensor cores in digits"},
                    "sweep": {"levels": nlev, "lagged_couplings": nlag},
                    "parallelism": "replicas" if world > 1 else "single GPU"},
         "e2e": {"value": e2e, "unit": "s", "h2d_bytes_per_step": 2 * 8 * N,

@@ -2047,8 +2047,8 @@ static int plan_launches(const ApplyPlan* p) {
 // Multiply-adds of the scattering product from which FP64 plans with the
 // tensor cores (rtg_scat64.cu; FP32 plans: more shapes, tune_plan) are timed beside those of the FP64 pipe, and from
 // which they alone are.  Whole applies, FP64 pipe against tensor cores, in us: 19.8
-// and 27.9 at 1.2e6 (33,056 DOF adaptive: an extra launch), 51.6 and 49.9 at 8.6e6
-// (218,581 DOF adaptive), 73 and 38 at 2.1e7, 459 and 103 at 1.6e8, 4067 and 870 at
+// and 27.9 at 1.2e6 (33,056 DOF adaptive: an extra launch), 51.6 and 45.4 at 8.6e6
+// (218,581 DOF adaptive), 73 and 38 at 2.1e7, 459 and 103 at 1.6e8, 4067 and 920 at
 // 1.5e9 (7.95e6 DOF, two scatterers).
 constexpr int64_t kTcOffer = 4'000'000, kTc64Alone = 100'000'000;
 
