@@ -972,8 +972,11 @@ apply_tiled_kernel(OpView<T> v, TileParity<T> par, uint32_t flags, const int4* _
 // another stream (exactly two terms on zero, so the sum does not depend on
 // their order); rows of inflow-boundary nodes stay zero.
 // Each value is split into TF32 hi + lo parts (hi = round-to-nearest TF32,
-// lo = value - hi, exact in FP32) and D accumulates A_lo B_hi + A_hi B_lo +
-// A_hi B_hi with tcgen05.mma (kind::tf32, M = 128, N = nij padded to 16,
+// lo = value - hi, exact in FP32) and A_lo B_hi + A_hi B_lo accumulate beside
+// A_hi B_hi, whose sum then takes a third of the additions, each of which the
+// tensor cores cut off to FP32 (error of a whole apply 1.07e-7 against 1.33e-7 with one
+// accumulator at 1.02e6 DOF, two scatterers, 0.83e-7 on the FP32 pipe; the same
+// time), with tcgen05.mma (kind::tf32, M = 128, N = nij padded to 16,
 // K = 8 per instruction, one issuing thread) in tensor memory.  The K axis
 // (the column's angular nodes) is walked in chunks of kTcK: W's hi/lo tile of
 // the chunk is built once per handle on the host in the shared-memory image
@@ -1044,7 +1047,7 @@ scat_tc_kernel(OpView<float> v, uint32_t flags, const TcItem* __restrict__ items
     const ColDev C = v.cols[it.col];
     const ApplyFlags fl = decode(flags);
     const int nij = C.nx * C.ny, Nth = C.nth_col, ncell = C.elem_end - C.elem_begin;
-    const int np = tc_np(nij), ncols = tc_tmem_cols(np);
+    const int np = tc_np(nij), ncols = tc_tmem_cols(2 * np);
     float* As = tsm;                       // W tile: hi [kTcM x kTcK] | lo
     float* Bh = As + kTcTileFloats;        // x: hi [np x kTcK] | lo
     float* Bl = Bh + np * kTcK;
@@ -1131,9 +1134,9 @@ scat_tc_kernel(OpView<float> v, uint32_t flags, const TcItem* __restrict__ items
 #pragma unroll
                 for (int s = 0; s < kTcK / 8; ++s) {
                     const int o = 64 * s;   // two K-adjacent core matrices per K = 8
-                    tc_mma(tmem, tc_desc(Al + o), tc_desc(Bh + o), idesc, ch > 0 || s > 0);
-                    tc_mma(tmem, tc_desc(Ah + o), tc_desc(Bl + o), idesc, 1);
-                    tc_mma(tmem, tc_desc(Ah + o), tc_desc(Bh + o), idesc, 1);
+                    tc_mma(tmem + np, tc_desc(Al + o), tc_desc(Bh + o), idesc, ch > 0 || s > 0);
+                    tc_mma(tmem + np, tc_desc(Ah + o), tc_desc(Bl + o), idesc, 1);
+                    tc_mma(tmem, tc_desc(Ah + o), tc_desc(Bh + o), idesc, ch > 0 || s > 0);
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                                  mb_mma)
@@ -1162,13 +1165,15 @@ scat_tc_kernel(OpView<float> v, uint32_t flags, const TcItem* __restrict__ items
         const float dxdy8 = v.colc[it.col];
         const int half = np / 2;
         for (int cb = h * half; cb < (h + 1) * half; cb += 8) {
-            uint32_t d[8];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
-                "tcgen05.wait::ld.sync.aligned;"
-                : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
-                : "r"(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)cb)
-                : "memory");
+            uint32_t d[2][8];   // hi hi, and the terms with a lo
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                             : "=r"(d[u][0]), "=r"(d[u][1]), "=r"(d[u][2]), "=r"(d[u][3]), "=r"(d[u][4]), "=r"(d[u][5]),
+                               "=r"(d[u][6]), "=r"(d[u][7])
+                             : "r"(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(u * np + cb))
+                             : "memory");
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (!valid) continue;
 #pragma unroll
             for (int jj = 0; jj < 8; ++jj) {
@@ -1177,7 +1182,7 @@ scat_tc_kernel(OpView<float> v, uint32_t flags, const TcItem* __restrict__ items
                 const int i = ij / C.ny, j = ij % C.ny;
                 if (fl.mask_rows && bdry_node(s_cflg[kc] >> 4, i, j, C.nx, C.ny)) continue;
                 const int64_t dof = C.dof_off + (int64_t)nij * s_crow[kc] + (int64_t)ij * nth + r;
-                atomicAdd(y + dof, -dxdy8 * v.sw[C.node_off + ij] * __uint_as_float(d[jj]));
+                atomicAdd(y + dof, -dxdy8 * v.sw[C.node_off + ij] * (__uint_as_float(d[0][jj]) + __uint_as_float(d[1][jj])));
             }
         }
     }
