@@ -114,8 +114,9 @@ __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast
 // outT[c][r] = relu(sum_k inT[k][r] W[k][c] + b[c]); thread: 4 rows x 4 columns
 template <int K, int LDW>
 __device__ __forceinline__ void layer_relu(const float* __restrict__ inT, const float* __restrict__ W,
-                                           const float* __restrict__ b, float* __restrict__ outT) {
+                                           const float* __restrict__ b, float* __restrict__ outT, int nr) {
     const int w = threadIdx.x >> 5;
+    if (16 * (w & 3) >= nr) return;   // no row of the tile's
     const int r0 = 16 * (w & 3) + 4 * lane4(), c0 = 32 * (w >> 2) + 4 * lane8();
     float2 acc[2][4];   // [row pair][column]
 #pragma unroll
@@ -153,14 +154,14 @@ __device__ __forceinline__ float row_gate(float f0, float f1) {
 // outputs in sO[c][r].
 // f holds this thread's features of the tile (load_features), which are loaded a
 // tile ahead.
-__device__ __forceinline__ void load_features(float (&f)[kFeat], const float* __restrict__ F, int64_t r0, int64_t rows) {
+__device__ __forceinline__ void load_features(float (&f)[kFeat], const float* __restrict__ F, int64_t r0, int64_t end) {
 #pragma unroll
     for (int u = 0; u < kFeat; ++u) {
         const int t = threadIdx.x + u * kMlpThreads;
-        f[u] = r0 + t / kIn < rows ? F[r0 * kIn + t] : 0.f;
+        f[u] = r0 + t / kIn < end ? F[r0 * kIn + t] : 0.f;
     }
 }
-__device__ __forceinline__ void forward_tile(const float (&f)[kFeat], float* sm) {
+__device__ __forceinline__ void forward_tile(const float (&f)[kFeat], int nr, float* sm) {
     float* Ft = sm + sF;
 #pragma unroll
     for (int u = 0; u < kFeat; ++u) {
@@ -169,9 +170,9 @@ __device__ __forceinline__ void forward_tile(const float (&f)[kFeat], float* sm)
     }
     __syncthreads();
     if (threadIdx.x < kTile) sm[sG + threadIdx.x] = row_gate(Ft[threadIdx.x], Ft[kLd + threadIdx.x]);
-    layer_relu<kIn, kHid>(Ft, sm + sW1, sm + sB1, sm + sH1);
+    layer_relu<kIn, kHid>(Ft, sm + sW1, sm + sB1, sm + sH1, nr);
     __syncthreads();
-    layer_relu<kHid, kLd2>(sm + sH1, sm + sW2, sm + sB2, sm + sH2);
+    layer_relu<kHid, kLd2>(sm + sH1, sm + sW2, sm + sB2, sm + sH2, nr);
     __syncthreads();
     if (threadIdx.x < 128) {   // one warp per scheduler, 6 columns each; lanes of 2 rows
         const int r = 2 * (threadIdx.x & 31), c0 = 6 * (threadIdx.x >> 5);
@@ -200,19 +201,19 @@ __device__ __forceinline__ void forward_tile(const float (&f)[kFeat], float* sm)
 }
 
 __global__ void __launch_bounds__(kMlpThreads, 1)
-nn_forward_kernel(const float* __restrict__ P, const float* __restrict__ F, int64_t rows, float* __restrict__ O) {
+nn_forward_kernel(const float* __restrict__ P, const float* __restrict__ F, int64_t rows, int64_t per,
+                  float* __restrict__ O) {
     extern __shared__ float4 smem4[];
     float* sm = reinterpret_cast<float*>(smem4);
     float f[kFeat];
-    load_features(f, F, (int64_t)blockIdx.x * kTile, rows);
+    const int64_t begin = min(blockIdx.x * per, rows), end = min(begin + per, rows);
+    load_features(f, F, begin, end);
     stage_params(P, sm);
     __syncthreads();
-    const int64_t ntiles = (rows + kTile - 1) / kTile;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t r0 = tile * kTile;
-        const int nr = (int)(rows - r0 < kTile ? rows - r0 : kTile);
-        forward_tile(f, sm);
-        load_features(f, F, (tile + gridDim.x) * kTile, rows);
+    for (int64_t r0 = begin; r0 < end; r0 += kTile) {
+        const int nr = (int)(end - r0 < kTile ? end - r0 : kTile);
+        forward_tile(f, nr, sm);
+        load_features(f, F, r0 + kTile, end);
         for (int t = threadIdx.x; t < nr * kOut; t += blockDim.x) O[r0 * kOut + t] = sm[sO + t % kOut * kLd + t / kOut];
         __syncthreads();
     }
@@ -224,19 +225,21 @@ nn_forward_kernel(const float* __restrict__ P, const float* __restrict__ F, int6
 // bounds it besides is the operands from shared memory.  Register tiles of 4 x 4
 // (forward, dh) and 4 x 8 (dW2) outputs per thread, lanes that share operands next
 // to each other, 16 warps in one CTA per SM, and dh2 and dh1 in buffers of their
-// own, so that two products run between barriers: 110 us at 32,768 rows (54e3
+// own, so that two products run between barriers: 106 us at 32,768 rows (54e3
 // cycles per tile, 46e3 of them in the four 128-wide products), 182 us with 256
 // threads, scalar reads of dO, W3 and W2 and two CTAs in turn on half of the SMs.
 // The chains of the forward pass keep their order of k, so the loss does not
 // depend on the tiling.
 __global__ void __launch_bounds__(kMlpThreads, 1)
 nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const float* __restrict__ Mo,
-               const float* __restrict__ S, int64_t rows, float* __restrict__ work, double* __restrict__ lossw) {
+               const float* __restrict__ S, int64_t rows, int64_t per, float* __restrict__ work,
+               double* __restrict__ lossw) {
     extern __shared__ float4 smem4[];
     float* sm = reinterpret_cast<float*>(smem4);
     __shared__ double red[kTile / 32];
     float f[kFeat];
-    load_features(f, F, (int64_t)blockIdx.x * kTile, rows);
+    const int64_t begin = min(blockIdx.x * per, rows), end = min(begin + per, rows);
+    load_features(f, F, begin, end);
     stage_params(P, sm);
     __syncthreads();
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -264,18 +267,17 @@ nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const f
     float* h2T = sm + sH2;
     float* dT = sm + sD;
     float* dOT = sm + sO;
-    const int64_t ntiles = (rows + kTile - 1) / kTile;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t r0 = tile * kTile;
-        const int nr = (int)(rows - r0 < kTile ? rows - r0 : kTile);
+    for (int64_t r0 = begin; r0 < end; r0 += kTile) {
+        const int nr = (int)(end - r0 < kTile ? end - r0 : kTile);
+        const int rlim = (nr + 3) & ~3;   // the rows past nr have no gradient
         // the row's moments and statistics, in flight during the forward pass
         float m[kMom], s[10];
 #pragma unroll
         for (int l = 0; l < kMom; ++l) m[l] = t < nr ? Mo[(r0 + t) * kMom + l] : 0.f;
 #pragma unroll
         for (int l = 0; l < 10; ++l) s[l] = t < nr ? S[(r0 + t) * kSt + l] : 0.f;
-        forward_tile(f, sm);
-        load_features(f, F, (tile + gridDim.x) * kTile, rows);
+        forward_tile(f, nr, sm);
+        load_features(f, F, r0 + kTile, end);
         // o = C m, loss, dL/dC = (dL/do) m^T, and dL/d(pre-gate outputs) = g dL/dC in place of C
         if (t < kTile) {
             float d[3] = {0.f, 0.f, 0.f};
@@ -309,7 +311,7 @@ nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const f
             const float* hp = h2T + (16 * (w >> 1) + l8) * kLd;
             const float* dp = dOT + (12 * (w & 1) + 3 * l4) * kLd;
 #pragma unroll 4
-            for (int r = 0; r < kTile; r += 4) {
+            for (int r = 0; r < rlim; r += 4) {
                 float4 a[2], b[3];
 #pragma unroll
                 for (int p = 0; p < 2; ++p) a[p] = ld4(hp + 8 * p * kLd + r);
@@ -328,7 +330,7 @@ nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const f
         }
         // dh2[r][k] = [h2 > 0] sum_c dO[r][c] W3[k][c], and db2
         const int rr = 16 * (w & 3) + 4 * l4, kk = 32 * (w >> 2) + l8;   // 4 rows, units kk + 8j
-        {
+        if (16 * (w & 3) < nr) {
             float2 acc[4][2];   // [unit][row pair]
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_float2(0.f, 0.f);
@@ -367,7 +369,7 @@ nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const f
             const float* hp = h1T + (32 * (w & 3) + l8) * kLd;
             const float* dp = dT + (32 * (w >> 2) + l4) * kLd;
 #pragma unroll 1
-            for (int r = 0; r < kTile; r += 4) {
+            for (int r = 0; r < rlim; r += 4) {
                 float4 a[4];
 #pragma unroll
                 for (int p = 0; p < 4; ++p) a[p] = ld4(hp + 8 * p * kLd + r);
@@ -382,7 +384,7 @@ nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const f
             }
         }
         // dh1[r][k] = [h1 > 0] sum_c dh2[r][c] W2[k][c] in place of h2, and db1
-        {
+        if (16 * (w & 3) < nr) {
             float2 acc[4][2];   // [unit][row pair]
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_float2(0.f, 0.f);
@@ -421,7 +423,7 @@ nn_grad_kernel(const float* __restrict__ P, const float* __restrict__ F, const f
             const float* fp = Ft + l8 * kLd;
             const float* dp = h2T + (8 * w + l4) * kLd;
 #pragma unroll 4
-            for (int r = 0; r < kTile; r += 4) {
+            for (int r = 0; r < rlim; r += 4) {
                 float4 a[2], b[2];
 #pragma unroll
                 for (int p = 0; p < 2; ++p) a[p] = ld4(fp + 8 * p * kLd + r), b[p] = ld4(dp + 4 * p * kLd + r);
@@ -933,12 +935,18 @@ void nn_features(rtg_handle* h, float* feat, cudaStream_t s) {
     RTG_CUDA(cudaGetLastError());
 }
 
+// Rows of a CTA: an equal share, so that no SM has a whole tile more than another
+// (the kernels leave out the part of a CTA's last tile that has no rows: 512 tiles on
+// 152 SMs are 3.4 rounds of work instead of 4), but no less than a tile.
+static int64_t rows_per_cta(int64_t rows) {
+    return std::max<int64_t>(kTile, ((rows + kGradCtas - 1) / kGradCtas + 3) & ~3);
+}
+
 void nn_forward(const float* params, const float* feat, int64_t rows, float* coef, cudaStream_t s) {
     if (rows <= 0) return;
     mlp_attributes();
-    const int64_t ntiles = (rows + kTile - 1) / kTile;
-    const int grid = (int)std::min<int64_t>(ntiles, kGradCtas);
-    nn_forward_kernel<<<grid, kMlpThreads, kMlpSmem, s>>>(params, feat, rows, coef), count_launch();
+    const int64_t per = rows_per_cta(rows);
+    nn_forward_kernel<<<(int)((rows + per - 1) / per), kMlpThreads, kMlpSmem, s>>>(params, feat, rows, per, coef), count_launch();
     RTG_CUDA(cudaGetLastError());
 }
 
@@ -1010,11 +1018,11 @@ int64_t nn_work_floats() { return (int64_t)kGradCtas * kNP + 2 * kGradCtas; }
 void nn_loss_grad(const float* params, const float* feat, const float* mom, const float* stats, int64_t rows,
                   float* work, float* grad, double* loss, cudaStream_t s) {
     mlp_attributes();
-    const int64_t ntiles = std::max<int64_t>(1, (rows + kTile - 1) / kTile);
-    const int grid = (int)std::min<int64_t>(ntiles, kGradCtas);
+    rows = std::max<int64_t>(rows, 0);
+    const int64_t per = rows_per_cta(rows);
+    const int grid = (int)std::max<int64_t>(1, (rows + per - 1) / per);
     double* lossw = reinterpret_cast<double*>(work + (int64_t)kGradCtas * kNP);
-    nn_grad_kernel<<<grid, kMlpThreads, kMlpSmem, s>>>(params, feat, mom, stats, std::max<int64_t>(rows, 0), work,
-                                                       lossw), count_launch();
+    nn_grad_kernel<<<grid, kMlpThreads, kMlpSmem, s>>>(params, feat, mom, stats, rows, per, work, lossw), count_launch();
     nn_reduce_grad_kernel<<<(kNP + kRedParams - 1) / kRedParams, kRedParams * kRedSlices, 0, s>>>(work, grid, lossw, grad, loss), count_launch();
     RTG_CUDA(cudaGetLastError());
 }
