@@ -92,14 +92,19 @@ class Projection:
             self.cols[ck] = ProjectionColumn(col, cells)
         self._flat = (vec, views)
 
+    def __getstate__(self):
+        """Copies and pickles hold the cells' values, not the vector besides."""
+        state = self.__dict__.copy()
+        state.pop("_flat", None)
+        return state
+
     def to_vector(self):
         out = []
         for ck in sorted(self.cols.keys()):
             cells = self.cols[ck].cells
             out += [cells[kk].vals for kk in sorted(cells.keys())]
-        # as built: every cell still holds its own view of the vector (a copied or
-        # unpickled projection's arrays are no views)
-        vec, views = self._flat
+        # as built: every cell still holds its own view of the vector
+        vec, views = self.__dict__.get("_flat", (None, ()))
         if len(out) == len(views) and all(map(operator.is_, out, views)) and all(v.base is vec for v in views):
             return vec.reshape(-1).copy()
         return np.concatenate([a.reshape(-1) for a in out])
