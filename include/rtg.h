@@ -212,6 +212,15 @@ int rtg_apply_tuning(rtg_handle* h, int32_t* table, int cap_rows, int* nclasses,
  * autotuning on the next apply.  Synchronizes the device and drops the
  * solver's captured graphs (they hold the old plan's launches). */
 int rtg_apply_shape(rtg_handle* h, int prec, const int32_t* shape);
+/* The table of rtg_apply_tuning for either precision (a fixed plan: its one
+ * row).  In FP64 the fourth value is 1 where the scattering product runs on the
+ * tensor cores. */
+int rtg_apply_plans(rtg_handle* h, int prec, int32_t* table, int cap_rows, int* nshapes, void* stream);
+/* As rtg_apply_shape with {rows, 1, 0, 0} in FP64, but with the scattering
+ * product on the tensor cores.  RTG_ERR_SIZE, and the plan stays as it is, when
+ * a column has more than 256 angular nodes or the digits cannot hold a
+ * scattering matrix. */
+int rtg_apply_digits(rtg_handle* h, int rows);
 /* mask[N] (device, uint8): 1 for unknowns, 0 for inflow-boundary DOFs. */
 int rtg_interior_mask(rtg_handle* h, uint8_t* mask, void* stream);
 /* out = x with the entries of one part zeroed: part 0 keeps the unknowns,

@@ -2105,6 +2105,20 @@ static float time_plan(rtg_handle* h, ApplyPlan* p, const T* x, T* y, cudaEvent_
     return tt;
 }
 
+// Digit tables of the tiled columns, into par->s64 (null when a W cannot be held)
+static void make_digits(rtg_handle* h, ParityTables* par) {
+    std::vector<int> cap(h->host.cols.size(), kTileRows);
+    ApplyPlan* probe = make_plan<double>(h, &cap, nullptr, kChunk64, par, 0, 0, 1);
+    try {
+        par->s64 = build_scat64(h, probe->tiled, par->scls.data(), par->thr.data(), par->d_thr);
+        par->s64_cols = probe->tiled;
+    } catch (...) {
+        free_plan(probe);
+        throw;
+    }
+    free_plan(probe);
+}
+
 // Autotuner of the apply: every plan shape of the candidate list (rows per
 // item 4 to 64, one CTA per column or per item, one launch or one per
 // shared-memory class, with or without the tensor-core scattering) is built
@@ -2141,18 +2155,7 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
             prod += (int64_t)C.nx * C.ny * C.nth_col * C.nth_col;
             all_fit &= scat64_fits(C);
         }
-        if (f64 && all_fit && prod >= kTcOffer) {
-            std::vector<int> cap(h->host.cols.size(), kTileRows);
-            ApplyPlan* probe = make_plan<T>(h, &cap, nullptr, kChunk64, par, 0, 0, 1);
-            try {
-                par->s64 = build_scat64(h, probe->tiled, par->scls.data(), par->thr.data(), par->d_thr);
-                par->s64_cols = probe->tiled;
-            } catch (...) {
-                free_plan(probe);
-                throw;
-            }
-            free_plan(probe);
-        }
+        if (f64 && all_fit && prod >= kTcOffer) make_digits(h, par);
         const bool tc64 = f64 && par->s64;
         std::vector<PlanShape> shapes;
         if (f64 && prod < kTc64Alone) {
@@ -2259,8 +2262,20 @@ static void force_shape(rtg_handle* h, const PlanShape& sh) {
     ParityTables* par = f64 ? build_parity(h) : nullptr;
     ApplyPlan* p = nullptr;
     try {
+        if constexpr (f64) {
+            if (sh.tc) {
+                bool fit = true;
+                for (const ColDev& C : h->host.cols)
+                    fit &= C.elem_end - C.elem_begin > kMaxCellsStaged || scat64_fits(C);
+                if (fit) make_digits(h, par);
+                if (!par->s64) throw RtgError{RTG_ERR_SIZE, "the digits cannot hold this operator's scattering matrices"};
+            }
+        }
         p = shape_plan<T>(h, sh, par);
+        if (f64 && sh.tc && p->tiled != par->s64_cols)
+            throw RtgError{RTG_ERR_SIZE, "rows per item: not the columns of the digit tables"};
     } catch (...) {
+        free_plan(p);
         if (par) free_parity(par);
         throw;
     }
@@ -2295,12 +2310,21 @@ int apply_shape(rtg_handle* h, int prec, const int32_t* shape) {
     return 0;
 }
 
-int apply_tuning(rtg_handle* h, int32_t* out, int cap_rows, cudaStream_t s) {
-    if (!h->plan32) {
+void apply_digits(rtg_handle* h, int rows) {
+    if (rows < 1 || rows > 1024) throw RtgError{RTG_ERR_ARG, "rows in [1, 1024]"};
+    force_shape<double>(h, PlanShape{rows, 1, 0, 1});
+}
+
+int apply_tuning(rtg_handle* h, int prec, int32_t* out, int cap_rows, cudaStream_t s) {
+    if (prec == RTG_FP64 && !h->plan64) {
+        h->plan64 = tune_plan<double>(h, s);
+        set_plan_attributes<double>(h->plan64);
+    }
+    if (prec == RTG_FP32 && !h->plan32) {
         h->plan32 = tune_plan<float>(h, s);
         set_plan_attributes<float>(h->plan32);
     }
-    const auto& rec = h->plan32->tuning;
+    const auto& rec = (prec == RTG_FP64 ? h->plan64 : h->plan32)->tuning;
     const int n = (int)rec.size();
     for (int i = 0; i < std::min(n, cap_rows); ++i) {
         int32_t* o = out + (size_t)i * 9;

@@ -429,7 +429,7 @@ int rtg_sweep_trace(rtg_handle* h, int prec, const void* r, void* z, uint64_t* t
 int rtg_apply_tuning(rtg_handle* h, int32_t* table, int cap_rows, int* nclasses, void* stream) {
     return guard("rtg_apply_tuning", [&] {
         if (!h || !nclasses || (cap_rows > 0 && !table)) throw RtgError{RTG_ERR_ARG, "null argument"};
-        *nclasses = apply_tuning(h, table, cap_rows, (cudaStream_t)stream);
+        *nclasses = apply_tuning(h, RTG_FP32, table, cap_rows, (cudaStream_t)stream);
     });
 }
 
@@ -444,6 +444,25 @@ int rtg_apply_shape(rtg_handle* h, int prec, const int32_t* shape) {
         free_workspace(h);
         free_batch(h);
         apply_shape(h, prec, shape);
+    });
+}
+
+int rtg_apply_plans(rtg_handle* h, int prec, int32_t* table, int cap_rows, int* nshapes, void* stream) {
+    return guard("rtg_apply_plans", [&] {
+        if (!h || !nshapes || (cap_rows > 0 && !table)) throw RtgError{RTG_ERR_ARG, "null argument"};
+        if (prec != RTG_FP64 && prec != RTG_FP32) throw RtgError{RTG_ERR_ARG, "prec must be RTG_FP64 or RTG_FP32"};
+        *nshapes = apply_tuning(h, prec, table, cap_rows, (cudaStream_t)stream);
+    });
+}
+
+int rtg_apply_digits(rtg_handle* h, int rows) {
+    return guard("rtg_apply_digits", [&] {
+        if (!h) throw RtgError{RTG_ERR_ARG, "null handle"};
+        RTG_CUDA(cudaSetDevice(h->device));
+        RTG_CUDA(cudaDeviceSynchronize());
+        free_workspace(h);
+        free_batch(h);
+        apply_digits(h, rows);
     });
 }
 

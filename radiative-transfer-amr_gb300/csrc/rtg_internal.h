@@ -273,13 +273,14 @@ void free_apply_plans(rtg_handle* h);
 // RTG_ERR_TIMEOUT (and the handle poisoned) if a tensor-core wait of the FP32
 // apply gave up since the plan was built, else RTG_OK; one device read
 int apply_status(rtg_handle* h, cudaStream_t s);
-// FP32 apply autotuning table (tunes on first use): rows of [nx, ny, nth_b,
-// cap, ns per candidate cap]; returns the number of degree classes
-int apply_tuning(rtg_handle* h, int32_t* out, int cap_rows, cudaStream_t s);
+// Autotuning table of a precision's apply (tunes on first use; rows as
+// rtg_apply_tuning lists them); returns the number of shapes
+int apply_tuning(rtg_handle* h, int prec, int32_t* out, int cap_rows, cudaStream_t s);
 // true when an apply in this precision ends with kernels on its own stream only
 // (no side stream joined): the kernel after it may be launched with launch_after()
 bool apply_chains(const rtg_handle* h, int prec);
 int apply_shape(rtg_handle* h, int prec, const int32_t* shape);
+void apply_digits(rtg_handle* h, int rows);
 
 // Sweep preconditioner (rtg_sweep.cu): z = P^{-1} r
 template <typename T>
