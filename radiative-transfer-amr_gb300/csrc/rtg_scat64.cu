@@ -17,12 +17,10 @@
 // an FP64 sum.  The epilogue adds the eight integers in 64 bits.
 //
 // Drop rule (rt/preconditioner_matrix.py:450-495): a node of class 2 keeps the
-// terms with |W| >= t.  Where all nodes of a CTA drop all of a block of 16 rows
-// and 16 angular nodes, the block's digits are cleared before they are
-// multiplied.  The dropped terms of the other blocks are in the product; they
-// are summed by the CUDA cores while the tensor cores run and subtracted: each
-// is below 1e-14 / |cw|, and their sum, in FP32 over 8 terms and in pairs of FP32
-// beyond, is off by about 2^-26 of itself.  The test |W| < t runs on FP32
+// terms with |W| >= t.  The nodes of a CTA share one threshold (a column has few:
+// the four or eight nodes of a symmetric rule share theirs), and the digits of
+// the dropped entries are cleared in shared memory before they are multiplied, so
+// a dropped term is left out exactly.  The test |W| < t runs on FP32
 // copies; the thresholds are moved at set-up to where the rounded test decides
 // as the exact one.  Nodes for which none does (two W entries of one FP32 value
 // on both sides of t), nodes with a non-finite x and nodes with max |x| outside
@@ -52,15 +50,13 @@ constexpr int kOzN = 32;         // nodes of a CTA, at most
 constexpr int kOzK = 16;         // angular nodes per stage: one tcgen05.mma step
 constexpr int kOzD = 8;          // digits
 constexpr int kOzMaxNth = 256;   // angular nodes a column may have (bound of the FP32 sums)
-constexpr int kDigBytes = kOzD * kOzK * 2;            // digits of a row of W per stage
-constexpr int kRowBytes = kDigBytes + kOzK * 4;       // and its FP32 copy
+constexpr int kRowBytes = kOzD * kOzK * 2;            // digits of a row of W per stage
 constexpr int kABytes = kOzM * kRowBytes;
 constexpr int kBBytes = kOzD * kOzN * kOzK * 2;
-constexpr int kXfBytes = kOzK * kOzN * 4;
-constexpr int kOzSmem = 2 * (kABytes + kBBytes + kXfBytes) + kOzMaxNth * (int)sizeof(int2);
+constexpr int kOzSmem = 2 * (kABytes + kBBytes) + kOzMaxNth * (int)sizeof(int2);
 
 struct OzItem {
-    int32_t col, row0, rows, n0, nn, drops;   // drops: a node of class 2;  rows row0 .. row0 + rows - 1, nodes perm[n0] .. perm[n0 + nn - 1]
+    int32_t col, row0, rows, n0, nn;        // rows row0 .. row0 + rows - 1, nodes perm[n0] .. perm[n0 + nn - 1] of one threshold
     int64_t tile;                           // first byte of the row tile's digits of W
     int64_t wrange;                         // first of the row tile's |W| ranges (per stage, eight groups of 16 rows)
 };
@@ -119,13 +115,6 @@ __device__ __forceinline__ double oz_times_pow2(double v, int e) {
     return (hi << 1) ? __hiloint2double(hi + (e << 20), __double2loint(v)) : v;
 }
 
-// 16 f as a double, for f zero or normal (integer work alone)
-__device__ __forceinline__ double oz_widen16(float f) {
-    const uint32_t b = __float_as_uint(f);
-    const uint32_t hi = (b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (900u << 20));
-    return (b << 1) >= 0x01000000u ? __hiloint2double((int)hi, (int)(b << 29)) : 0.;
-}
-
 // 2^e as a double, -1022 <= e <= 1023
 __host__ __device__ __forceinline__ double oz_pow2(int e) {
     const unsigned long long b = (unsigned long long)(e + 1023) << 52;
@@ -138,26 +127,6 @@ __host__ __device__ __forceinline__ double oz_pow2(int e) {
 #endif
 }
 
-// acc += (w0, w1) * x, two FP32 fused multiply-adds
-__device__ __forceinline__ void fma2(unsigned long long& acc, float w0, float w1, unsigned long long x) {
-    asm("{\n\t.reg .b64 w;\n\tmov.b64 w, {%1, %2};\n\tfma.rn.f32x2 %0, w, %3, %0;\n\t}"
-        : "+l"(acc)
-        : "f"(w0), "f"(w1), "l"(x));
-}
-
-// hi + lo += t (two sums side by side): the rounding error of hi + t goes to lo,
-// exactly where |hi| >= |t|
-__device__ __forceinline__ void add_pair(unsigned long long& hi, unsigned long long& lo, unsigned long long t) {
-    asm("{\n\t.reg .b64 s, z, e, m;\n\tmov.b64 m, {%3, %3};\n\t"
-        "add.rn.f32x2 s, %0, %2;\n\t"
-        "fma.rn.f32x2 z, %0, m, s;\n\t"      // z = s - hi
-        "fma.rn.f32x2 e, z, m, %2;\n\t"      // e = t - z
-        "add.rn.f32x2 %1, %1, e;\n\t"
-        "mov.b64 %0, s;\n\t}"
-        : "+l"(hi), "+l"(lo)
-        : "l"(t), "f"(-1.f));
-}
-
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -165,21 +134,20 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  : "memory");
 }
 
-// Warps 0-7 stage x, sum the corrections and write y; warp 8 brings the digits
-// of W in, one stage ahead, and issues the multiplies.
+// Warps 0-7 stage x, clear the dropped entries of W and write y; warp 8 brings
+// the digits of W in, one stage ahead, and issues the multiplies.
 __global__ void __launch_bounds__(kOzThreads + 32, 2)
 scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items,
-              const unsigned char* __restrict__ digits, const int* __restrict__ frow,
+              const unsigned char* __restrict__ digits, const float4* __restrict__ w32, const int* __restrict__ frow,
               const int64_t* __restrict__ sig_row, const float2* __restrict__ wrange,
               const uint8_t* __restrict__ perm, const uint64_t* __restrict__ thr, const float* __restrict__ thr32,
               const double* __restrict__ x, double* __restrict__ y, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char osm[];
     __shared__ __align__(8) uint64_t s_bar[6];   // W arrived 0, 1; multiplied 0, 1; x staged 0, 1
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort, s_tmax, s_tmin, s_bad, s_need;
+    __shared__ int s_abort, s_bad, s_need;
     __shared__ unsigned s_max[kOzN];
     __shared__ int s_E[kOzN];          // exponent field of the node's largest |x|; 0: node not in the product
-    __shared__ float s_thr[kOzN];
     __shared__ float2 s_wr[kOzMaxNth / kOzK][8];   // range of |W| per stage and 16 rows
     __shared__ int s_node[kOzN];       // node in the column
     __shared__ double s_g[kOzN];       // -cw 2^(E - 1056); 0: nothing to add
@@ -194,25 +162,23 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     const int nch = (Nth + kOzK - 1) / kOzK;
     unsigned char* As = osm;
     unsigned char* Bs = As + 2 * kABytes;
-    float* Xf = reinterpret_cast<float*>(Bs + 2 * kBBytes);   // [2][kOzK][kOzN]
-    float* Cf = reinterpret_cast<float*>(As);                 // after the product: the corrections [2][kOzN][kOzM]
     // per angular row: DOF offset in the column; nth and, from bit 8, the inflow-boundary faces of its cell
-    int2* s_row = reinterpret_cast<int2*>(Xf + 2 * kOzK * kOzN);
+    int2* s_row = reinterpret_cast<int2*>(Bs + 2 * kBBytes);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
     const unsigned char* wsrc = digits + it.tile;
-    // a stage's image: the digits of the rows, then (read where terms are dropped) FP32 W [kOzK][rows8]
-    const uint32_t stage = (uint32_t)rows8 * kRowBytes, dig = (uint32_t)rows8 * kDigBytes;
+    const uint32_t stage = (uint32_t)rows8 * kRowBytes;   // bytes of a stage: the digits of the rows
+    const float4* w32t = w32 + it.tile / kRowBytes * (kOzK / 4);   // their FP32 copies, per stage [kOzK / 4][rows8]
     const uint32_t as_addr = (uint32_t)__cvta_generic_to_shared(As);
-    // node tid's constants (loaded before they are needed)
-    float t_node = 0.f;
+    // the CTA's threshold (0: nothing is dropped; NaN: term by term)
+    const float thr_cta = thr32[C.node_off + perm[it.n0]];
+    // node tid's constant (loaded before it is needed)
     double cw = 0.;
-    float lo = 3.4e38f;   // smallest |W| of stage tid - 32
+    float lo = INFINITY;   // smallest |W| of stage tid - 32
     if (tid < kOzN) {
         s_max[tid] = 0u;
         const int ij = perm[it.n0 + min(tid, it.nn - 1)];   // the pad nodes repeat the last (their x is zero)
         s_node[tid] = ij;
-        t_node = thr32[C.node_off + ij];
         cw = v.colc[it.col] * v.sw[C.node_off + ij];
     } else if (tid - 32 < nch) {
         for (int q = 0; q < 8; ++q) {
@@ -234,8 +200,6 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     if ((v.stop && *v.stop) || (v.skip && v.skip[it.col])) return;
     if (tid == 0) {
         s_abort = 0;
-        s_tmax = 0;
-        s_tmin = 0x7F7FFFFF;
         s_bad = 0;
         s_need = 0;
         for (int q = 0; q < 6; ++q)
@@ -244,9 +208,8 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // the first stages' digits travel while the tables are made
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const uint32_t bytes = it.drops ? stage : dig;
-        bulk_load(as_addr, wsrc, bytes, bar);
-        if (nch > 1) bulk_load(as_addr + kABytes, wsrc + stage, bytes, bar + 8);
+        bulk_load(as_addr, wsrc, stage, bar);
+        if (nch > 1) bulk_load(as_addr + kABytes, wsrc + stage, stage, bar + 8);
     }
     if (warp == 8) {
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s_tmem);
@@ -258,6 +221,8 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
+    // the stages in which some |W| is dropped
+    if (lo < thr_cta) atomicOr(&s_need, 1 << (tid - 32));
     // per node the largest |x| (a lane takes a node)
     const double* xc = x + C.dof_off;
     for (int k = warp; k < ncell; k += kOzThreads / 32 + 1) {
@@ -278,37 +243,22 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     if (tid < kOzN) {
         int E = 0;
         double g = 0.;
-        float t = t_node;
         if (tid < it.nn) {
             const unsigned mx = s_max[tid];
             const int e = (int)(mx >> 20);
-            if (e < 100 || e > 2000 || t != t) {
+            if (e < 100 || e > 2000 || thr_cta != thr_cta) {
                 g = mx ? -cw : 0.;          // summed term by term below, or x is zero
                 if (mx) s_bad = 1;
-                if (mx || t != t) t = 0.f;
             } else {
                 E = e;
                 g = -cw * oz_pow2(e - 1056);
-                atomicMax(&s_tmax, __float_as_int(t));
-                atomicMin(&s_tmin, __float_as_int(t));
             }
         }
         s_E[tid] = E;
         s_g[tid] = g;
-        s_thr[tid] = t;
     }
     __syncthreads();
-    // largest and smallest threshold of the CTA's nodes (0: nothing is dropped)
-    const float tmax = __int_as_float(s_tmax), tmin = __int_as_float(s_tmin);
-    if (tmax > 0.f) {
-        // the stages in which some |W| may be dropped
-        if (lo < tmax) atomicOr(&s_need, 1 << (tid - 32));
-        __syncthreads();
-    }
     const int needs = s_need;
-    // correction tile of the thread: rows 16 warp + 4 (lane % 4) .., nodes 4 (lane / 4) ..
-    // (two nodes side by side; the sum is corr + cerr)
-    unsigned long long corr[4][2] = {}, cerr[4][2] = {};
     bool ok = true;
     if (warp == 8) {
         // kind::f16: D F32 (bits 4-5 = 1), A and B FP16 (bits 7-9, 10-12 = 0), K-major, N >> 3 at bit 17, M >> 4 at 24
@@ -335,8 +285,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                 if (ch >= 1 && ch + 1 < nch) {
                     ok = mbar_wait(bar + 16 + 8 * (b ^ 1), (uint32_t)(((ch - 1) >> 1) & 1));
                     if (ok)
-                        bulk_load(as_addr + (b ^ 1) * kABytes, wsrc + (int64_t)(ch + 1) * stage,
-                                  needs >> (ch + 1) & 1 ? stage : dig, bar + 8 * (b ^ 1));
+                        bulk_load(as_addr + (b ^ 1) * kABytes, wsrc + (int64_t)(ch + 1) * stage, stage, bar + 8 * (b ^ 1));
                 }
             }
             if (!ok) s_abort = 1;
@@ -353,18 +302,20 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
             return xc[ro.x + ijn * (ro.y & 0xFF)];
         };
         const uint32_t boff = (uint32_t)((nb >> 3) * 256 + (kp >> 3) * 128 + (nb & 7) * 16 + (kp & 7) * 2);
-        float th[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) th[j] = s_thr[4 * (lane >> 2) + j];
-        // nodes are in the order of their thresholds, of which a column has few (four nodes
-        // of a symmetric rule share one): one test for the four nodes of every thread
-        const bool same = __all_sync(0xffffffffu, th[0] == th[1] && th[0] == th[2] && th[0] == th[3]);
+        // thread -> (row mr, eight angular nodes from 8 mh) of the entries it may clear
+        const int mr = tid & (kOzM - 1), mh = tid >> 7;
+        float4 wa{}, wb{};
+        auto load_w = [&](int ch) {
+            if (mr >= rows8 || ch >= nch || !(needs >> ch & 1)) return;
+            const float4* p = w32t + ((int64_t)ch * (kOzK / 4) + 2 * mh) * rows8 + mr;
+            wa = p[0];
+            wb = p[rows8];
+        };
+        load_w(0);
         double x0 = load_x(kp), x1 = load_x(kp + 1);
         for (int ch = 0; ch < nch; ++ch) {
             const int b = ch & 1, c0 = ch * kOzK;
             unsigned char* Bb = Bs + b * kBBytes;
-            float* Xb = Xf + b * kOzK * kOzN;
-            const bool need = needs >> ch & 1;
             // stage ch - 2 has been multiplied: its buffers are free
             if (ch >= 2 && !mbar_wait(bar + 16 + 8 * b, (uint32_t)(((ch >> 1) - 1) & 1))) {
                 s_abort = 1;
@@ -378,21 +329,27 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                 for (int j = 0; j < kOzD; ++j)
                     *reinterpret_cast<uint32_t*>(Bb + boff + j * np * 32) =
                         j < 4 ? oz_pair(h0, h1, 3 - j) : oz_pair(l0, l1, 7 - j);
-                if (need) {
-                    // x in units of 2^(E - 1052) for the corrections
-                    Xb[kp * kOzN + nb] = (float)(int)(q0 >> 32);
-                    Xb[(kp + 1) * kOzN + nb] = (float)(int)(q1 >> 32);
-                }
             }
-            // a block of which every node drops every term is taken out of the product
-            const float2 wr = s_wr[ch][warp];   // smallest and largest |W| of the warp's 16 rows
-            if (need && 16 * warp < rows8 && wr.y < tmin) {
+            if (needs >> ch & 1) {
+                // the digits of the dropped entries: cleared once they are there
                 ok = mbar_wait(bar + 8 * b, (uint32_t)((ch >> 1) & 1)) && ok;
-                if (16 * lane < min(512, rows8 * 32 - 512 * warp))
+                if (mr < rows8 && s_wr[ch][mr >> 4].x < thr_cta) {
+                    auto kept = [&](float a, float c) {
+                        return (fabsf(a) >= thr_cta ? 0xFFFFu : 0u) | (fabsf(c) >= thr_cta ? 0xFFFF0000u : 0u);
+                    };
+                    const uint4 k4 = make_uint4(kept(wa.x, wa.y), kept(wa.z, wa.w), kept(wb.x, wb.y), kept(wb.z, wb.w));
+                    unsigned char* p = As + b * kABytes + (mr >> 3) * 256 + mh * 128 + (mr & 7) * 16;
 #pragma unroll
-                    for (int k = 0; k < kOzD; ++k)
-                        *reinterpret_cast<uint4*>(As + b * kABytes + k * rows8 * 32 + 512 * warp + 16 * lane) =
-                            make_uint4(0u, 0u, 0u, 0u);
+                    for (int k = 0; k < kOzD; ++k) {
+                        uint4* q = reinterpret_cast<uint4*>(p + k * rows8 * 32);
+                        uint4 d = *q;
+                        d.x &= k4.x;
+                        d.y &= k4.y;
+                        d.z &= k4.z;
+                        d.w &= k4.w;
+                        *q = d;
+                    }
+                }
             }
             // generic-proxy writes -> visible to the tensor cores
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -401,51 +358,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar + 32 + 8 * b) : "memory");
             x0 = load_x(c0 + kOzK + kp);
             x1 = load_x(c0 + kOzK + kp + 1);
-            if (needs == 0) continue;
-            // every warp has staged x (and is done with the stage before)
-            const uint32_t par = (uint32_t)((ch >> 1) & 1);
-            ok = mbar_wait(bar + 32 + 8 * b, par) && ok;
-            if (!need || 16 * warp >= it.rows) continue;
-            if (wr.x >= tmax || wr.y < tmin) continue;
-            ok = mbar_wait(bar + 8 * b, par) && ok;
-            const float* wp = reinterpret_cast<const float*>(As + b * kABytes + dig) + 16 * warp + 4 * (lane & 3);
-            const float* xp = Xb + 4 * (lane >> 2);
-#pragma unroll
-            for (int c8 = 0; c8 < kOzK; c8 += 8) {
-                unsigned long long part[4][2] = {};
-                if (same) {
-#pragma unroll 4
-                    for (int c = c8; c < c8 + 8; ++c) {
-                        const float4 w4 = *reinterpret_cast<const float4*>(wp + c * rows8);
-                        const ulonglong2 x4 = *reinterpret_cast<const ulonglong2*>(xp + c * kOzN);
-                        const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float w = fabsf(wv[i]) < th[0] ? wv[i] : 0.f;
-                            fma2(part[i][0], w, w, x4.x);
-                            fma2(part[i][1], w, w, x4.y);
-                        }
-                    }
-                } else {
-#pragma unroll 2
-                    for (int c = c8; c < c8 + 8; ++c) {
-                        const float4 w4 = *reinterpret_cast<const float4*>(wp + c * rows8);
-                        const ulonglong2 x4 = *reinterpret_cast<const ulonglong2*>(xp + c * kOzN);
-                        const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float a = fabsf(wv[i]);
-                            fma2(part[i][0], a < th[0] ? wv[i] : 0.f, a < th[1] ? wv[i] : 0.f, x4.x);
-                            fma2(part[i][1], a < th[2] ? wv[i] : 0.f, a < th[3] ? wv[i] : 0.f, x4.y);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    add_pair(corr[i][0], cerr[i][0], part[i][0]);
-                    add_pair(corr[i][1], cerr[i][1], part[i][1]);
-                }
-            }
+            load_w(ch + 1);
         }
         if (!ok) s_abort = 1;
     }
@@ -461,22 +374,6 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         }
         if (tid == 0 && status) atomicExch(status, RTG_ERR_TIMEOUT);
     } else {
-        // corrections to [node][row] (the buffers are free)
-        if (needs && warp < 8) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float* o = Cf + (4 * (lane >> 2) + j) * kOzM + 16 * warp + 4 * (lane & 3);
-                float hi[4], lo[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    hi[i] = __uint_as_float((uint32_t)(corr[i][j >> 1] >> (32 * (j & 1))));
-                    lo[i] = __uint_as_float((uint32_t)(cerr[i][j >> 1] >> (32 * (j & 1))));
-                }
-                *reinterpret_cast<float4*>(o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<float4*>(o + kOzN * kOzM) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-            }
-        }
-        __syncthreads();
         const int q = warp & 3, h = warp >> 2;
         const int m = 32 * q + lane, R = it.row0 + m;
         const bool valid = warp < 8 && m < it.rows;
@@ -512,8 +409,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                     H = (H << 8) + __float2int_rn(__uint_as_float(d[k][jj]));
                     L = (L << 8) + __float2int_rn(__uint_as_float(d[k + 4][jj]));
                 }
-                double s = oz_times_pow2(oz_double(H, L), fr);
-                if (needs) s -= oz_widen16(Cf[n * kOzM + m]) + oz_widen16(Cf[(kOzN + n) * kOzM + m]);
+                const double s = oz_times_pow2(oz_double(H, L), fr);
                 atomicAdd(yc + ij * nth, s * s_g[n]);
             }
         }
@@ -545,14 +441,15 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
 }
 
 // One block per row of a distinct W: its digits into the row tile's image (per
-// stage of kOzK columns: digit, 8-row group, 8-column group, row, column), its
+// stage of kOzK columns: digit, 8-row group, 8-column group, row, column), its FP32
+// copy (per stage four columns of every row together), its
 // scale, and the range of the nonzero off-diagonal |W| per stage and 16 rows.  bad: an entry is not
 // finite, or the row's largest is outside [2^-100, 2^100].
 __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __restrict__ W32,
                                  const int64_t* __restrict__ W_off, const int2* __restrict__ rows,
                                  const int64_t* __restrict__ sig_tile, const int64_t* __restrict__ sig_wrange,
                                  const int32_t* __restrict__ sig_n, unsigned char* __restrict__ out,
-                                 int* __restrict__ frow, float2* __restrict__ wrange, int* __restrict__ bad) {
+                                 float* __restrict__ out32, int* __restrict__ frow, float2* __restrict__ wrange, int* __restrict__ bad) {
     __shared__ unsigned long long s_mx[4];
     const int sg = rows[blockIdx.x].x, R = rows[blockIdx.x].y, n = sig_n[sg];
     const double* w = W + W_off[sg] + (int64_t)R * n;
@@ -572,7 +469,9 @@ __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __re
     if (!ok || !mx) return;   // the digits stay zero
     const int mt = R / kOzM, rr = R % kOzM, nch = (n + kOzK - 1) / kOzK;
     const int rows8 = (min(kOzM, n - mt * kOzM) + 7) & ~7;
-    unsigned char* tile = out + sig_tile[sg] + (int64_t)mt * nch * kOzM * kRowBytes;
+    const int64_t at = sig_tile[sg] + (int64_t)mt * nch * kOzM * kRowBytes;
+    unsigned char* tile = out + at;
+    float* tile32 = out32 + at / kRowBytes * kOzK;
     for (int c = threadIdx.x; c < n; c += blockDim.x) {
         if (c == R) continue;
         const unsigned long long u = oz_digits(oz_fixed(w[c], E));
@@ -582,7 +481,7 @@ __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __re
             *reinterpret_cast<uint16_t*>(p + k * rows8 * kOzK * 2) =
                 (uint16_t)oz_pair(k < 4 ? (uint32_t)(u >> 32) : (uint32_t)u, 0u, 3 - (k & 3));
         const float w32 = W32[W_off[sg] + (int64_t)R * n + c];
-        reinterpret_cast<float*>(st + rows8 * kDigBytes)[(c % kOzK) * rows8 + rr] = w32;
+        tile32[((int64_t)(c / 4) * rows8 + rr) * 4 + (c & 3)] = w32;
         const float a = fabsf(w32);
         if (a > 0.f) {
             float2* wr = wrange + sig_wrange[sg] + 8 * ((int64_t)mt * nch + c / kOzK) + (rr >> 4);
@@ -620,6 +519,7 @@ struct Scat64 {
     OzItem* d_items = nullptr;
     int nitems = 0;
     unsigned char* d_digits = nullptr;
+    float* d_w32 = nullptr;
     int* d_frow = nullptr;   // per row: exponent of its scale
     int64_t* d_sig_row = nullptr;
     float2* d_wrange = nullptr;
@@ -662,42 +562,28 @@ Scat64* build_scat64(const rtg_handle* h, const std::vector<char>& cols, const u
         if (!cols[ci]) continue;
         const ColDev& C = t.cols[ci];
         const int nij = C.nx * C.ny, nch = (C.nth_col + kOzK - 1) / kOzK;
-        // the nodes whose product is used, by threshold, those of thresholds
-        // shared by 4, 8, .. nodes first: the kernel tests four nodes at once
+        // the nodes whose product is used, by threshold; a CTA takes nodes of one
         std::vector<uint8_t> ord;
-        std::map<float, int> share;
-        auto thr_f = [&](int q) {
-            double t;
-            std::memcpy(&t, &thr[C.node_off + q], 8);
-            return (float)t;
-        };
         for (int q = 0; q < nij; ++q) {
             const uint8_t cls = scls[C.node_off + q];
-            if (cls == 1 || cls == 2) {
-                ord.push_back((uint8_t)q);
-                ++share[thr_f(q)];
-            }
+            if (cls == 1 || cls == 2) ord.push_back((uint8_t)q);
             if (cls == 2) nodes.push_back(make_int2(C.node_off + q, C.sig));
         }
-        std::stable_sort(ord.begin(), ord.end(), [&](uint8_t a, uint8_t b) {
-            const float ta = thr_f(a), tb = thr_f(b);
-            const bool ra = share[ta] % 4 != 0, rb = share[tb] % 4 != 0;
-            return ra != rb ? rb : ta < tb;
-        });
-        const int na = (int)ord.size(), ntl = (na + kOzN - 1) / kOzN;
-        const int per = ntl ? ((na + ntl - 1) / ntl + 3) & ~3 : 4, p0 = (int)perm.size();
+        std::stable_sort(ord.begin(), ord.end(),
+                         [&](uint8_t a, uint8_t b) { return thr[C.node_off + a] < thr[C.node_off + b]; });
+        const int na = (int)ord.size(), p0 = (int)perm.size();
         perm.insert(perm.end(), ord.begin(), ord.end());
-        for (int n0 = 0; n0 < na; n0 += per) {
-            const int nn = std::min(per, na - n0);
-            int drops = 0;
-            for (int q = n0; q < n0 + nn; ++q) drops |= scls[C.node_off + ord[q]] == 2;
-            for (int r0 = 0; r0 < C.nth_col; r0 += kOzM) {
-                const int mt = r0 / kOzM;
-                items.push_back(OzItem{ci, r0, std::min(kOzM, C.nth_col - r0), p0 + n0, nn, drops,
-                                       sig_tile[C.sig] + (int64_t)mt * nch * kOzM * kRowBytes,
-                                       sig_wrange[C.sig] + 8 * (int64_t)mt * nch});
-                cost[C.sig] += (int64_t)nch * kOzM;
-            }
+        for (int g0 = 0, g1; g0 < na; g0 = g1) {
+            for (g1 = g0; g1 < na && thr[C.node_off + ord[g1]] == thr[C.node_off + ord[g0]];) ++g1;
+            const int ntl = (g1 - g0 + kOzN - 1) / kOzN, per = (g1 - g0 + ntl - 1) / ntl;
+            for (int n0 = g0; n0 < g1; n0 += per)
+                for (int r0 = 0; r0 < C.nth_col; r0 += kOzM) {
+                    const int mt = r0 / kOzM;
+                    items.push_back(OzItem{ci, r0, std::min(kOzM, C.nth_col - r0), p0 + n0, std::min(per, g1 - n0),
+                                           sig_tile[C.sig] + (int64_t)mt * nch * kOzM * kRowBytes,
+                                           sig_wrange[C.sig] + 8 * (int64_t)mt * nch});
+                    cost[C.sig] += (int64_t)nch * kOzM;
+                }
         }
     }
     // the CTAs that read one row tile run next to each other, so that its
@@ -724,6 +610,7 @@ Scat64* build_scat64(const rtg_handle* h, const std::vector<char>& cols, const u
         p->nitems = (int)items.size();
         p->d_items = (OzItem*)up(items.data(), sizeof(OzItem) * items.size());
         p->d_digits = (unsigned char*)alloc((size_t)bytes);
+        p->d_w32 = (float*)alloc((size_t)bytes / kRowBytes * kOzK * sizeof(float));
         p->d_frow = (int*)alloc(sizeof(int) * rows.size());
         p->d_sig_row = (int64_t*)up(sig_row.data(), sizeof(int64_t) * nsig);
         p->d_wrange = (float2*)alloc(sizeof(float2) * (size_t)nw);
@@ -740,12 +627,13 @@ Scat64* build_scat64(const rtg_handle* h, const std::vector<char>& cols, const u
         RTG_CUDA(cudaMemset(p->d_status, 0, sizeof(int)));
         RTG_CUDA(cudaMemset(d_bad, 0, sizeof(int)));
         RTG_CUDA(cudaMemset(p->d_digits, 0, (size_t)bytes));
+        RTG_CUDA(cudaMemset(p->d_w32, 0, (size_t)bytes / kRowBytes * kOzK * sizeof(float)));
         const std::vector<float2> none((size_t)nw, make_float2(3.4e38f, 0.f));
         RTG_CUDA(cudaMemcpy(p->d_wrange, none.data(), sizeof(float2) * (size_t)nw, cudaMemcpyHostToDevice));
         RTG_CUDA(cudaMemset(p->d_thr32, 0, sizeof(float) * (size_t)t.nnodes));
         if (!rows.empty()) {
             oz_digits_kernel<<<(int)rows.size(), 128>>>(h->v64.W, h->v32.W, h->v64.W_off, d_rows, d_st, d_sw, d_n,
-                                                        p->d_digits, p->d_frow, p->d_wrange, d_bad), count_launch();
+                                                        p->d_digits, p->d_w32, p->d_frow, p->d_wrange, d_bad), count_launch();
             RTG_LAUNCHED("oz_digits_kernel");
         }
         if (!nodes.empty()) {
@@ -776,7 +664,8 @@ void free_scat64(Scat64* p) {
 void launch_scat64(const Scat64* p, const OpView<double>& v, uint32_t flags, const double* x,
                    double* y, cudaStream_t s) {
     if (!p->nitems) return;
-    launch_after(scat64_kernel, p->nitems, kOzThreads + 32, kOzSmem, s, v, flags, p->d_items, p->d_digits, p->d_frow,
+    launch_after(scat64_kernel, p->nitems, kOzThreads + 32, kOzSmem, s, v, flags, p->d_items, p->d_digits,
+                 reinterpret_cast<const float4*>(p->d_w32), p->d_frow,
                  p->d_sig_row, p->d_wrange, p->d_perm, p->d_thr, p->d_thr32, x, y, p->d_status);
 }
 

@@ -74,6 +74,30 @@ def test_pinned_product(name):
         assert float(torch.linalg.norm(a - r)) <= 1e-14 * size
 
 
+@pytest.mark.parametrize("name", ["nth147_n6", "nth129_n7", "nth17", "nth40"])
+def test_dropped_terms_are_left_out(name):
+    """A beam (one angular node of x) in columns whose terms are dropped or kept by their size: where the FP64 pipe
+    drops all of an output's terms, the sum is exactly zero."""
+    import torch
+    from rtg import DeviceContext, _lib, workloads as W
+    ctx = _ctx(name) if name in CASES else small_ctx(name)
+    spec = W.two_disc_problem()
+    # sigma falls by 10 from strip to strip of columns, so that the drop rule cuts at every level of the kernel
+    thin = DeviceContext(ctx.layout.mesh, spec.kappa, lambda x, y: 10. ** (-2. - np.floor(4. * x)) + 0. * y, spec.Phi)
+    lay = thin.layout
+    x = torch.zeros(thin.N, dtype=torch.float64, device=thin.device)
+    rng = np.random.default_rng(0)
+    for c in range(lay.ncols):
+        e = int(rng.integers(lay.col_elem_start[c], lay.col_elem_start[c + 1]))
+        nth = int(lay.cell_ndof[e])
+        o = np.arange(int(lay.elem_off[e]) + int(rng.integers(nth)), int(lay.elem_off[e + 1]), nth)
+        x[torch.as_tensor(o)] = torch.as_tensor(rng.uniform(0.5, 2., size=len(o)), device=thin.device)
+    a, r = both(thin, _lib.RTG_SCAT, x)
+    assert (r == 0).any() and (r != 0).any()
+    assert bool((a[r == 0] == 0).all())
+    assert bool((a[r != 0] != 0).all())
+
+
 def test_tuned_table():
     """The autotuned FP64 table: one row chosen, the fastest, and the digits among the shapes of a product of 1e8."""
     from rtg import _lib
