@@ -3,18 +3,27 @@
 // Y[R][ij] = sum_c W[R][c] x[c][ij] over a column's angular nodes is the dense
 // contraction of the FP64 apply, and GB300 runs FP64 at 2 FMAs per SM and
 // clock: on the FP64 pipe the product took 3.3 of the 4.07 ms of an apply at
-// 7.95e6 DOF.  Here every operand is a sum of eight signed 8-bit digits (the
+// 7.95e6 DOF.  Here every operand is a sum of ten signed 8-bit digits (the
 // splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012, with
 // fixed-point digits): a row of W and a node's line of x are scaled by the
-// power of two of their largest entry to 62-bit fixed point, whose balanced
-// digits d_1 .. d_8 (|d_1| <= 64, |d_k| <= 128) are exact in FP16.  A digit
-// product is an integer below 2^14, and D_s = sum over i + j = s of W_i x_j, s =
-// 2 .. 9, accumulates in FP32 in tensor memory without rounding: with at most
-// 256 angular nodes |D_s| <= 2^24 for s <= 6, and D_7 .. D_9 (whose bound is
-// 2^24.8, reached by no sum of random digits) stand 2^40 and more below D_2.
-// The terms left out (s >= 10, and W and x below 2^-62 of their row's or node's
-// largest entry) are below 2^-58 of |W|_max |x|_max, finer than the rounding of
-// an FP64 sum.  The epilogue adds the eight integers in 64 bits.
+// power of two of their largest entry to 78-bit fixed point, whose balanced
+// digits d_1 .. d_10 (|d_1| <= 64, |d_k| <= 128) are exact in FP16.  A digit
+// product is an integer of at most 2^14, and D_s = sum over i + j = s of W_i x_j,
+// s = 2 .. 11, accumulates in FP32 in tensor memory, without rounding for s <= 9:
+// set-up checks on the digits of W that |D_s| <= 2^24 for every x (random digits
+// of 292 angular nodes reach it; a column has at most 256).  D_10 and D_11 stand
+// 2^64 and more below D_2.  The epilogue adds the ten integers in 80 bits and rounds
+// once: T in units of 2^-82 to 2^-84 of |W|_max |x|_max.
+//
+// What is left out (s >= 12, and W and x below 2^-78 of their largest entry) is
+// at most 700 of these units a term, 2^17.5 for 256.  Against the FP64 sum of a row
+// that is small only where the sum is not itself small beside |W|_max |x|_max: so an
+// output with |T| < 2^70 (below about 2^-12 of it: one in a few thousand for
+// random x; most outputs far from a beam) is summed again, term by term in FP64, by a
+// warp.  Every other output is within 2^-52 of the sum of its terms, as an
+// FP64 sum of so many terms is not.  With eight digits and no second sum the apply
+// at 7.95e6 DOF takes 1286 us in place of 1437, but a beam's terms were off by 1e-13 of
+// their size for the g = 0.95 kernel and 3e-7 for exp(20 (cos - 1)).
 //
 // Drop rule (rt/preconditioner_matrix.py:450-495): a node of class 2 keeps the
 // terms with |W| >= t.  The nodes of a CTA share one threshold (a column has few:
@@ -24,14 +33,14 @@
 // copies; the thresholds are moved at set-up to where the rounded test decides
 // as the exact one.  Nodes for which none does (two W entries of one FP32 value
 // on both sides of t), nodes with a non-finite x and nodes with max |x| outside
-// [2^-923, 2^977] are summed term by term in FP64.
+// [2^-823, 2^977] are summed term by term in the same way.
 //
-// One CTA takes up to 128 rows and 32 nodes of a column: 8 accumulators of 32
+// One CTA takes up to 128 rows and 24 nodes of a column: 10 accumulators of 24
 // columns fill half of the tensor memory, so two CTAs share an SM and one
 // stages while the other multiplies.  B holds the digits of x stacked along N
-// (row 32 (j - 1) + n), so that one tcgen05.mma multiplies W_i with x_1 ..
-// x_{9-i} into D_{i+1} .. D_9, which lie next to each other: 8 instructions per 16
-// angular nodes in place of 36.
+// (row np (j - 1) + n, np the nodes rounded up to 8), so that one tcgen05.mma
+// multiplies W_i with x_1 .. x_{11-i} into D_{i+1} .. D_11, which lie next to each
+// other: 10 instructions per 16 angular nodes in place of 55.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -46,9 +55,10 @@ namespace {
 
 constexpr int kOzThreads = 256;
 constexpr int kOzM = 128;        // rows of a CTA (TMEM lanes)
-constexpr int kOzN = 32;         // nodes of a CTA, at most
+constexpr int kOzN = 24;         // nodes of a CTA, at most
 constexpr int kOzK = 16;         // angular nodes per stage: one tcgen05.mma step
-constexpr int kOzD = 8;          // digits
+constexpr int kOzD = 10;         // digits
+constexpr long long kOzSmall = 1ll << 30;   // |T| below 2^40 of these: summed again
 constexpr int kOzMaxNth = 256;   // angular nodes a column may have (bound of the FP32 sums)
 constexpr int kRowBytes = kOzD * kOzK * 2;            // digits of a row of W per stage
 constexpr int kABytes = kOzM * kRowBytes;
@@ -73,21 +83,32 @@ __device__ __forceinline__ void oz_mma(uint32_t d, uint64_t a, uint64_t b, uint3
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
 
-// Q with v = Q 2^(E - 1084), |Q| < 2^62, for |v| < 2^(E - 1022), E >= 1 (bits below 2^(E - 1084) cut off)
-__device__ __forceinline__ long long oz_fixed(double v, int E) {
+// The ten balanced digits of Q, v = Q 2^(E - 1100), |Q| < 2^78, for |v| < 2^(E - 1022),
+// E >= 1 (bits below 2^(E - 1100) cut off), each plus 128: d_1 .. d_8 in the bytes of u,
+// d_1 on top, d_9 and d_10 in the lower two of w
+struct OzDigits {
+    unsigned long long u;
+    uint32_t w;
+};
+__device__ __forceinline__ OzDigits oz_digits(double v, int E) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
     int e = (int)(b >> 52) & 0x7FF;
     unsigned long long m = b & 0xFFFFFFFFFFFFFull;
     if (e) m |= 1ull << 52;
     else e = 1;
-    const int sh = E - e;
-    const unsigned long long q = sh < 63 ? (m << 9) >> sh : 0ull;
-    return (long long)b < 0 ? -(long long)q : (long long)q;
-}
-
-// the eight balanced digits of Q, each plus 128, in the bytes of the result (d_1 on top)
-__device__ __forceinline__ unsigned long long oz_digits(long long q) {
-    return ((unsigned long long)q + 0x0080808080808080ull) ^ 0x8000000000000000ull;
+    m <<= 9;
+    const int sh = E - e;   // Q = m 2^16 >> sh, in 62 and 16 bits
+    long long hi = sh < 63 ? (long long)(m >> sh) : 0ll;
+    int lo = (int)(sh < 16 ? m << (16 - sh) : sh < 79 ? m >> (sh - 16) : 0ull) & 0xFFFF;
+    if ((long long)b < 0) {
+        hi = -hi;
+        lo = -lo;
+    }
+    const int w = lo + 0x8080;   // the carry into d_8 above 16 bits
+    OzDigits d;
+    d.u = ((unsigned long long)(hi + (w >> 16)) + 0x0080808080808080ull) ^ 0x8000000000000000ull;
+    d.w = (uint32_t)w & 0xFFFFu;
+    return d;
 }
 
 // digits k (bytes k of u and w) as FP16, exactly: 1024 + byte - 1152
@@ -97,16 +118,20 @@ __device__ __forceinline__ uint32_t oz_pair(uint32_t u, uint32_t w, int k) {
     asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(b), "r"(0x64806480u));
     return d;
 }
+// digit j + 1 of both
+__device__ __forceinline__ uint32_t oz_pair(const OzDigits& a, const OzDigits& b, int j) {
+    return j < 4   ? oz_pair((uint32_t)(a.u >> 32), (uint32_t)(b.u >> 32), 3 - j)
+           : j < 8 ? oz_pair((uint32_t)a.u, (uint32_t)b.u, 7 - j)
+                   : oz_pair(a.w, b.w, 9 - j);
+}
 
-// H 2^32 + L rounded once, for |H| < 2^46 and |L| < 2^50, with two FP64 operations
+// hi 2^40 + lo rounded once, for |hi| < 2^58 and 0 <= lo < 2^40, with two FP64 operations
 // (the pipe takes 16 cycles for each of a warp's): its upper and lower parts
-// are put into the mantissas of 3 2^91 (one unit 2^40) and of 2^52 (one unit 1)
-__device__ __forceinline__ double oz_double(long long H, long long L) {
-    const long long t = ((H & 0xFF) << 32) + L;                  // H 2^32 + L = (H >> 8) 2^40 + t
-    const long long hi = (H >> 8) + (t >> 40), lo = t & 0xFFFFFFFFFFll;
-    const double a = __longlong_as_double(0x45B8000000000000ll + hi);
-    const double b = __longlong_as_double(0x4330000000000000ll | lo);
-    return (a - (0x1.8p92 + 0x1p52)) + b;
+// are put into the mantissas of 3 2^99 (one unit 2^48) and of 2^52 (one unit 1)
+__device__ __forceinline__ double oz_double(long long hi, long long lo) {
+    const double a = __longlong_as_double(0x4638000000000000ll + (hi >> 8));
+    const double b = __longlong_as_double(0x4330000000000000ll | ((hi & 0xFF) << 40) | lo);
+    return (a - (0x1.8p100 + 0x1p52)) + b;
 }
 
 // v 2^e for v zero or normal, with v 2^e normal (integer work alone)
@@ -145,19 +170,21 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     extern __shared__ __align__(128) unsigned char osm[];
     __shared__ __align__(8) uint64_t s_bar[6];   // W arrived 0, 1; multiplied 0, 1; x staged 0, 1
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort, s_bad, s_need;
+    __shared__ int s_abort, s_need, s_nlist;
+    __shared__ uint8_t s_any[kOzM];    // row keeps a term
     __shared__ unsigned s_max[kOzN];
     __shared__ int s_E[kOzN];          // exponent field of the node's largest |x|; 0: node not in the product
     __shared__ float2 s_wr[kOzMaxNth / kOzK][8];   // range of |W| per stage and 16 rows
     __shared__ int s_node[kOzN];       // node in the column
-    __shared__ double s_g[kOzN];       // -cw 2^(E - 1056); 0: nothing to add
+    __shared__ double s_g[kOzN];       // -cw 2^(E - 1064); 0: nothing to add
+    __shared__ double s_cw[kOzN];      // -cw
     after_trigger();
     const OzItem it = items[blockIdx.x];
     const ColDev C = v.cols[it.col];
     const bool mask_rows = flags & RTG_MASK_ROWS;
     const int nij = C.nx * C.ny, Nth = C.nth_col, ncell = C.elem_end - C.elem_begin;
     const int np = (it.nn + 7) & ~7;
-    const int tcols = np <= 16 ? 128 : 256;
+    const int tcols = np <= 8 ? 128 : 256;
     const int rows8 = (it.rows + 7) & ~7;
     const int nch = (Nth + kOzK - 1) / kOzK;
     unsigned char* As = osm;
@@ -180,7 +207,8 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         const int ij = perm[it.n0 + min(tid, it.nn - 1)];   // the pad nodes repeat the last (their x is zero)
         s_node[tid] = ij;
         cw = v.colc[it.col] * v.sw[C.node_off + ij];
-    } else if (tid - 32 < nch) {
+        s_cw[tid] = -cw;
+    } else if (tid >= 32 && tid - 32 < nch) {
         for (int q = 0; q < 8; ++q) {
             const float2 w = wrange[it.wrange + 8 * (tid - 32) + q];
             s_wr[tid - 32][q] = w;
@@ -200,8 +228,8 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     if ((v.stop && *v.stop) || (v.skip && v.skip[it.col])) return;
     if (tid == 0) {
         s_abort = 0;
-        s_bad = 0;
         s_need = 0;
+        s_nlist = 0;
         for (int q = 0; q < 6; ++q)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8 * q), "r"(q < 4 ? 1 : kOzThreads / 32)
                          : "memory");
@@ -223,6 +251,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     const uint32_t tmem = s_tmem;
     // the stages in which some |W| is dropped
     if (lo < thr_cta) atomicOr(&s_need, 1 << (tid - 32));
+    if (tid < kOzM) s_any[tid] = 0;
     // per node the largest |x| (a lane takes a node)
     const double* xc = x + C.dof_off;
     for (int k = warp; k < ncell; k += kOzThreads / 32 + 1) {
@@ -246,12 +275,11 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         if (tid < it.nn) {
             const unsigned mx = s_max[tid];
             const int e = (int)(mx >> 20);
-            if (e < 100 || e > 2000 || thr_cta != thr_cta) {
+            if (e < 200 || e > 2000 || thr_cta != thr_cta) {
                 g = mx ? -cw : 0.;          // summed term by term below, or x is zero
-                if (mx) s_bad = 1;
             } else {
                 E = e;
-                g = -cw * oz_pow2(e - 1056);
+                g = -cw * oz_pow2(e - 1064);
             }
         }
         s_E[tid] = E;
@@ -274,7 +302,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                 const uint64_t db = oz_desc((uint32_t)__cvta_generic_to_shared(Bs + b * kBBytes));
 #pragma unroll
                 for (int i = 0; i < kOzD; ++i) {
-                    const uint32_t n = (uint32_t)(((kOzD - i) * np + 15) & ~15);   // columns past D_9 are not read
+                    const uint32_t n = (uint32_t)(((kOzD - i) * np + 15) & ~15);   // columns past D_11 are not read
                     oz_mma(tmem + (uint32_t)(i * np), oz_desc(aa + (uint32_t)(i * rows8 * 32)), db,
                            idesc0 | ((n >> 3) << 17), ch > 0 || i > 0);
                 }
@@ -292,10 +320,10 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         }
         __syncwarp();
     } else {
-        // thread -> (two angular nodes, one node): eight digits of each into B
+        // thread -> (two angular nodes, one node): ten digits of each into B
         const int kp = 8 * (warp & 1) + 2 * (lane & 3), nb = 8 * (warp >> 1) + (lane >> 2);
         const bool bact = nb < np;
-        const int En = bact ? s_E[nb] : 0, ijn = s_node[nb & (kOzN - 1)];
+        const int En = bact ? s_E[nb] : 0, ijn = s_node[min(nb, kOzN - 1)];
         auto load_x = [&](int c) -> double {
             if (!En || c >= Nth) return 0.;
             const int2 ro = s_row[c];
@@ -305,6 +333,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         // thread -> (row mr, eight angular nodes from 8 mh) of the entries it may clear
         const int mr = tid & (kOzM - 1), mh = tid >> 7;
         float4 wa{}, wb{};
+        bool any = false;   // the row keeps one of them
         auto load_w = [&](int ch) {
             if (mr >= rows8 || ch >= nch || !(needs >> ch & 1)) return;
             const float4* p = w32t + ((int64_t)ch * (kOzK / 4) + 2 * mh) * rows8 + mr;
@@ -322,13 +351,10 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                 ok = false;
             }
             if (bact) {
-                const long long q0 = En ? oz_fixed(x0, En) : 0ll, q1 = En ? oz_fixed(x1, En) : 0ll;
-                const unsigned long long u0 = oz_digits(q0), u1 = oz_digits(q1);
-                const uint32_t h0 = (uint32_t)(u0 >> 32), l0 = (uint32_t)u0, h1 = (uint32_t)(u1 >> 32), l1 = (uint32_t)u1;
+                const OzDigits d0 = oz_digits(x0, max(En, 1)), d1 = oz_digits(x1, max(En, 1));   // x is zero where En is
 #pragma unroll
                 for (int j = 0; j < kOzD; ++j)
-                    *reinterpret_cast<uint32_t*>(Bb + boff + j * np * 32) =
-                        j < 4 ? oz_pair(h0, h1, 3 - j) : oz_pair(l0, l1, 7 - j);
+                    *reinterpret_cast<uint32_t*>(Bb + boff + j * np * 32) = oz_pair(d0, d1, j);
             }
             if (needs >> ch & 1) {
                 // the digits of the dropped entries: cleared once they are there
@@ -338,6 +364,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                         return (fabsf(a) >= thr_cta ? 0xFFFFu : 0u) | (fabsf(c) >= thr_cta ? 0xFFFF0000u : 0u);
                     };
                     const uint4 k4 = make_uint4(kept(wa.x, wa.y), kept(wa.z, wa.w), kept(wb.x, wb.y), kept(wb.z, wb.w));
+                    any |= (k4.x | k4.y | k4.z | k4.w) != 0u;
                     unsigned char* p = As + b * kABytes + (mr >> 3) * 256 + mh * 128 + (mr & 7) * 16;
 #pragma unroll
                     for (int k = 0; k < kOzD; ++k) {
@@ -349,7 +376,11 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                         d.w &= k4.w;
                         *q = d;
                     }
+                } else {
+                    any = true;
                 }
+            } else {
+                any = true;
             }
             // generic-proxy writes -> visible to the tensor cores
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -360,6 +391,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
             x1 = load_x(c0 + kOzK + kp + 1);
             load_w(ch + 1);
         }
+        if (any) s_any[mr] = 1;
         if (!ok) s_abort = 1;
     }
     // the last commit follows every multiply of the CTA
@@ -386,7 +418,10 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
             const int i = small_div(ij, rny);
             return bm && bdry_node(bm, i, ij - i * C.ny, C.nx, C.ny);
         };
-        double* yc = y + C.dof_off + ro.x;
+        double* yc = y + C.dof_off;
+        // outputs to be summed again, row + 256 node (the buffers are free)
+        uint16_t* s_list = reinterpret_cast<uint16_t*>(As);
+        auto again = [&](int n) { s_list[atomicAdd(&s_nlist, 1)] = (uint16_t)(m | n << 8); };
         for (int cb = 4 * h; cb < np && warp < 8; cb += 8) {
             uint32_t d[kOzD][4];
 #pragma unroll
@@ -400,36 +435,44 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj) {
                 const int n = cb + jj;
-                if (n >= it.nn || !s_E[n]) continue;
+                if (n >= it.nn || s_g[n] == 0.) continue;
                 const int ij = s_node[n];
                 if (masked(ij)) continue;
+                if (!s_E[n]) {
+                    again(n);
+                    continue;
+                }
                 long long H = 0, L = 0;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
+                for (int k = 0; k < 5; ++k) {
                     H = (H << 8) + __float2int_rn(__uint_as_float(d[k][jj]));
-                    L = (L << 8) + __float2int_rn(__uint_as_float(d[k + 4][jj]));
+                    L = (L << 8) + __float2int_rn(__uint_as_float(d[k + 5][jj]));
                 }
-                const double s = oz_times_pow2(oz_double(H, L), fr);
-                atomicAdd(yc + ij * nth, s * s_g[n]);
+                H += L >> 40;
+                if (H > -kOzSmall && H < kOzSmall) {
+                    if (s_any[m]) again(n);   // else every term is dropped
+                    continue;
+                }
+                const double s = oz_times_pow2(oz_double(H, L & 0xFFFFFFFFFFll), fr);
+                atomicAdd(yc + ro.x + ij * nth, s * s_g[n]);
             }
         }
-        if (s_bad && valid && h == 0) {
-            // nodes left out of the product: kept terms one by one (the bits of |W| against the threshold)
-            const double* Wr = v.W + v.W_off[C.sig] + (int64_t)R * Nth;
-            for (int n = 0; n < it.nn; ++n) {
-                if (s_E[n] || s_g[n] == 0.) continue;
-                const int ij = s_node[n];
-                if (masked(ij)) continue;
-                const unsigned long long tb = thr[C.node_off + ij];
-                double s = 0.;
-                for (int c = 0; c < Nth; ++c) {
-                    const unsigned long long wb = (unsigned long long)__double_as_longlong(Wr[c]);
-                    const bool keep = c != R && (wb & 0x7FFFFFFFFFFFFFFFull) >= tb;
-                    const int2 rc = s_row[c];
-                    s = fma(keep ? Wr[c] : 0., xc[rc.x + ij * (rc.y & 0xFF)], s);
-                }
-                atomicAdd(yc + ij * nth, s * s_g[n]);
+        __syncthreads();
+        // a warp per output: the kept terms one by one (the bits of |W| against the threshold)
+        for (int i = warp; i < s_nlist; i += kOzThreads / 32 + 1) {
+            const int n = s_list[i] >> 8, Ra = it.row0 + (s_list[i] & 0xFF), ij = s_node[n];
+            const double* Wr = v.W + v.W_off[C.sig] + (int64_t)Ra * Nth;
+            const unsigned long long tb = thr[C.node_off + ij];
+            double s = 0.;
+            for (int c = lane; c < Nth; c += 32) {
+                const double w = Wr[c];
+                const bool keep = c != Ra && ((unsigned long long)__double_as_longlong(w) & 0x7FFFFFFFFFFFFFFFull) >= tb;
+                const int2 rc = s_row[c];
+                s = fma(keep ? w : 0., xc[rc.x + ij * (rc.y & 0xFF)], s);
             }
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            const int2 ra = s_row[Ra];
+            if (lane == 0) atomicAdd(yc + ra.x + ij * (ra.y & 0xFF), s * s_cw[n]);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -444,13 +487,14 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
 // stage of kOzK columns: digit, 8-row group, 8-column group, row, column), its FP32
 // copy (per stage four columns of every row together), its
 // scale, and the range of the nonzero off-diagonal |W| per stage and 16 rows.  bad: an entry is not
-// finite, or the row's largest is outside [2^-100, 2^100].
+// finite, the row's largest is outside [2^-100, 2^100], or the digits allow an x whose D_2 .. D_9 pass 2^24.
 __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __restrict__ W32,
                                  const int64_t* __restrict__ W_off, const int2* __restrict__ rows,
                                  const int64_t* __restrict__ sig_tile, const int64_t* __restrict__ sig_wrange,
                                  const int32_t* __restrict__ sig_n, unsigned char* __restrict__ out,
                                  float* __restrict__ out32, int* __restrict__ frow, float2* __restrict__ wrange, int* __restrict__ bad) {
     __shared__ unsigned long long s_mx[4];
+    __shared__ int s_sum[kOzD];   // sum of the |d_i|
     const int sg = rows[blockIdx.x].x, R = rows[blockIdx.x].y, n = sig_n[sg];
     const double* w = W + W_off[sg] + (int64_t)R * n;
     unsigned long long mx = 0;
@@ -458,13 +502,14 @@ __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __re
         if (c != R) mx = max(mx, (unsigned long long)__double_as_longlong(w[c]) & 0x7FFFFFFFFFFFFFFFull);
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0) s_mx[threadIdx.x >> 5] = mx;
+    if (threadIdx.x < kOzD) s_sum[threadIdx.x] = 0;
     __syncthreads();
     for (int q = 0; q < (int)blockDim.x / 32; ++q) mx = max(mx, s_mx[q]);
     const int E = (int)(mx >> 52);
     const bool ok = mx == 0 || (E >= 923 && E <= 1123);
     if (threadIdx.x == 0) {
         if (!ok) atomicExch(bad, 1);
-        frow[blockIdx.x] = ok && mx ? E - 1056 : 0;
+        frow[blockIdx.x] = ok && mx ? E - 1064 : 0;
     }
     if (!ok || !mx) return;   // the digits stay zero
     const int mt = R / kOzM, rr = R % kOzM, nch = (n + kOzK - 1) / kOzK;
@@ -474,12 +519,15 @@ __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __re
     float* tile32 = out32 + at / kRowBytes * kOzK;
     for (int c = threadIdx.x; c < n; c += blockDim.x) {
         if (c == R) continue;
-        const unsigned long long u = oz_digits(oz_fixed(w[c], E));
+        const OzDigits u = oz_digits(w[c], E);
         unsigned char* st = tile + (int64_t)(c / kOzK) * rows8 * kRowBytes;
         unsigned char* p = st + (rr >> 3) * 256 + ((c % kOzK) >> 3) * 128 + (rr & 7) * 16 + (c & 7) * 2;
-        for (int k = 0; k < kOzD; ++k)
-            *reinterpret_cast<uint16_t*>(p + k * rows8 * kOzK * 2) =
-                (uint16_t)oz_pair(k < 4 ? (uint32_t)(u >> 32) : (uint32_t)u, 0u, 3 - (k & 3));
+#pragma unroll
+        for (int k = 0; k < kOzD; ++k) {
+            *reinterpret_cast<uint16_t*>(p + k * rows8 * kOzK * 2) = (uint16_t)oz_pair(u, u, k);
+            const int byte = (int)(k < 8 ? u.u >> (8 * (7 - k)) : u.w >> (8 * (9 - k))) & 0xFF;
+            atomicAdd(&s_sum[k], abs(byte - 128));
+        }
         const float w32 = W32[W_off[sg] + (int64_t)R * n + c];
         tile32[((int64_t)(c / 4) * rows8 + rr) * 4 + (c & 3)] = w32;
         const float a = fabsf(w32);
@@ -488,6 +536,12 @@ __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __re
             atomicMin(reinterpret_cast<int*>(&wr->x), __float_as_int(a));
             atomicMax(reinterpret_cast<int*>(&wr->y), __float_as_int(a));
         }
+    }
+    __syncthreads();
+    if (threadIdx.x >= 2 && threadIdx.x <= 9) {
+        int most = 0;   // of |D_s|, s = threadIdx.x
+        for (int i = 1; i < (int)threadIdx.x; ++i) most += s_sum[i - 1] * (i == (int)threadIdx.x - 1 ? 64 : 128);
+        if (most > 1 << 24) atomicExch(bad, 1);
     }
 }
 

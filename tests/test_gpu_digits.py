@@ -98,6 +98,41 @@ def test_dropped_terms_are_left_out(name):
     assert bool((a[r != 0] != 0).all())
 
 
+def _forward(th, phi):
+    """A forward cone: falls by 2^57 across the circle."""
+    return 3.14 * np.exp(20. * (np.cos(th - phi) - 1.))
+
+
+@pytest.mark.parametrize("peaked", [False, True])
+@pytest.mark.parametrize("name", ["nth256_n4", "nth147_n6", "nth160_n9", "nth17", "nth40"])
+def test_every_output_against_its_own_terms(name, peaked):
+    """Each output is within the rounding of an FP64 sum of its own terms, also where these are small beside the row's
+    largest |W| times the node's largest |x|: a beam alone, over a floor of 1e-30, values spread over many decades.
+    Both sums obey Nth 2^-53 of the sum of the terms' sizes, so twice that between them."""
+    import torch
+    from rtg import DeviceContext, _lib, workloads as W
+    ctx = _ctx(name) if name in CASES else small_ctx(name)
+    if peaked:
+        spec = W.two_disc_problem()
+        ctx = DeviceContext(ctx.layout.mesh, spec.kappa, spec.sigma, _forward)
+    lay = ctx.layout
+    nth = int(lay.cell_ndof[:lay.col_elem_start[1]].sum())
+    rng = np.random.default_rng(1)
+    beam = np.zeros(ctx.N)
+    for c in range(lay.ncols):
+        e = int(rng.integers(lay.col_elem_start[c], lay.col_elem_start[c + 1]))
+        o = np.arange(int(lay.elem_off[e]) + int(rng.integers(lay.cell_ndof[e])), int(lay.elem_off[e + 1]), int(lay.cell_ndof[e]))
+        beam[o] = rng.uniform(0.5, 2., size=len(o))
+    noise = rng.standard_normal(ctx.N)
+    xs = [torch.as_tensor(x, device=ctx.device) for x in (beam, beam + 1e-30 * noise, noise * np.exp(12. * rng.standard_normal(ctx.N)), noise)]
+    pin(ctx, False)
+    ref = [(ctx.apply(_lib.RTG_SCAT, x), ctx.apply(_lib.RTG_SCAT, x.abs()).abs()) for x in xs]
+    pin(ctx, True)
+    for x, (r, size) in zip(xs, ref):
+        a = ctx.apply(_lib.RTG_SCAT, x)
+        assert float(((a - r).abs() - 2. * nth * 2. ** -53 * size).max()) <= 0.
+
+
 def test_tuned_table():
     """The autotuned FP64 table: one row chosen, the fastest, and the digits among the shapes of a product of 1e8."""
     from rtg import _lib
