@@ -9,20 +9,24 @@
 // power of two of their largest entry to 78-bit fixed point, whose balanced
 // digits d_1 .. d_10 (|d_1| <= 64, |d_k| <= 128) are exact in FP16.  A digit
 // product is an integer of at most 2^14, and D_s = sum over i + j = s of W_i x_j,
-// s = 2 .. 11, accumulates in FP32 in tensor memory, without rounding for s <= 9:
+// s = 2 .. 11, accumulates in FP32 in tensor memory, without rounding for s <= 10:
 // set-up checks on the digits of W that |D_s| <= 2^24 for every x (random digits
-// of 292 angular nodes reach it; a column has at most 256).  D_10 and D_11 stand
-// 2^64 and more below D_2.  The epilogue adds the ten integers in 80 bits and rounds
-// once: T in units of 2^-82 to 2^-84 of |W|_max |x|_max.
+// of 270 angular nodes reach it; a column has at most 256).  The epilogue adds the
+// ten integers in 80 bits and rounds once: T in units of 2^-82 to 2^-84 of
+// |W|_max |x|_max.
 //
 // What is left out (s >= 12, and W and x below 2^-78 of their largest entry) is
-// at most 700 of these units a term, 2^17.5 for 256.  Against the FP64 sum of a row
-// that is small only where the sum is not itself small beside |W|_max |x|_max: so an
-// output with |T| < 2^70 (below about 2^-12 of it: one in a few thousand for
-// random x; most outputs far from a beam) is summed again, term by term in FP64, by a
-// warp.  Every other output is within 2^-52 of the sum of its terms, as an
-// FP64 sum of so many terms is not.  With eight digits and no second sum the apply
-// at 7.95e6 DOF takes 1286 us in place of 1437, but a beam's terms were off by 1e-13 of
+// at most 578 + 128 of these units for every x that is not zero in fixed point, and
+// D_11, if it passes 2^24, is off by at most 2 a multiply, 320.  Against the FP64 sum
+// of a row that is small only where the sum is not itself small beside |W|_max
+// |x|_max: so an output below 2^52 times that (kOzLost, kOzRound; 2^-12 of the
+// largest product at 256 nonzero x) is summed again, term by term in FP64: one in a
+// few thousand outputs for random x.  The apply at 7.95e6 DOF takes 1456 us for
+// random x, 1787 for a solution, 2309 for a beam in every column, 3353 for
+// randn exp(12 randn), 4234 on the FP64 pipe.
+// Every other output is within 2^-52 of the sum of its terms, as an FP64 sum of so
+// many terms is not.  With eight digits and no second sum the apply
+// at 7.95e6 DOF takes 1286 us, but a beam's terms were off by 1e-13 of
 // their size for the g = 0.95 kernel and 3e-7 for exp(20 (cos - 1)).
 //
 // Drop rule (rt/preconditioner_matrix.py:450-495): a node of class 2 keeps the
@@ -58,7 +62,7 @@ constexpr int kOzM = 128;        // rows of a CTA (TMEM lanes)
 constexpr int kOzN = 24;         // nodes of a CTA, at most
 constexpr int kOzK = 16;         // angular nodes per stage: one tcgen05.mma step
 constexpr int kOzD = 10;         // digits
-constexpr long long kOzSmall = 1ll << 30;   // |T| below 2^40 of these: summed again
+constexpr int kOzLost = 710, kOzRound = 512;   // what an x, and the sum, may be off by (units of T)
 constexpr int kOzMaxNth = 256;   // angular nodes a column may have (bound of the FP32 sums)
 constexpr int kRowBytes = kOzD * kOzK * 2;            // digits of a row of W per stage
 constexpr int kABytes = kOzM * kRowBytes;
@@ -89,6 +93,7 @@ __device__ __forceinline__ void oz_mma(uint32_t d, uint64_t a, uint64_t b, uint3
 struct OzDigits {
     unsigned long long u;
     uint32_t w;
+    __device__ bool zero() const { return u == 0x8080808080808080ull && w == 0x8080u; }
 };
 __device__ __forceinline__ OzDigits oz_digits(double v, int E) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -178,6 +183,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     __shared__ int s_node[kOzN];       // node in the column
     __shared__ double s_g[kOzN];       // -cw 2^(E - 1064); 0: nothing to add
     __shared__ double s_cw[kOzN];      // -cw
+    __shared__ int s_nz[kOzN];         // x that are not zero in fixed point
     after_trigger();
     const OzItem it = items[blockIdx.x];
     const ColDev C = v.cols[it.col];
@@ -208,6 +214,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         s_node[tid] = ij;
         cw = v.colc[it.col] * v.sw[C.node_off + ij];
         s_cw[tid] = -cw;
+        s_nz[tid] = 0;
     } else if (tid >= 32 && tid - 32 < nch) {
         for (int q = 0; q < 8; ++q) {
             const float2 w = wrange[it.wrange + 8 * (tid - 32) + q];
@@ -342,6 +349,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         };
         load_w(0);
         double x0 = load_x(kp), x1 = load_x(kp + 1);
+        int nz = 0;
         for (int ch = 0; ch < nch; ++ch) {
             const int b = ch & 1, c0 = ch * kOzK;
             unsigned char* Bb = Bs + b * kBBytes;
@@ -352,6 +360,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
             }
             if (bact) {
                 const OzDigits d0 = oz_digits(x0, max(En, 1)), d1 = oz_digits(x1, max(En, 1));   // x is zero where En is
+                nz += !d0.zero() + !d1.zero();
 #pragma unroll
                 for (int j = 0; j < kOzD; ++j)
                     *reinterpret_cast<uint32_t*>(Bb + boff + j * np * 32) = oz_pair(d0, d1, j);
@@ -392,6 +401,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
             load_w(ch + 1);
         }
         if (any) s_any[mr] = 1;
+        if (nz) atomicAdd(&s_nz[nb], nz);
         if (!ok) s_abort = 1;
     }
     // the last commit follows every multiply of the CTA
@@ -449,7 +459,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                     L = (L << 8) + __float2int_rn(__uint_as_float(d[k + 5][jj]));
                 }
                 H += L >> 40;
-                if (H > -kOzSmall && H < kOzSmall) {
+                if (llabs(H) < (long long)(kOzLost * s_nz[n] + kOzRound) << 12) {   // units of 2^40: |T| below 2^52 times that
                     if (s_any[m]) again(n);   // else every term is dropped
                     continue;
                 }
@@ -458,21 +468,26 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
             }
         }
         __syncthreads();
-        // a warp per output: the kept terms one by one (the bits of |W| against the threshold)
-        for (int i = warp; i < s_nlist; i += kOzThreads / 32 + 1) {
-            const int n = s_list[i] >> 8, Ra = it.row0 + (s_list[i] & 0xFF), ij = s_node[n];
+        // eight lanes per output: the kept terms one by one (the bits of |W| against the
+        // threshold).  A warp per output spends half of its FP64 operations on the sum of the
+        // lanes' parts (randn exp(12 randn) at 7.95e6 DOF: 5537 us in place of 3353)
+        const int lane8 = lane & 7;
+        for (int i0 = 4 * warp; i0 < s_nlist; i0 += 4 * (kOzThreads / 32 + 1)) {
+            const int i = i0 + (lane >> 3);
+            const int at = s_list[min(i, s_nlist - 1)], n = at >> 8, Ra = it.row0 + (at & 0xFF), ij = s_node[n];
             const double* Wr = v.W + v.W_off[C.sig] + (int64_t)Ra * Nth;
             const unsigned long long tb = thr[C.node_off + ij];
             double s = 0.;
-            for (int c = lane; c < Nth; c += 32) {
+#pragma unroll 4
+            for (int c = lane8; c < Nth; c += 8) {
                 const double w = Wr[c];
                 const bool keep = c != Ra && ((unsigned long long)__double_as_longlong(w) & 0x7FFFFFFFFFFFFFFFull) >= tb;
                 const int2 rc = s_row[c];
                 s = fma(keep ? w : 0., xc[rc.x + ij * (rc.y & 0xFF)], s);
             }
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             const int2 ra = s_row[Ra];
-            if (lane == 0) atomicAdd(yc + ra.x + ij * (ra.y & 0xFF), s * s_cw[n]);
+            if (lane8 == 0 && i < s_nlist) atomicAdd(yc + ra.x + ij * (ra.y & 0xFF), s * s_cw[n]);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -487,7 +502,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
 // stage of kOzK columns: digit, 8-row group, 8-column group, row, column), its FP32
 // copy (per stage four columns of every row together), its
 // scale, and the range of the nonzero off-diagonal |W| per stage and 16 rows.  bad: an entry is not
-// finite, the row's largest is outside [2^-100, 2^100], or the digits allow an x whose D_2 .. D_9 pass 2^24.
+// finite, the row's largest is outside [2^-100, 2^100], or the digits allow an x whose D_2 .. D_10 pass 2^24.
 __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __restrict__ W32,
                                  const int64_t* __restrict__ W_off, const int2* __restrict__ rows,
                                  const int64_t* __restrict__ sig_tile, const int64_t* __restrict__ sig_wrange,
@@ -538,7 +553,7 @@ __global__ void oz_digits_kernel(const double* __restrict__ W, const float* __re
         }
     }
     __syncthreads();
-    if (threadIdx.x >= 2 && threadIdx.x <= 9) {
+    if (threadIdx.x >= 2 && threadIdx.x <= 10) {
         int most = 0;   // of |D_s|, s = threadIdx.x
         for (int i = 1; i < (int)threadIdx.x; ++i) most += s_sum[i - 1] * (i == (int)threadIdx.x - 1 ? 64 : 128);
         if (most > 1 << 24) atomicExch(bad, 1);
