@@ -198,7 +198,7 @@ int rtg_apply(rtg_handle* h, uint32_t flags, int prec, const void* x, void* y,
  * product on the tensor cores, the scattering CTAs of one angular mesh next to
  * each other.  FP64: one CTA per work item of 4 to 64 rows, and from 4e6
  * multiply-adds in the product 16 to 64 rows with the product on the tensor
- * cores, these alone from 1e8) is built and the whole apply timed; the fastest
+ * cores, beside one of the former from 1e8, or all where it wins) is built and the whole apply timed; the fastest
  * is kept.  This returns the FP32 table (host, cap_rows rows of 9 int32: rows
  * per item, items per CTA (0: the whole column), split launches (0/1),
  * tensor-core scattering (0: none; 1: scattering CTAs heaviest first; 2:

@@ -2050,12 +2050,15 @@ static int plan_launches(const ApplyPlan* p) {
 }
 
 // Multiply-adds of the scattering product from which FP64 plans with the
-// tensor cores (rtg_scat64.cu; FP32 plans: more shapes, tune_plan) are timed beside those of the FP64 pipe, and from
-// which they alone are.  Whole applies, FP64 pipe against tensor cores, in us: 19.8
-// and 27.9 at 1.2e6 (33,056 DOF adaptive: an extra launch), 51.6 and 45.4 at 8.6e6
-// (218,581 DOF adaptive), 73 and 38 at 2.1e7, 459 and 103 at 1.6e8, 4067 and 920 at
-// 1.5e9 (7.95e6 DOF, two scatterers).
-constexpr int64_t kTcOffer = 4'000'000, kTc64Alone = 100'000'000;
+// tensor cores (rtg_scat64.cu; FP32 plans: more shapes, tune_plan) are timed beside
+// those of the FP64 pipe, and from which one of the latter stands for all of them
+// until it wins.  The product alone does not decide: a column's cost on the tensor
+// cores goes by its tiles of 128 rows and its thresholds.  Whole applies, FP64 pipe
+// against tensor cores, in us: 19.8 and 27.9 at 1.2e6 (33,056 DOF adaptive: an extra
+// launch), 51.6 and 47.2 at 8.6e6 (218,581 DOF adaptive), 4234 and 1456 at
+// 1.5e9 (7.95e6 DOF, two scatterers), 2435 and 559 at 1.1e9 (256 angles), but 502 and
+// 549 at 2.1e7 in 16,384 columns of 3 x 3 nodes and 12 angles (1.77e6 DOF).
+constexpr int64_t kTcOffer = 4'000'000, kTc64Large = 100'000'000;
 
 // where the tensor-core kernel of a plan reports a wait that gave up
 static int* plan_status(const ApplyPlan* p) { return p->par ? scat64_status(p->par->s64) : p->d_status; }
@@ -2157,20 +2160,22 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
         }
         if (f64 && all_fit && prod >= kTcOffer) make_digits(h, par);
         const bool tc64 = f64 && par->s64;
-        std::vector<PlanShape> shapes;
-        if (f64 && prod < kTc64Alone) {
+        std::vector<PlanShape> shapes, rest;   // rest: timed where a shape of the FP64 pipe is the best of the first
+        if (f64 && prod < kTc64Large) {
             // one CTA per item, down to a cell: a column per CTA leaves the FP64 pipes
             // of a small mesh's other SMs idle (84.6 against 51.6 us at 218,581 DOF)
             for (int rows : {4, 8, 16, 32, 64}) shapes.push_back(PlanShape{rows, 1, 0, 0});
-        } else if (!tc64) {
+        } else {
             // on larger meshes launches split by shared-memory class (none differed by 2 %
             // at 218,581 DOF and above) and a column of 16 or 32 rows per CTA (never the
             // best there) are left out
             for (int rows : {16, 32, 64})
                 for (int gcap : {0, 1})
                     for (int split : {0, 1})
-                        if (f64 || prod < kTcOffer || (!split && (gcap || rows == 64)))
-                            shapes.push_back(PlanShape{rows, gcap, split, 0});
+                        if (f64 || prod < kTcOffer || (!split && (gcap || rows == 64))) {
+                            const bool later = tc64 && (rows != 32 || gcap != 1 || split);
+                            (later ? rest : shapes).push_back(PlanShape{rows, gcap, split, 0});
+                        }
         }
         // tensor-core scattering, FP32, the scattering CTAs of one angular mesh next
         // to each other (their heaviest-first order is 1.7 % slower on the
@@ -2189,58 +2194,62 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
         }
         // FP64: one CTA per item (one per column leaves SMs idle at its end)
         if (tc64)
-            for (int rows : {16, 32, 64}) shapes.push_back(PlanShape{rows, 1, 0, 1});
+            for (int rows : {64, 32, 16}) shapes.insert(shapes.begin(), PlanShape{rows, 1, 0, 1});
         // the plans are built on host threads at once (host tables read only;
         // each thread makes its own uploads), then timed one by one
         int dev = 0;
         RTG_CUDA(cudaGetDevice(&dev));
-        std::vector<std::future<ApplyPlan*>> built;
-        for (const PlanShape& sh : shapes)
-            built.push_back(std::async(std::launch::async, [h, sh, par, dev]() {
-                RTG_CUDA(cudaSetDevice(dev));
-                return shape_plan<T>(h, sh, par);
-            }));
-        std::vector<ApplyPlan*> plans(shapes.size(), nullptr);
-        std::exception_ptr failed;
-        for (size_t q = 0; q < built.size(); ++q) {
-            try {
-                plans[q] = built[q].get();
-            } catch (...) {
-                if (!failed) failed = std::current_exception();
+        auto time_shapes = [&](const std::vector<PlanShape>& list) {
+            std::vector<std::future<ApplyPlan*>> built;
+            for (const PlanShape& sh : list)
+                built.push_back(std::async(std::launch::async, [h, sh, par, dev]() {
+                    RTG_CUDA(cudaSetDevice(dev));
+                    return shape_plan<T>(h, sh, par);
+                }));
+            std::vector<ApplyPlan*> plans(list.size(), nullptr);
+            std::exception_ptr failed;
+            for (size_t q = 0; q < built.size(); ++q) {
+                try {
+                    plans[q] = built[q].get();
+                } catch (...) {
+                    if (!failed) failed = std::current_exception();
+                }
             }
-        }
-        if (failed) {
-            for (ApplyPlan* p : plans) free_plan(p);
-            std::rethrow_exception(failed);
-        }
-        for (size_t q = 0; q < shapes.size(); ++q) {
-            const PlanShape& sh = shapes[q];
-            ApplyPlan* p = plans[q];
-            plans[q] = nullptr;
-            if (f64 && sh.tc && p->tiled != par->s64_cols) {   // not the columns of the digit tables
-                free_plan(p);
-                continue;
+            if (failed) {
+                for (ApplyPlan* p : plans) free_plan(p);
+                std::rethrow_exception(failed);
             }
-            TuneRecord r{sh, 0, -1, p->ntiles, p->tg_begin[kSmemClasses], plan_launches(p)};
-            float tt = 1e30f;
-            try {
-                tt = time_plan<T>(h, p, x, y, e0, e1, s, tbest);
-            } catch (...) {
-                free_plan(p);
-                for (ApplyPlan* rest : plans) free_plan(rest);
-                throw;
+            for (size_t q = 0; q < list.size(); ++q) {
+                const PlanShape& sh = list[q];
+                ApplyPlan* p = plans[q];
+                plans[q] = nullptr;
+                if (f64 && sh.tc && p->tiled != par->s64_cols) {   // not the columns of the digit tables
+                    free_plan(p);
+                    continue;
+                }
+                TuneRecord r{sh, 0, -1, p->ntiles, p->tg_begin[kSmemClasses], plan_launches(p)};
+                float tt = 1e30f;
+                try {
+                    tt = time_plan<T>(h, p, x, y, e0, e1, s, tbest);
+                } catch (...) {
+                    free_plan(p);
+                    for (ApplyPlan* rest : plans) free_plan(rest);
+                    throw;
+                }
+                r.ns = (int)std::min(tt * 1e6f, 2.e9f);
+                recs.push_back(r);
+                if (tt < tbest) {
+                    free_plan(best);
+                    best = p;
+                    tbest = tt;
+                    ibest = (int)recs.size() - 1;
+                } else {
+                    free_plan(p);
+                }
             }
-            r.ns = (int)std::min(tt * 1e6f, 2.e9f);
-            recs.push_back(r);
-            if (tt < tbest) {
-                free_plan(best);
-                best = p;
-                tbest = tt;
-                ibest = (int)recs.size() - 1;
-            } else {
-                free_plan(p);
-            }
-        }
+        };
+        time_shapes(shapes);
+        if (best && !best->tc) time_shapes(rest);
         if (!best) throw RtgError{RTG_ERR_ARG, "apply: no plan fits"};
     } catch (...) {
         free_plan(best);
@@ -2251,6 +2260,10 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
     release();
     recs[ibest].chosen = 1;
     best->own_par = f64;
+    if (f64 && !best->tc) {   // no plan reads the digits
+        free_scat64(par->s64);
+        par->s64 = nullptr;
+    }
     best->tuning = std::move(recs);
     return best;
 }

@@ -139,6 +139,22 @@ def test_tuned_table():
     t = plans(_ctx("nth128_n7"), _lib.RTG_FP64)
     assert int(t[:, 4].sum()) == 1 and t[t[:, 4] == 1][0][5] == t[:, 5].min()
     assert (t[:, 3] == 1).any()
+    assert (t[:, 3] == 0).any()                # the FP64 pipe is timed beside them
+
+
+def test_tuned_table_of_few_angles():
+    """4,096 columns of 3 x 3 nodes and 12 angles: the product is large, its tiles of 128 rows are not filled."""
+    from rtg import DeviceContext, _lib, workloads as W
+    from rtg.mesh import Mesh
+    m = Mesh([2., 2.], [False, False], [3, 3, 3], True)
+    for _ in range(2):
+        m.ref_mesh(kind="ang", form="h")
+    for _ in range(6):
+        m.ref_mesh(kind="spt", form="h")
+    spec = W.two_disc_problem()
+    t = plans(DeviceContext(m, spec.kappa, spec.sigma, spec.Phi), _lib.RTG_FP64)
+    assert (t[:, 3] == 1).any() and (t[:, 3] == 0).any()
+    assert t[t[:, 4] == 1][0][5] == t[:, 5].min()
 
 
 def test_refused():
