@@ -218,8 +218,8 @@ int rtg_apply_shape(rtg_handle* h, int prec, const int32_t* shape);
 int rtg_apply_plans(rtg_handle* h, int prec, int32_t* table, int cap_rows, int* nshapes, void* stream);
 /* As rtg_apply_shape with {rows, 1, 0, 0} in FP64, but with the scattering
  * product on the tensor cores.  RTG_ERR_SIZE, and the plan stays as it is, when
- * a column has more than 256 angular nodes or the digits cannot hold a
- * scattering matrix. */
+ * a column has more than 256 angular nodes, the digits cannot hold a
+ * scattering matrix, or there is no device memory for them. */
 int rtg_apply_digits(rtg_handle* h, int rows);
 /* mask[N] (device, uint8): 1 for unknowns, 0 for inflow-boundary DOFs. */
 int rtg_interior_mask(rtg_handle* h, uint8_t* mask, void* stream);

@@ -2125,9 +2125,10 @@ static void make_digits(rtg_handle* h, ParityTables* par) {
 // Autotuner of the apply: every plan shape of the candidate list (rows per
 // item 4 to 64, one CTA per column or per item, one launch or one per
 // shared-memory class, with or without the tensor-core scattering) is built
-// and the whole apply timed; the fastest plan is kept.
+// and the whole apply timed; the fastest plan is kept.  digits false: no FP64 plans
+// with the tensor cores.
 template <typename T>
-static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
+static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s, bool digits = true) {
     constexpr bool f64 = sizeof(T) == 8;
     const int64_t N = h->host.ndof;
     T *x = nullptr, *y = nullptr;
@@ -2158,7 +2159,7 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
             prod += (int64_t)C.nx * C.ny * C.nth_col * C.nth_col;
             all_fit &= scat64_fits(C);
         }
-        if (f64 && all_fit && prod >= kTcOffer) make_digits(h, par);
+        if (f64 && digits && all_fit && prod >= kTcOffer) make_digits(h, par);
         const bool tc64 = f64 && par->s64;
         std::vector<PlanShape> shapes, rest;   // rest: timed where a shape of the FP64 pipe is the best of the first
         if (f64 && prod < kTc64Large) {
@@ -2252,10 +2253,19 @@ static ApplyPlan* tune_plan(rtg_handle* h, cudaStream_t s) {
         if (best && !best->tc) time_shapes(rest);
         if (!best) throw RtgError{RTG_ERR_ARG, "apply: no plan fits"};
     } catch (...) {
+        const bool held = f64 && par->s64;
         free_plan(best);
         if (par) free_parity(par);
         release();
-        throw;
+        if (!held) throw;
+        try {
+            throw;
+        } catch (const RtgError& e) {
+            if (e.msg.find(cudaGetErrorString(cudaErrorMemoryAllocation)) == std::string::npos) throw;
+        }
+        // the digit tables may have taken the room that the plans need
+        cudaGetLastError();
+        return tune_plan<T>(h, s, false);
     }
     release();
     recs[ibest].chosen = 1;

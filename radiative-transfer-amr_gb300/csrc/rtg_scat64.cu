@@ -663,11 +663,14 @@ Scat64* build_scat64(const rtg_handle* h, const std::vector<char>& cols, const u
         if (sa != sb) return sa < sb;
         return a.row0 < b.row0;
     });
+    struct NoRoom {};
     Scat64* p = new Scat64();
     try {
         auto alloc = [&](size_t n) -> void* {
             void* d = nullptr;
-            RTG_CUDA(cudaMalloc(&d, std::max<size_t>(n, 16)));
+            const cudaError_t e = cudaMalloc(&d, std::max<size_t>(n, 16));
+            if (e == cudaErrorMemoryAllocation) throw NoRoom{};
+            RTG_CUDA(e);
             p->allocs.push_back(d);
             return d;
         };
@@ -717,6 +720,10 @@ Scat64* build_scat64(const rtg_handle* h, const std::vector<char>& cols, const u
             return nullptr;
         }
         raise_smem_limit((const void*)scat64_kernel, kOzSmem);
+    } catch (const NoRoom&) {   // the FP64 pipe needs none of this
+        cudaGetLastError();
+        free_scat64(p);
+        return nullptr;
     } catch (...) {
         free_scat64(p);
         throw;

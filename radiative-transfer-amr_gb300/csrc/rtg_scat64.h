@@ -11,7 +11,8 @@ struct Scat64;   // digits of W, thresholds and CTAs of one handle
 bool scat64_fits(const ColDev& C);
 // For the columns flagged in cols (each one fits): scls and thr are the
 // drop-rule classes and thresholds per spatial node, d_thr their device copy,
-// which must outlive the result.  nullptr when a W cannot be scaled.
+// which must outlive the result.  nullptr when the digits cannot hold a W or
+// there is no device memory for the tables.
 Scat64* build_scat64(const rtg_handle* h, const std::vector<char>& cols, const uint8_t* scls, const uint64_t* thr,
                      const uint64_t* d_thr);
 void free_scat64(Scat64* p);
