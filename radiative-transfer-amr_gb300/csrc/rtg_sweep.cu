@@ -969,6 +969,16 @@ __global__ void to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __re
         out[i] = __float2bfloat16_rn(in[i]);
 }
 
+// One block per part: its element's record with the part's angular nodes
+__global__ void split_records_kernel(const int32_t* __restrict__ rec, int stride, const int2* __restrict__ parts,
+                                     int32_t* __restrict__ out) {
+    const int2 p = parts[blockIdx.x];
+    for (int w = threadIdx.x; w < stride; w += blockDim.x)
+        out[(int64_t)blockIdx.x * stride + w] = w == kRecR0   ? p.y & 0xFFFF
+                                                : w == kRecNr ? p.y >> 16
+                                                              : rec[(int64_t)p.x * stride + w];
+}
+
 // Builds the upwind maps of the one-phase elements in FP64 (and the FP32
 // sweep's BF16 copies, rounded to nearest even; rows of map_row_layout entries,
 // padding left zero): entry (coupling k, jj) of the row of output l = (ij, r) is -dcoeff_k
@@ -1054,8 +1064,9 @@ struct Sweep {
     float shape_ms[2][kSweepShapes] = {};
     int32_t *d_greg32 = nullptr, *d_greg64 = nullptr;
     int32_t* d_rec = nullptr;            // element records in claim order
-    int32_t* d_rec_split = nullptr;      // the same in parts of kSplitNth angular nodes (FP64)
+    int32_t* d_rec_split = nullptr;      // the same in parts of kSplitNth angular nodes (FP64, from its first sweep on)
     int nsplit = 0;
+    std::vector<int2> parts;             // until then: record, first angular node and from bit 16 their number
     int rec_stride = 0;                  // words per record (a multiple of 32)
     int n_lagged = 0;
     std::vector<void*> allocs;
@@ -1553,28 +1564,49 @@ Sweep* get_sweep(rtg_handle* h, cudaStream_t st) {
         s->d_rec = sw_alloc<int32_t>(s, flat.size());
         RTG_CUDA(cudaMemcpy(s->d_rec, flat.data(), sizeof(int32_t) * flat.size(), cudaMemcpyHostToDevice));
         // the FP64 split list: elements whose parts all fit take one item per
-        // part, next to each other in the claim order
-        std::vector<int32_t> sp;
+        // part, next to each other in the claim order (make_split_list copies the
+        // records once an FP64 sweep is asked for)
+        s->parts.reserve(2 * (size_t)ne);
         for (int idx = 0; idx < ne; ++idx) {
             const std::vector<int32_t>& R = recs[idx];
             const int nth = R[kRecNth], nn = R[kRecNx] * R[kRecNy];
             const int64_t region = map_region<double>(map_row_layout<double>(R[kRecNup] + R[kRecNupN], 0), kSplitNth,
                                                       nn * kSplitNth, R[kRecRaw], R[kRecEt]);
-            const bool parts = (R[kRecOk] & 2) && nth > kSplitNth &&
-                               (region + 2 * (int64_t)rhs_cap) * 8 <= (int64_t)kSplitBudget;
-            for (int r0 = 0; r0 < nth; r0 += parts ? kSplitNth : nth) {
-                const size_t at = sp.size();
-                sp.resize(at + s->rec_stride, 0);
-                std::copy(R.begin(), R.end(), sp.begin() + at);
-                sp[at + kRecR0] = r0;
-                sp[at + kRecNr] = parts ? std::min(kSplitNth, nth - r0) : nth;
-                ++s->nsplit;
-            }
+            const bool fits = (R[kRecOk] & 2) && nth > kSplitNth &&
+                              (region + 2 * (int64_t)rhs_cap) * 8 <= (int64_t)kSplitBudget;
+            for (int r0 = 0; r0 < nth; r0 += fits ? kSplitNth : nth)
+                s->parts.push_back(int2{idx, fits ? r0 | std::min(kSplitNth, nth - r0) << 16 : nth << 16});
         }
-        s->d_rec_split = sw_alloc<int32_t>(s, sp.size());
-        RTG_CUDA(cudaMemcpy(s->d_rec_split, sp.data(), sizeof(int32_t) * sp.size(), cudaMemcpyHostToDevice));
     }
     return s;
+}
+
+// The records of the FP64 sweep's parts, copied on the device from those of the
+// elements.  Built on the host for every handle they took 8 of the 39 ms of the
+// first sweep at 1.95e6 DOF, and at 7.95e6 up to 95 MB beside an FP32 sweep that does
+// not read them.  Without room for them the sweep has whole elements alone.
+static void make_split_list(Sweep* s, cudaStream_t st) {
+    const size_t n = s->parts.size();
+    int2* d_parts = nullptr;
+    cudaError_t e = cudaMalloc(&d_parts, sizeof(int2) * std::max<size_t>(n, 1));
+    if (e == cudaSuccess) {
+        e = cudaMalloc(&s->d_rec_split, sizeof(int32_t) * std::max<size_t>(n, 1) * s->rec_stride);
+        if (e != cudaSuccess) cudaFree(d_parts);
+    }
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return;
+    }
+    RTG_CUDA(e);
+    s->allocs.push_back(s->d_rec_split);
+    s->allocs.push_back(d_parts);
+    if (n) {
+        RTG_CUDA(cudaMemcpy(d_parts, s->parts.data(), sizeof(int2) * n, cudaMemcpyHostToDevice));
+        split_records_kernel<<<(int)n, 128, 0, st>>>(s->d_rec, s->rec_stride, d_parts, s->d_rec_split), count_launch();
+        RTG_CUDA(cudaGetLastError());
+    }
+    s->nsplit = (int)n;
+    std::vector<int2>().swap(s->parts);
 }
 
 // z = P^{-1} r (full-length vectors; inflow-boundary entries of z are zero).
@@ -1604,7 +1636,8 @@ void apply_sweep(rtg_handle* h, const T* r, T* z, cudaStream_t st, unsigned long
     using TG = typename MapStore<T>::type;
     um.G = f64 ? (const TG*)(const void*)s->d_G64 : (const TG*)(const void*)s->d_G16;
     const int ne = (int)h->host.elems.size();
-    const int nshapes = f64 ? kSweepShapes : kWholeShapes;
+    if (f64 && s->pick[pi] < 0 && !s->d_rec_split) make_split_list(s, st);
+    const int nshapes = f64 && s->d_rec_split ? kSweepShapes : kWholeShapes;
     auto launch = [&](const Sweep::Shape& sh) {
         const bool split = sh.split && !trace;   // a trace has one record per element
         um.reg_cap = sh.reg_cap;
