@@ -80,10 +80,17 @@ class _Copied:
     attributes as copy.deepcopy's own walk in a third of its time (every solve
     returns its solution with a copy of the mesh)."""
 
+    def __init_subclass__(cls, **kw):
+        """A subclass of a mesh class may keep state elsewhere than in its attributes: it
+        is copied as it says itself, or by copy.deepcopy's own walk."""
+        super().__init_subclass__(**kw)
+        if _Copied not in cls.__bases__:
+            own = [k.__dict__["__deepcopy__"] for k in cls.__mro__
+                   if k is not _Copied and k.__dict__.get("__deepcopy__") is not None]
+            cls.__deepcopy__ = own[0] if own else None
+
     def __deepcopy__(self, memo):
         cls = type(self)
-        if cls.__module__ != __name__:      # a subclass may keep its state elsewhere
-            return copy._reconstruct(self, memo, *self.__reduce_ex__(4))
         out = cls.__new__(cls)
         memo[id(self)] = out
         attrs = out.__dict__

@@ -79,3 +79,30 @@ def test_vector_follows_the_cells(make):
     assert q.from_vector(np.concatenate([v, [5.]])).to_vector().tolist() == v.tolist()
     v[0] = 4.
     assert q.to_vector()[0] != 4.
+
+
+def test_subclasses_are_copied_as_they_say():
+    """Wherever a subclass is defined (here: one that names the package's module as its own): state outside of the
+    attributes is copied, and a __deepcopy__ of its own or of another base is taken."""
+    class Slotted(Mesh):
+        __slots__ = ("kept",)
+
+    Slotted.__module__ = Mesh.__module__
+    s = Slotted([1., 1.], [False, False], [2, 2, 2], True)
+    s.kept, s.q = [1], [2]
+    t = copy.deepcopy(s)
+    assert type(t) is Slotted and t == s
+    assert t.kept == [1] and t.kept is not s.kept and t.q == [2] and t.q is not s.q
+
+    class Own:
+        def __deepcopy__(self, memo):
+            return "own"
+
+    class First(Own, Mesh):
+        pass
+
+    class Last(Slotted, Own):
+        pass
+
+    for cls in (First, Last):
+        assert copy.deepcopy(cls([1., 1.], [False, False], [2, 2, 2], True)) == "own"
