@@ -728,6 +728,8 @@ int solve_batched(rtg_handle* h, int nb, const int64_t* inst_off, const double* 
     }
     if (sweep_status(h, s) != RTG_OK)
         throw RtgError{RTG_ERR_TIMEOUT, "a sweep wait gave up; the solution is not valid"};
+    if (apply_status(h, s) != RTG_OK)
+        throw RtgError{RTG_ERR_TIMEOUT, "a tensor-core wait of an apply gave up; the solution is not valid"};
     // u = x on the unknowns, g on the inflow-boundary DOFs
     bscale_kernel<double, double><<<nc, kBThreads, 0, s>>>(w->d_ch, w->x, w->gb, nullptr, 0, 1., 1.), count_launch();
     RTG_CUDA(cudaMemcpyAsync(u, w->gb, sizeof(double) * N, cudaMemcpyDeviceToDevice, s));
