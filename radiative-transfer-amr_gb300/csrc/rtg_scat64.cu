@@ -16,11 +16,12 @@
 // |W|_max |x|_max.
 //
 // What is left out (s >= 12, and W and x below 2^-78 of their largest entry) is
-// at most 578 + 128 of these units for every x that is not zero in fixed point, and
+// at most 578 + 128 of these units for every x that is not zero in fixed point, 64 for
+// one that only fixed point makes zero, and
 // D_11, if it passes 2^24, is off by at most 2 a multiply, 320.  Against the FP64 sum
 // of a row that is small only where the sum is not itself small beside |W|_max
-// |x|_max: so an output below 2^52 times that (kOzLost, kOzRound; 2^-12 of the
-// largest product at 256 nonzero x) is summed again, term by term in FP64: one in a
+// |x|_max: so an output below 2^52 times that (kOzLost, kOzTiny, kOzRound; 2^-12 of
+// the largest product at 256 nonzero x) is summed again, term by term in FP64: one in a
 // few thousand outputs for random x.  The apply at 7.95e6 DOF takes 1456 us for
 // random x, 1787 for a solution, 2309 for a beam in every column, 3353 for
 // randn exp(12 randn), 4234 on the FP64 pipe.
@@ -62,7 +63,8 @@ constexpr int kOzM = 128;        // rows of a CTA (TMEM lanes)
 constexpr int kOzN = 24;         // nodes of a CTA, at most
 constexpr int kOzK = 16;         // angular nodes per stage: one tcgen05.mma step
 constexpr int kOzD = 10;         // digits
-constexpr int kOzLost = 710, kOzRound = 512;   // what an x, and the sum, may be off by (units of T)
+// what an x, one that is zero in fixed point, and the sum may be off by (units of T)
+constexpr int kOzLost = 710, kOzTiny = 64, kOzRound = 512;
 constexpr int kOzMaxNth = 256;   // angular nodes a column may have (bound of the FP32 sums)
 constexpr int kRowBytes = kOzD * kOzK * 2;            // digits of a row of W per stage
 constexpr int kABytes = kOzM * kRowBytes;
@@ -183,7 +185,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     __shared__ int s_node[kOzN];       // node in the column
     __shared__ double s_g[kOzN];       // -cw 2^(E - 1064); 0: nothing to add
     __shared__ double s_cw[kOzN];      // -cw
-    __shared__ int s_nz[kOzN];         // x that are not zero in fixed point
+    __shared__ int s_off[kOzN];        // units of T that the node's sums may be off by
     after_trigger();
     const OzItem it = items[blockIdx.x];
     const ColDev C = v.cols[it.col];
@@ -214,7 +216,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         s_node[tid] = ij;
         cw = v.colc[it.col] * v.sw[C.node_off + ij];
         s_cw[tid] = -cw;
-        s_nz[tid] = 0;
+        s_off[tid] = kOzRound;
     } else if (tid >= 32 && tid - 32 < nch) {
         for (int q = 0; q < 8; ++q) {
             const float2 w = wrange[it.wrange + 8 * (tid - 32) + q];
@@ -349,7 +351,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
         };
         load_w(0);
         double x0 = load_x(kp), x1 = load_x(kp + 1);
-        int nz = 0;
+        int off = 0;
         for (int ch = 0; ch < nch; ++ch) {
             const int b = ch & 1, c0 = ch * kOzK;
             unsigned char* Bb = Bs + b * kBBytes;
@@ -360,7 +362,8 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
             }
             if (bact) {
                 const OzDigits d0 = oz_digits(x0, max(En, 1)), d1 = oz_digits(x1, max(En, 1));   // x is zero where En is
-                nz += !d0.zero() + !d1.zero();
+                off += d0.zero() ? (x0 != 0. ? kOzTiny : 0) : kOzLost;
+                off += d1.zero() ? (x1 != 0. ? kOzTiny : 0) : kOzLost;
 #pragma unroll
                 for (int j = 0; j < kOzD; ++j)
                     *reinterpret_cast<uint32_t*>(Bb + boff + j * np * 32) = oz_pair(d0, d1, j);
@@ -401,7 +404,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
             load_w(ch + 1);
         }
         if (any) s_any[mr] = 1;
-        if (nz) atomicAdd(&s_nz[nb], nz);
+        if (off) atomicAdd(&s_off[nb], off);
         if (!ok) s_abort = 1;
     }
     // the last commit follows every multiply of the CTA
@@ -459,7 +462,7 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
                     L = (L << 8) + __float2int_rn(__uint_as_float(d[k + 5][jj]));
                 }
                 H += L >> 40;
-                if (llabs(H) < (long long)(kOzLost * s_nz[n] + kOzRound) << 12) {   // units of 2^40: |T| below 2^52 times that
+                if (llabs(H) < (long long)s_off[n] << 12) {   // units of 2^40: |T| below 2^52 times that
                     if (s_any[m]) again(n);   // else every term is dropped
                     continue;
                 }
