@@ -2055,7 +2055,7 @@ static int plan_launches(const ApplyPlan* p) {
 // until it wins.  The product alone does not decide: a column's cost on the tensor
 // cores goes by its tiles of 128 rows and its thresholds.  Whole applies, FP64 pipe
 // against tensor cores, in us: 19.8 and 27.9 at 1.2e6 (33,056 DOF adaptive: an extra
-// launch), 51.6 and 47.2 at 8.6e6 (218,581 DOF adaptive), 4234 and 1456 at
+// launch), 51.6 and 47.2 at 8.6e6 (218,581 DOF adaptive), 4230 and 1407 at
 // 1.5e9 (7.95e6 DOF, two scatterers), 2435 and 559 at 1.1e9 (256 angles), but 502 and
 // 549 at 2.1e7 in 16,384 columns of 3 x 3 nodes and 12 angles (1.77e6 DOF).
 constexpr int64_t kTcOffer = 4'000'000, kTc64Large = 100'000'000;

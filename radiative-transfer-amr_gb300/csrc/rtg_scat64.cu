@@ -22,12 +22,12 @@
 // of a row that is small only where the sum is not itself small beside |W|_max
 // |x|_max: so an output below 2^52 times that (kOzLost, kOzTiny, kOzRound; 2^-12 of
 // the largest product at 256 nonzero x) is summed again, term by term in FP64: one in a
-// few thousand outputs for random x.  The apply at 7.95e6 DOF takes 1456 us for
-// random x, 1787 for a solution, 2309 for a beam in every column, 3353 for
-// randn exp(12 randn), 4234 on the FP64 pipe.
+// few thousand outputs for random x.  The apply at 7.95e6 DOF takes 1407 us for
+// random x, 1744 for a solution, 2273 for a beam in every column, 3329 for
+// randn exp(12 randn); 4230 on the FP64 pipe.
 // Every other output is within 2^-52 of the sum of its terms, as an FP64 sum of so
 // many terms is not.  With eight digits and no second sum the apply
-// at 7.95e6 DOF takes 1286 us, but a beam's terms were off by 1e-13 of
+// at 7.95e6 DOF took 1286 us, but a beam's terms were off by 1e-13 of
 // their size for the g = 0.95 kernel and 3e-7 for exp(20 (cos - 1)).
 //
 // Drop rule (rt/preconditioner_matrix.py:450-495): a node of class 2 keeps the
@@ -261,21 +261,23 @@ scat64_kernel(OpView<double> v, uint32_t flags, const OzItem* __restrict__ items
     // the stages in which some |W| is dropped
     if (lo < thr_cta) atomicOr(&s_need, 1 << (tid - 32));
     if (tid < kOzM) s_any[tid] = 0;
-    // per node the largest |x| (a lane takes a node)
+    // per node the largest |x|: a lane takes a node and, where few nodes share the
+    // CTA, a warp several cells at once (apply at 7.95e6 DOF 1448 -> 1405 us)
     const double* xc = x + C.dof_off;
-    for (int k = warp; k < ncell; k += kOzThreads / 32 + 1) {
-        const ElemDev E = v.elems[C.elem_begin + k];
-        if (lane < it.nn) {
-            const double* xk = xc + nij * E.row + s_node[lane] * E.nth;
-            unsigned mx = 0;
+    const int cells = 32 / np, node = lane - lane / np * np;
+    if (lane < cells * np && node < it.nn) {
+        unsigned mx = 0;
+        for (int k = warp * cells + lane / np; k < ncell; k += (kOzThreads / 32 + 1) * cells) {
+            const ElemDev E = v.elems[C.elem_begin + k];
+            const double* xk = xc + nij * E.row + s_node[node] * E.nth;
 #pragma unroll 4
             for (int r = 0; r < E.nth; ++r) {
                 const double xv = xk[r];
                 const unsigned hi = (unsigned)__double2hiint(xv) & 0x7FFFFFFFu;
                 mx = max(mx, hi ? hi : (__double2loint(xv) ? 1u : 0u));
             }
-            atomicMax(&s_max[lane], mx);
         }
+        atomicMax(&s_max[node], mx);
     }
     __syncthreads();
     if (tid < kOzN) {
