@@ -10,7 +10,7 @@
 // product from shared memory in 4 x 4 register tiles, factorised inflow face
 // fluxes, then every output DOF written in global order.  FP32 plans may hand
 // the scattering product to scat_tc_kernel (tcgen05 tensor cores, TF32 hi/lo
-// split), FP64 plans to rtg_scat64.cu (tcgen05, eight 8-bit digits).  The plan shape (rows per item, items per CTA, launches per
+// split), FP64 plans to rtg_scat64.cu (tcgen05, ten 8-bit digits).  The plan shape (rows per item, items per CTA, launches per
 // shared-memory class, tensor cores or not) is autotuned per handle
 // (tune_plan).  Columns too large for the tiled path use apply_col_kernel
 // (per-output chunks from shared memory) or apply_global_kernel (operands
